@@ -98,11 +98,13 @@ struct Cfg {
 // -------------------------------------------------------------- Hamiltonian
 
 // H = sum_t coeffs[t] P_t, P_t given by n characters (I, X, Y, Z; character q
-// acts on qubit q), grouped by X part for the joint kernel.
+// acts on qubit q), grouped by X part.
 struct Ham {
   HamTerms groups{};
   std::vector<uint64_t> zmask;
   std::vector<double2> coef;   // coeffs[t] * i^(number of Y)
+  HamPlan plan;                // the tile-pass executor's sweeps and their tables
+  std::vector<uint64_t> tables;
 };
 
 bool build_ham(int n, size_t nterms, const double* coeffs, const char* paulis, Ham& h, std::string& err) {
@@ -341,9 +343,9 @@ struct Pending {
 struct Workspace {
   int device = 0, num_sms = 148;
   cudaStream_t stream = nullptr;
-  DevBuf<double2> psi, joint, mats, coef;
+  DevBuf<double2> psi, joint, mats;
   DevBuf<double> red, gpart, gsum;
-  DevBuf<uint64_t> zmask;
+  DevBuf<uint64_t> ham;
   DevBuf<int> status;
   HostBuf<double2> hmats[2];
   HostBuf<double> hout[2];    // energies of the job's sets, then their gradient terms
@@ -388,7 +390,7 @@ struct Workspace {
     pend[0].active = pend[1].active = false;
     if (!psi.ensure(bd.psi_amps, err, "the states", stream) ||
         !joint.ensure(bd.joint_amps, err, "the joint arrays", stream) || !status.ensure(1, err, "the status word") ||
-        !red.ensure(bd.sets * (kRedBlocks + 1), err, "reduction partials", stream))
+        !red.ensure(bd.sets * (kHamPartials + 1), err, "reduction partials", stream))
       return false;
     return cudaMemsetAsync(status.p, 0, sizeof(int), stream) == cudaSuccess;
   }
@@ -400,8 +402,8 @@ struct Workspace {
 
   void release() {
     if (stream) cudaStreamSynchronize(stream);
-    psi.release(); joint.release(); mats.release(); coef.release(); red.release(); gpart.release(); gsum.release();
-    zmask.release(); status.release();
+    psi.release(); joint.release(); mats.release(); red.release(); gpart.release(); gsum.release();
+    ham.release(); status.release();
     for (int i = 0; i < 2; ++i) {
       hmats[i].release();
       hout[i].release();
@@ -599,7 +601,7 @@ bool launch_sets(Workspace& w, const Cfg& cfg, Circuit& c, const std::vector<siz
   const double2* psi0 = w.psi.p;
   const double2* joint0 = w.joint.p;
   if (!w.mats.ensure(2 * per * S, err, "matrices", w.stream) ||
-      !w.red.ensure((size_t)S * (kRedBlocks + 1), err, "reduction partials", w.stream) ||
+      !w.red.ensure((size_t)S * (kHamPartials + 1), err, "reduction partials", w.stream) ||
       (!want_grad && !w.psi.ensure(dim * S, err, "the states", w.stream)))
     return false;
   const unsigned max_grid = (unsigned)w.num_sms * (unsigned)std::max(1, cfg.tl.ctas_per_sm);
@@ -611,13 +613,9 @@ bool launch_sets(Workspace& w, const Cfg& cfg, Circuit& c, const std::vector<siz
     return false;
   if (w.psi.p != psi0 || w.joint.p != joint0) w.tmaps.clear();
   if (w.ham_of != &c) {
-    if (!w.zmask.ensure(c.ham.zmask.size(), err, "Hamiltonian", w.stream) ||
-        !w.coef.ensure(c.ham.coef.size(), err, "Hamiltonian", w.stream))
-      return false;
-    // copies from pageable memory: staged before cudaMemcpyAsync returns
-    if (!cuda_ok(cudaMemcpyAsync(w.zmask.p, c.ham.zmask.data(), c.ham.zmask.size() * 8, cudaMemcpyHostToDevice, w.stream),
-                 "H2D Hamiltonian", err) ||
-        !cuda_ok(cudaMemcpyAsync(w.coef.p, c.ham.coef.data(), c.ham.coef.size() * 16, cudaMemcpyHostToDevice, w.stream),
+    if (!w.ham.ensure(c.ham.tables.size(), err, "Hamiltonian", w.stream)) return false;
+    // a copy from pageable memory: staged before cudaMemcpyAsync returns
+    if (!cuda_ok(cudaMemcpyAsync(w.ham.p, c.ham.tables.data(), c.ham.tables.size() * 8, cudaMemcpyHostToDevice, w.stream),
                  "H2D Hamiltonian", err))
       return false;
     w.ham_of = &c;
@@ -630,14 +628,15 @@ bool launch_sets(Workspace& w, const Cfg& cfg, Circuit& c, const std::vector<siz
     return false;
 
   double* partials = w.red.p;
-  double* energy_dev = w.red.p + (size_t)S * kRedBlocks;
+  double* energy_dev = w.red.p + (size_t)S * kHamPartials;
+  const HamTables ht = c.ham.plan.tables(w.ham.p);
   if (!want_grad) {
     // forward from |0> for every set on the state buffer, then the energies
     if (!cuda_ok(launch_set_basis_sets(w.psi.p, dim, (int)S, w.stream), "reset", err)) return false;
     if (!run_shape(w, cfg, *fw, fw_cached, w.psi.p, S, dm, (uint32_t)nf, nullptr, 0, nullptr, st, err)) return false;
     st.fw_passes += (fw->tiled ? fw->plans.size() : fw->sops.size()) * S;
-    if (!cuda_ok(launch_hamiltonian_joint(w.psi.p, dim, c.n, (int)S, c.ham.groups, w.zmask.p, w.coef.p, nullptr, 0,
-                                          partials, energy_dev, w.stream),
+    if (!cuda_ok(launch_hamiltonian(c.ham.plan, ht, w.psi.p, dim, (int)S, nullptr, 0, partials, energy_dev, nullptr,
+                                    w.stream),
                  "energy kernel", err))
       return false;
     st.launches += 3;
@@ -654,11 +653,11 @@ bool launch_sets(Workspace& w, const Cfg& cfg, Circuit& c, const std::vector<siz
     if (!run_shape(w, cfg, *fw, fw_cached, w.joint.p, S, dm, (uint32_t)nf, nullptr, 0, nullptr, st, err, jdim))
       return false;
     st.fw_passes += (fw->tiled ? fw->plans.size() : fw->sops.size()) * S;
-    if (cfg.c64 ? !cuda_ok(launch_hamiltonian_c64(J64, jdim, c.n, (int)S, c.ham.groups, w.zmask.p, w.coef.p, J64 + dim,
-                                                  jdim, partials, energy_dev, w.stream),
+    if (cfg.c64 ? !cuda_ok(launch_hamiltonian_c64(c.ham.plan, ht, J64, jdim, (int)S, J64 + dim, jdim, partials,
+                                                  energy_dev, w.stream),
                            "Hamiltonian kernel", err)
-                : !cuda_ok(launch_hamiltonian_joint(w.joint.p, jdim, c.n, (int)S, c.ham.groups, w.zmask.p, w.coef.p,
-                                                    w.joint.p + dim, jdim, partials, energy_dev, w.stream),
+                : !cuda_ok(launch_hamiltonian(c.ham.plan, ht, w.joint.p, jdim, (int)S, w.joint.p + dim, jdim, partials,
+                                              energy_dev, nullptr, w.stream),
                            "Hamiltonian kernel", err))
       return false;
     unsigned grid = 0;
@@ -871,6 +870,9 @@ int run_batch(std::vector<std::unique_ptr<Circuit>>& circs, int nstreams, bool w
       resident_sets += c->nsets;
       continue;
     }
+    plan_hamiltonian(c->n, c->ham.groups, c->ham.zmask.data(), c->ham.coef.data(), c64 ? 1 : kHamMaxSweeps, c->ham.plan);
+    c->ham.tables.resize(c->ham.plan.table_bytes() / 8 + 1);
+    c->ham.plan.pack(c->ham.tables.data());
     const double per_set = (c64 ? 8.0 : 16.0) * std::ldexp(1.0, joint_bits(c->n));
     const size_t group = want_grad ? (size_t)std::max(1.0, std::floor(job_bytes / per_set)) : 1;
     // per set: at most 3 rotations per gate, each at most a dense 4x4 (16

@@ -599,52 +599,6 @@ cudaError_t launch_partial_trace(const double2* s, int nbits, const int* keep, i
 
 // ---------------------------------------------------- adjoint gradients
 
-// lambda = H psi written next to psi in the joint array (joint[2x] = psi[x],
-// joint[2x + 1] = lambda[x]; skipped when joint is null) and the block sums of
-// Re conj(psi) lambda.
-// H = sum over groups g of sum over terms t of c_t (-1)^popc((x ^ xmask_g) & zmask_t)
-// psi[x ^ xmask_g]: Pauli strings sharing their X part share one gather.
-__global__ void row_sum_kernel(const double* __restrict__ in, int cols, double* __restrict__ out);
-
-// blockIdx.y = set: psi + set * pstride, lam + set * lstride, partials + set * gridDim.x
-__global__ void hamiltonian_joint_kernel(const double2* __restrict__ psi, uint64_t pstride, uint64_t dim, HamTerms h,
-                                         const uint64_t* __restrict__ zmask, const double2* __restrict__ coef,
-                                         double2* __restrict__ lam_out, uint64_t lstride, double* __restrict__ partials) {
-  psi += blockIdx.y * pstride;
-  if (lam_out) lam_out += blockIdx.y * lstride;
-  partials += (size_t)blockIdx.y * gridDim.x;
-  double e = 0.0;
-  for (uint64_t x = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; x < dim; x += (uint64_t)gridDim.x * blockDim.x) {
-    const double2 px = psi[x];
-    double2 lam = make_double2(0.0, 0.0);
-    for (int g = 0; g < h.ngroups; ++g) {
-      const uint64_t src = x ^ h.xmask[g];
-      const double2 a = (h.xmask[g] == 0) ? px : psi[src];
-      double2 f = make_double2(0.0, 0.0);
-      for (int t = h.first[g]; t < h.first[g + 1]; ++t) {
-        const double2 c = coef[t];
-        if (__popcll(src & zmask[t]) & 1) { f.x -= c.x; f.y -= c.y; }
-        else { f.x += c.x; f.y += c.y; }
-      }
-      lam = cfma(lam, f, a);
-    }
-    if (lam_out) lam_out[x] = lam;
-    e += px.x * lam.x + px.y * lam.y;
-  }
-  e = block_sum(e);
-  if (threadIdx.x == 0) partials[blockIdx.x] = e;
-}
-
-cudaError_t launch_hamiltonian_joint(const double2* psi, uint64_t pstride, int n, int nsets, const HamTerms& h,
-                                     const uint64_t* zmask, const double2* coef, double2* lam, uint64_t lstride,
-                                     double* partials, double* energy, cudaStream_t st) {
-  if (nsets < 1) nsets = 1;
-  hamiltonian_joint_kernel<<<dim3(kRedBlocks, nsets), kRedThreads, 0, st>>>(psi, pstride, 1ULL << n, h, zmask, coef,
-                                                                            lam, lstride, partials);
-  row_sum_kernel<<<nsets, 256, 0, st>>>(partials, kRedBlocks, energy);
-  return cudaGetLastError();
-}
-
 // nsets joint arrays of jdim amplitudes end to end: psi half [0, dim) set to
 // e_0, everything above 2 * dim (zero padding of small circuits) to zero; the
 // lambda half [dim, 2 * dim) is left for the Hamiltonian kernel
@@ -659,48 +613,6 @@ __global__ void init_joint_kernel(double2* __restrict__ s, uint64_t dim, uint64_
 cudaError_t launch_init_joint(double2* s, int n, uint64_t jdim, int nsets, cudaStream_t st) {
   const uint64_t total = jdim * (uint64_t)(nsets < 1 ? 1 : nsets);
   init_joint_kernel<<<grid_for(total, 256), 256, 0, st>>>(s, 1ULL << n, jdim, total);
-  return cudaGetLastError();
-}
-
-// complex64 storage of the same: psi_s at psi + s * pstride (float2), lambda_s
-// written to lam + s * lstride (float2, rounded once), every product and sum in FP64
-__global__ void hamiltonian_c64_kernel(const float2* __restrict__ psi, uint64_t pstride, uint64_t dim, HamTerms h,
-                                       const uint64_t* __restrict__ zmask, const double2* __restrict__ coef,
-                                       float2* __restrict__ lam_out, uint64_t lstride, double* __restrict__ partials) {
-  psi += blockIdx.y * pstride;
-  if (lam_out) lam_out += blockIdx.y * lstride;
-  partials += (size_t)blockIdx.y * gridDim.x;
-  double e = 0.0;
-  for (uint64_t x = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; x < dim; x += (uint64_t)gridDim.x * blockDim.x) {
-    const float2 pf = psi[x];
-    const double2 px = make_double2(pf.x, pf.y);
-    double2 lam = make_double2(0.0, 0.0);
-    for (int g = 0; g < h.ngroups; ++g) {
-      const uint64_t src = x ^ h.xmask[g];
-      const float2 af = psi[src];
-      const double2 a = (h.xmask[g] == 0) ? px : make_double2(af.x, af.y);
-      double2 f = make_double2(0.0, 0.0);
-      for (int t = h.first[g]; t < h.first[g + 1]; ++t) {
-        const double2 c = coef[t];
-        if (__popcll(src & zmask[t]) & 1) { f.x -= c.x; f.y -= c.y; }
-        else { f.x += c.x; f.y += c.y; }
-      }
-      lam = cfma(lam, f, a);
-    }
-    if (lam_out) lam_out[x] = make_float2(__double2float_rn(lam.x), __double2float_rn(lam.y));
-    e += px.x * lam.x + px.y * lam.y;
-  }
-  e = block_sum(e);
-  if (threadIdx.x == 0) partials[blockIdx.x] = e;
-}
-
-cudaError_t launch_hamiltonian_c64(const float2* psi, uint64_t pstride, int n, int nsets, const HamTerms& h,
-                                   const uint64_t* zmask, const double2* coef, float2* lam, uint64_t lstride,
-                                   double* partials, double* energy, cudaStream_t st) {
-  if (nsets < 1) nsets = 1;
-  hamiltonian_c64_kernel<<<dim3(kRedBlocks, nsets), kRedThreads, 0, st>>>(psi, pstride, 1ULL << n, h, zmask, coef,
-                                                                          lam, lstride, partials);
-  row_sum_kernel<<<nsets, 256, 0, st>>>(partials, kRedBlocks, energy);
   return cudaGetLastError();
 }
 

@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <vector>
+
 #include "iq_plan.h"
 
 namespace iqb {
@@ -96,19 +98,57 @@ struct HamTerms {
   uint64_t xmask[kMaxHamGroups];
   int first[kMaxHamGroups + 1];
 };
+// The Hamiltonian sweeps of iq_ham.cu: a plan (host), its tables (device) and the launch.
+constexpr int kHamMaxSweeps = 6;
+constexpr int kHamBlocks = 2 * 148;    // CTAs per set and sweep: two tiles of 64 KiB fit an SM
+// partial sums a launch needs per set (twice that with the imaginary part)
+constexpr size_t kHamPartials = (size_t)kHamMaxSweeps * kHamBlocks;
+constexpr uint32_t HAM_GATHER = 1;     // partners from global memory, not from the tile
+constexpr uint32_t HAM_IMAG = 2;       // the strings' imaginary coefficients
+constexpr uint32_t HAM_FLAT = 4;       // no string's sign depends on the thread's register bits
+struct HamItem {                       // one group's real or imaginary strings in one sweep
+  uint64_t xmask;
+  uint32_t lmask;                      // xmask in tile-local bits
+  uint32_t flags;
+  int first[17];                       // strings by sign pattern over the tile-local bits 8..11
+};
+struct HamSweep {
+  uint64_t ntiles;
+  int nbits, add;
+  int item0, item1, term0, term1;      // its items, their strings
+  uint8_t bit[12];                     // physical bit of each tile-local bit, ascending
+};
+struct HamTables {
+  const HamItem* items;
+  const uint64_t* z;
+  const double* c;
+};
+struct HamPlan {
+  std::vector<HamSweep> sweeps;
+  std::vector<HamItem> items;
+  std::vector<uint64_t> z;
+  std::vector<double> c;
+  size_t table_bytes() const;
+  void pack(void* dst) const;          // table_bytes() bytes, 8-byte aligned
+  HamTables tables(const void* dev) const;
+};
+// max_sweeps (1..kHamMaxSweeps): groups left over after that many sweeps gather from global memory
+void plan_hamiltonian(int n, const HamTerms& h, const uint64_t* zmask, const double2* coef, int max_sweeps,
+                      HamPlan& hp);
 // For each of nsets states psi_s = psi + s * pstride (2^n amplitudes):
 // lambda_s = H psi_s written to lam + s * lstride (when lam is not null), and
-// energy[s] = Re <psi_s|H|psi_s>.  partials: nsets * kRedBlocks.
-cudaError_t launch_hamiltonian_joint(const double2* psi, uint64_t pstride, int n, int nsets, const HamTerms& h,
-                                     const uint64_t* zmask, const double2* coef, double2* lam, uint64_t lstride,
-                                     double* partials, double* energy, cudaStream_t st);
+// energy[s] = Re <psi_s|H|psi_s> (energy_im: the imaginary part, if not null).
+cudaError_t launch_hamiltonian(const HamPlan& hp, const HamTables& tb, const double2* psi, uint64_t pstride, int nsets,
+                               double2* lam, uint64_t lstride, double* partials, double* energy, double* energy_im,
+                               cudaStream_t st);
+// complex64 (float2) storage, products and sums in FP64; a plan of one sweep, so lambda is rounded once
+cudaError_t launch_hamiltonian_c64(const HamPlan& hp, const HamTables& tb, const float2* psi, uint64_t pstride,
+                                   int nsets, float2* lam, uint64_t lstride, double* partials, double* energy,
+                                   cudaStream_t st);
 // nsets joint arrays [psi | lambda | zero padding] of jdim amplitudes end to
 // end: psi halves (2^n amplitudes) set to e_0, padding above 2^(n+1) zeroed.
 cudaError_t launch_init_joint(double2* s, int n, uint64_t jdim, int nsets, cudaStream_t st);
-// The same two with complex64 (float2) storage; products and sums in FP64.
-cudaError_t launch_hamiltonian_c64(const float2* psi, uint64_t pstride, int n, int nsets, const HamTerms& h,
-                                   const uint64_t* zmask, const double2* coef, float2* lam, uint64_t lstride,
-                                   double* partials, double* energy, cudaStream_t st);
+// The same with complex64 (float2) storage.
 cudaError_t launch_init_joint_c64(float2* s, int n, uint64_t jdim, int nsets, cudaStream_t st);
 cudaError_t launch_row_sums(const double* in, int rows, int cols, double* out, cudaStream_t st);
 

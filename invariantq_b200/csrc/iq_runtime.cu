@@ -22,6 +22,7 @@
 #include <mutex>
 #include <random>
 #include <string>
+#include <unordered_map>
 #include <vector>
 
 #include "../../include/invariantq_b200.h"
@@ -277,7 +278,7 @@ struct Engine {
       d_state = nullptr;
       return false;
     }
-    scratch_bytes = std::max<size_t>(zsums_partials_doubles(nbits) * 8, (size_t)kRedBlocks * 16) + 4096;
+    scratch_bytes = std::max<size_t>({zsums_partials_doubles(nbits) * 8, (size_t)kRedBlocks * 16, kHamPartials * 16}) + 4096;
     if (!cuda_ok(cudaMalloc(&d_scratch, scratch_bytes), "cudaMalloc scratch")) return false;
     if (!cuda_ok(cudaMalloc(&d_status, sizeof(int)), "cudaMalloc status")) return false;
     if (!cuda_ok(cudaMallocHost(&h_small, 64 * 1024), "cudaMallocHost")) return false;
@@ -1110,31 +1111,62 @@ int iq_statevector_expval_pauli_sum(void* sv, size_t nterms, const double* coeff
   if (!e || !coeffs || !paulis || !val_real || !val_imag) return -1;
   const int n = e->nbits;
   if (!e->sync()) return -1;
-  double2* part = reinterpret_cast<double2*>(e->partials());
-  double2* res = reinterpret_cast<double2*>(e->result_slot());
-  cd total(0.0, 0.0);
-  static const cd ipow[4] = {cd(1, 0), cd(0, 1), cd(-1, 0), cd(0, -1)};
+  // strings sharing their X part form a group (HamTerms); every kMaxHamGroups of them share their sweeps (iq_ham.cu)
+  struct Group { uint64_t xm; std::vector<std::pair<uint64_t, double2>> terms; };
+  std::vector<Group> groups;
+  std::unordered_map<uint64_t, size_t> by_x;
   for (size_t t = 0; t < nterms; ++t) {
     uint64_t xm = 0, zm = 0;
     int ny = 0;
     for (int q = 0; q < n; ++q) {
       const char c = paulis[t * n + q];
       const uint64_t b = 1ULL << q;
-      if (c == 'X') xm ^= b;
-      else if (c == 'Y') { xm ^= b; zm ^= b; ++ny; }
-      else if (c == 'Z') zm ^= b;
+      if (c == 'X') xm |= b;
+      else if (c == 'Y') { xm |= b; zm |= b; ++ny; }
+      else if (c == 'Z') zm |= b;
       else if (c != 'I') {
         set_error(E_ARG, "expval_pauli_sum: invalid Pauli character");
         return -1;
       }
     }
+    const auto at = by_x.emplace(xm, groups.size());
+    if (at.second) groups.push_back({xm, {}});
+    const double c = (ny & 2) ? -coeffs[t] : coeffs[t];   // times i^ny
+    groups[at.first->second].terms.push_back({zm, (ny & 1) ? make_double2(0.0, c) : make_double2(c, 0.0)});
+  }
+  cd total(0.0, 0.0);
+  std::vector<double2> blob;
+  for (size_t g0 = 0; g0 < groups.size(); g0 += kMaxHamGroups) {
+    HamTerms h{};
+    h.ngroups = (int)std::min<size_t>(kMaxHamGroups, groups.size() - g0);
+    std::vector<uint64_t> z;
+    std::vector<double2> co;
+    for (int g = 0; g < h.ngroups; ++g) {
+      h.xmask[g] = groups[g0 + g].xm;
+      h.first[g] = (int)z.size();
+      for (const auto& t : groups[g0 + g].terms) {
+        z.push_back(t.first);
+        co.push_back(t.second);
+      }
+    }
+    h.first[h.ngroups] = (int)z.size();
+    HamPlan hp;
+    plan_hamiltonian(n, h, z.data(), co.data(), kHamMaxSweeps, hp);
+    blob.resize(hp.table_bytes() / 16 + 1);
+    hp.pack(blob.data());
+    if (!e->upload_pool(blob.data(), blob.size())) return -1;
+    e->st_h2d -= 16.0 * (double)blob.size();   // counts gate matrices only
+    const uint64_t launches = hp.sweeps.size() + 2;
+    g_launches += launches;
+    e->st_launches += (double)launches;
+    double* res = e->result_slot();
     double out[2];
-    g_launches += 2;
-    e->st_launches += 2;
-    if (!cuda_ok(launch_pauli_sum(e->d_state, e->dim, xm, zm, -1.0, part, res, e->stream), "pauli reduction") ||
-        !e->read_doubles(reinterpret_cast<double*>(res), 2, out))
+    if (!cuda_ok(launch_hamiltonian(hp, hp.tables(e->d_pool), e->d_state, 0, 1, nullptr, 0, e->partials(), res, res + 1,
+                                    e->stream),
+                 "pauli sum") ||
+        !e->read_doubles(res, 2, out))
       return -1;
-    total += coeffs[t] * cd(out[0], out[1]) * ipow[ny & 3];
+    total += cd(out[0], out[1]);
   }
   *val_real = total.real();
   *val_imag = total.imag();
