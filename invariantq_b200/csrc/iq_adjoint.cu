@@ -153,14 +153,13 @@ bool build_ham(int n, size_t nterms, const double* coeffs, const char* paulis, H
 // ------------------------------------------------------------ planned shapes
 
 // A planned operation list that depends only on the circuit's structure: the
-// matrices of one parameter set are gathered into its per-pass blocks with
-// `gather` (block[i] = pool[gather[i]]).
+// matrices of one parameter set are put into its per-pass blocks by `pack`.
 struct Shape {
   int nbits = 0;
   bool tiled = false;
   std::vector<PassPlan> plans;
   std::vector<SimpleOp> sops;
-  std::vector<uint32_t> gather;
+  PackRecipe pack;
   std::vector<SchedOp> sig;
   size_t pool_size = 0;
   unsigned grid = 0;       // tile-pass grid (gradient partials row length)
@@ -172,7 +171,7 @@ struct Shape {
 bool same_op(const SchedOp& a, const SchedOp& b) {
   if (a.k != b.k || a.mono != b.mono || a.perm != b.perm || a.unit != b.unit || a.mat != b.mat ||
       a.dense != b.dense || a.grad != b.grad || a.gen != b.gen || a.gidx != b.gidx || a.rot != b.rot ||
-      a.norm != b.norm || a.urows != b.urows || a.xpat != b.xpat || a.realm != b.realm)
+      a.norm != b.norm || a.urows != b.urows || a.nrows != b.nrows || a.xpat != b.xpat || a.realm != b.realm)
     return false;
   for (int i = 0; i < a.k; ++i)
     if (a.q[i] != b.q[i]) return false;
@@ -192,15 +191,15 @@ bool make_shape(const Cfg& cfg, int nbits, const std::vector<SchedOp>& fused, si
   s.sig = fused;
   s.pool_size = pool_size;
   s.tiled = nbits >= 7;
-  s.gather.clear();
+  s.pack = PackRecipe{};
   if (!s.tiled) {
     for (const SchedOp& o : fused) {
       SimpleOp so{};
       so.k = o.k;
       for (int j = 0; j < o.k; ++j) so.q[j] = o.q[j];
-      so.mat = (uint32_t)s.gather.size();
+      so.mat = (uint32_t)s.pack.base.size();
       const uint32_t d = 1u << o.k;
-      for (uint32_t i = 0; i < d * d; ++i) s.gather.push_back(o.dense + i);
+      for (uint32_t i = 0; i < d * d; ++i) s.pack.base.push_back(o.dense + i);
       s.sops.push_back(so);
     }
     return true;
@@ -211,11 +210,8 @@ bool make_shape(const Cfg& cfg, int nbits, const std::vector<SchedOp>& fused, si
   for (const SchedOp& o : fused) maxk = std::max<int>(maxk, o.k);
   p.R = std::min(5, std::max(cfg.sp.R, maxk));
   if (plan_passes(p, fused, s.plans, err) < 0) return false;
-  std::vector<cplx64> idx(pool_size), packed;
-  for (size_t i = 0; i < pool_size; ++i) idx[i] = {(double)i, 0.0};
-  pack_pass_matrices(s.plans, idx.data(), packed);
-  s.gather.resize(packed.size());
-  for (size_t i = 0; i < packed.size(); ++i) s.gather[i] = (uint32_t)packed[i].re;
+  merge_stage_diagonals(s.plans, fused);
+  pack_recipe(s.plans, s.pack);
   for (const PassPlan& pl : s.plans)
     if (pl.desc.mat_elems > (uint32_t)kSmemMatElems) {
       err = "a pass's matrices exceed the shared-memory block";
@@ -578,7 +574,7 @@ bool launch_sets(Workspace& w, const Cfg& cfg, Circuit& c, const std::vector<siz
   const int k = w.slot;
   w.slot ^= 1;
   if (!finish(w, k, err)) return false;
-  const size_t nf = fw->gather.size(), nb = want_grad ? bw->gather.size() : 0;
+  const size_t nf = fw->pack.base.size(), nb = want_grad ? bw->pack.base.size() : 0;
   const size_t per = nf + nb;
   if (!w.hmats[k].ensure(per * S, err) || !w.hout[k].ensure(S + (size_t)S * ngrads, err) || !w.hstat[k].ensure(1, err))
     return false;
@@ -586,10 +582,8 @@ bool launch_sets(Workspace& w, const Cfg& cfg, Circuit& c, const std::vector<siz
   const auto tg = std::chrono::steady_clock::now();
   for (uint32_t j = 0; j < S; ++j) {
     const JobOps& o = jo[j];
-    double2* f = hm + (size_t)j * nf;
-    for (size_t i = 0; i < nf; ++i) f[i] = make_double2(o.fpool[fw->gather[i]].re, o.fpool[fw->gather[i]].im);
-    double2* b = hm + (size_t)S * nf + (size_t)j * nb;
-    for (size_t i = 0; i < nb; ++i) b[i] = make_double2(o.bpool[bw->gather[i]].re, o.bpool[bw->gather[i]].im);
+    fw->pack.fill(o.fpool.data(), reinterpret_cast<cplx64*>(hm + (size_t)j * nf));
+    if (want_grad) bw->pack.fill(o.bpool.data(), reinterpret_cast<cplx64*>(hm + (size_t)S * nf + (size_t)j * nb));
   }
   st.host_ns += (uint64_t)std::chrono::duration_cast<std::chrono::nanoseconds>(std::chrono::steady_clock::now() - tg)
                     .count();

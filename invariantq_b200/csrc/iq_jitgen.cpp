@@ -274,6 +274,26 @@ bool gen_stage(Gen& g, const PassDesc& d, int s, int NT, std::string& err, int g
         o << "        grad_accumulate(" << acc << ", gs + " << od.gidx << ", lane8, omask);\n";
         break;
       }
+      case OP_DGR: {   // merged diagonal: entries that are exactly 1 or -1 take no product
+        for (int v = 0; v < NV; ++v) {
+          if ((od.gidx >> v) & 1) continue;
+          if ((od.gidx >> (16 + v)) & 1) cur[v] = def("make_double2(-" + cur[v] + ".x, -" + cur[v] + ".y)");
+          else cur[v] = def("cmul(" + mat(m + (uint32_t)(v & od.flags)) + ", " + cur[v] + ")");
+        }
+        break;
+      }
+      case OP_GDZ: {   // Z terms of the slots in `flags` from one product per (psi, lambda) pair
+        if (!g_set_mode) { err = "adjoint steps need the shared-memory form"; return false; }
+        const std::string w = g.fresh();
+        o << "        const double " << w << "[" << NV / 2 << "] = {";
+        for (int v = 0; v < NV; v += 2) o << (v ? ", " : "") << "z_product(" << cur[v] << ", " << cur[v | 1] << ")";
+        o << "};\n";
+        int at = 0;
+        for (int b = 1; b < R; ++b)
+          if ((od.flags >> b) & 1)
+            o << "        grad_accumulate(z_sum(" << w << ", " << b - 1 << "), gs + " << od.gidx + at++ << ", lane8, omask);\n";
+        break;
+      }
       default:
         err = "operation kind " + std::to_string((int)od.kind) + " is not specialised";
         return false;
@@ -296,7 +316,7 @@ std::string jit_pass_key(const PassDesc& d, int min_blocks, int threads, bool se
   std::string k;
   k.reserve(64 + d.nstages * 32 + d.nops * 16);
   auto put = [&](uint32_t v) { k.append(reinterpret_cast<const char*>(&v), sizeof(v)); };
-  put(1);   // key format
+  put(2);   // key format
   put((uint32_t)min_blocks);
   put((uint32_t)threads);
   put(set_mode ? (narrow ? 2u : 1u) : 0u);
@@ -346,7 +366,7 @@ std::string jit_pass_source(const PassDesc& d, std::string& err, int min_blocks,
   const uint32_t nmat = d.mat_elems ? d.mat_elems : 1;
   Gen g;
   std::ostringstream& o = g.o;
-  o << "// generated by iq_jitgen (iq-jit-2): NT=" << NT << " sets=" << (set_mode ? 1 : 0)
+  o << "// generated by iq_jitgen (iq-jit-3): NT=" << NT << " sets=" << (set_mode ? 1 : 0)
     << " narrow=" << (narrow ? 1 : 0) << " M=" << (int)d.M
     << " c=" << (int)d.c << " R=" << (int)d.R
     << " stages=" << (int)d.nstages << " ops=" << d.nops << "\n";

@@ -259,6 +259,25 @@ __device__ __forceinline__ double grad_term(double2 p0, double2 p1, double2 l0, 
   }
 }
 
+// Im conj(l) p of one (psi, lambda) pair: the product every Z term is a signed sum of
+__device__ __forceinline__ double z_product(double2 p, double2 l) { return fma(l.x, p.y, -(l.y * p.x)); }
+
+// sum of w[0..NW) with the entries whose index bit `b` is set subtracted, as a
+// pairwise tree (bit 0 first): the trees of several bits share their plain sums
+template <int NW>
+__device__ __forceinline__ double z_sum(const double (&w)[NW], int b) {
+  double t[NW];
+#pragma unroll
+  for (int i = 0; i < NW; ++i) t[i] = w[i];
+  int bit = 0;
+#pragma unroll
+  for (int n = NW / 2; n >= 1; n >>= 1, ++bit)
+#pragma unroll
+    for (int i = 0; i < NW / 2; ++i)
+      if (i < n) t[i] = bit == b ? t[2 * i] - t[2 * i + 1] : t[2 * i] + t[2 * i + 1];
+  return t[0];
+}
+
 // the octet's eight lanes hold the same registers of eight tile rows: sum
 // their shares, and the octet's lane 0 -- the only writer of its row of
 // accumulators -- adds it there.  Tiles reach a CTA, and tile rows reach an

@@ -86,6 +86,12 @@ enum OpKind : uint8_t {
                 // relaxation channels and of their products; stored whole (16 entries); flags
                 // bit 0: the corners are real, bit 1: the middle is real (3 to 6 FMAs per
                 // amplitude)
+  OP_DGR = 13,  // diagonal over the register slots of mask `flags`: register v is multiplied by
+                // table entry v & flags (2^R entries at `mat`, R <= 4); gidx bit v: the entry is
+                // exactly 1, bit 16 + v: exactly -1 (merge_stage_diagonals)
+  OP_GDZ = 14,  // Z terms of several adjoint steps: for every slot of mask `flags`, in ascending
+                // order, Im<lambda|Z|psi> is added to gradient terms gidx, gidx + 1, ...; the
+                // amplitudes stay as they are (select bit in slot 0)
 };
 
 // SchedOp::xpat bits (0: not OP_X2R's shape)
@@ -176,6 +182,7 @@ struct SchedOp {
   uint8_t xpat;          // k = 2 dense matrix of OP_X2R's shape: XPAT_* bits (0: not)
   uint8_t realm;         // k = 1 dense matrix with real entries (OPF_REAL)
   uint8_t gen;           // adjoint step generator: 0 = X, 1 = Y, 2 = Z
+  uint8_t nrows;         // two-qubit monomial: bit r = row r's phase is exactly -1
   uint32_t gidx;         // adjoint step gradient term index (increasing in queue order)
   // factor the operation multiplies the scale of a scaled backward sweep by
   // (stored amplitudes = true amplitudes / scale; 0 means 1): a scaled
@@ -199,11 +206,19 @@ struct SchedParams {
 }  // namespace iqb
 #include <vector>
 namespace iqb {
+// One diagonal merged into an OP_DGR: on slot a (k = 1) or slots a (row bit 0)
+// and b (k = 2), row r's phase is pool element mat[r] unless bit r of ones
+// (exactly 1) or negs (exactly -1) is set.
+struct DiagFactor {
+  uint8_t a, b, k, ones, negs;
+  uint32_t mat[4];
+};
 struct PassPlan {
   PassDesc desc;
   int nsrc;              // number of scheduled ops
   double cost;           // planned arithmetic cost per amplitude
-  std::vector<uint32_t> src;   // index of desc.ops[i]'s operation in the scheduled list
+  std::vector<uint32_t> src;   // the scheduled operations' indices in the order the pass runs them
+  std::vector<std::vector<DiagFactor>> diag;   // factors of the pass's OP_DGR operations, by OpDesc::mat before packing
 };
 #endif
 
@@ -417,6 +432,27 @@ void decompose_one_qubit_ops(std::vector<SchedOp>& ops, std::vector<cplx64>& poo
 // every op's `mat` relative to its pass block, which the kernel stages in
 // shared memory.
 void pack_pass_matrices(std::vector<PassPlan>& plans, const cplx64* pool, std::vector<cplx64>& packed);
+
+// The same as a recipe over any pool of the plans' structure: element i starts
+// as pool[base[i]] (or as 1 / -1 for kPackOne / kPackMinusOne), then every
+// (i, j) of `mults`, in order, multiplies element i by pool[j].
+constexpr uint32_t kPackOne = 0xFFFFFFFFu, kPackMinusOne = 0xFFFFFFFEu;
+struct PackRecipe {
+  std::vector<uint32_t> base;
+  std::vector<std::pair<uint32_t, uint32_t>> mults;
+  // dst: base.size() elements
+  void fill(const cplx64* pool, cplx64* dst) const;
+};
+void pack_recipe(std::vector<PassPlan>& plans, PackRecipe& r);
+
+// Merge the diagonals of each register stage: the phases of one- and two-qubit
+// monomials (and of Z adjoint steps) that can act at the same point of the
+// stage become one OP_DGR -- one complex product per amplitude at most, where
+// k one-qubit phases alone take k / 2 -- and the Z steps' gradient terms one
+// OP_GDZ.  The stage's other operations keep their order per slot.  For plans
+// of 3 or 4 register slots, before packing; `ops` is the list the plans were
+// made from.
+void merge_stage_diagonals(std::vector<PassPlan>& plans, const std::vector<SchedOp>& ops);
 
 // ---- adjoint-method gradients ----------------------------------------------
 // Gate kinds of a parametrised circuit (the values of the C ABI's IQ_GATE_*).

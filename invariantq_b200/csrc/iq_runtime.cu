@@ -490,6 +490,7 @@ struct Engine {
         set_error(E_STATE, "scheduler: %s", err.c_str());
         return false;
       }
+      if (spec) merge_stage_diagonals(pg.plans, fused);
       pack_pass_matrices(pg.plans, pool.data(), packed);
       src = packed.data();
       nsrc = packed.size();

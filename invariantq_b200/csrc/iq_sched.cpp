@@ -948,7 +948,8 @@ struct Decomposer {
     }
     const cplx64 s0 = Dp[0];
     const cplx64 x1 = cdiv(Dp[1], s0), y1 = cdiv(Dp[2], s0);
-    const cplx64 gamma = cdiv(Dp[3], cm(s0, cm(x1, y1)));
+    // a diagonal gate's own part does not depend on the pending diagonals (CZ: exactly -1)
+    const cplx64 gamma = src.perm == 0xE4 ? cdiv(cm(ph[0], ph[3]), cm(ph[1], ph[2])) : cdiv(Dp[3], cm(s0, cm(x1, y1)));
     G = cm(G, s0);
     pa[q0] = pa[q1] = {1.0, 0.0};
     pb[q0] = x1;
@@ -957,6 +958,7 @@ struct Decomposer {
     const bool unit = is_one(gamma);
     o.unit = unit ? 1 : 0;
     o.urows = unit ? 15 : 7;
+    o.nrows = (gamma.re == -1.0 && gamma.im == 0.0) ? 8 : 0;
     o.mat = put({{1.0, 0.0}, {1.0, 0.0}, {1.0, 0.0}, gamma});
     o.dense = (uint32_t)pool.size();
     for (int r = 0; r < 4; ++r)
@@ -1048,6 +1050,7 @@ void push_op(std::vector<SchedOp>& out, std::vector<cplx64>& pool, int k, const 
     for (int i = 0; i < d; ++i) {
       pool.push_back({ph[2 * i], ph[2 * i + 1]});
       if (ph[2 * i] == 1.0 && ph[2 * i + 1] == 0.0) o.urows |= (uint8_t)(1u << i);   // its product is skipped
+      if (k == 2 && ph[2 * i] == -1.0 && ph[2 * i + 1] == 0.0) o.nrows |= (uint8_t)(1u << i);   // CZ
     }
   } else if (k == 1) {
     bool real = true;
@@ -1269,22 +1272,278 @@ void exec_grad_scales(const std::vector<PassPlan>* plans, const std::vector<Sche
     for (uint32_t i : pl.src) visit(ops[i]);
 }
 
-void pack_pass_matrices(std::vector<PassPlan>& plans, const cplx64* pool, std::vector<cplx64>& packed) {
-  packed.clear();
+namespace {
+
+constexpr uint8_t kPermIdentity2 = 0xE4;   // two-qubit monomial whose rows read their own column
+
+// complex elements of an operation in its pass's matrix block
+uint32_t pack_elems(const OpDesc& o, int R) {
+  switch (o.kind) {
+    case OP_GDZ: return 0;
+    case OP_DGR: return 1u << R;
+    case OP_GRAD2: return 4;
+    case OP_M1R: case OP_M1L: case OP_M2R: return 1u << o.k;
+    default: return 1u << (2 * o.k);
+  }
+}
+
+// one operation of a stage on its way through merge_stage_diagonals
+struct StageItem {
+  OpDesc od;
+  uint32_t src;
+  uint32_t mask;         // register slots (bits 0..4) and lane bits (8..10) it acts on
+  bool diag = false;     // a diagonal: commutes with the other diagonals
+  bool term = false;     // a Z adjoint step: its term is taken where its phase acts
+  bool primary = true;   // carries the source index (the phases split off a permutation do not)
+  DiagFactor f{};
+};
+
+uint32_t slot_mask(const OpDesc& o) {
+  switch (o.kind) {
+    case OP_D1R: case OP_N1R: case OP_R1R: case OP_M1R: return 1u << o.a;
+    case OP_D1L: case OP_R1L: case OP_M1L: return 1u << (8 + o.a);
+    case OP_D2R: case OP_M2R: case OP_X2R: return (1u << o.a) | (1u << o.b);
+    case OP_GRAD2: return 1u << o.b;   // steps on different qubits commute, whatever their select bit
+    default: return 0xFFu;
+  }
+}
+
+// entries of a merged diagonal that are exactly 1 (bits 0..15) and -1 (16..31)
+uint32_t diag_units(const std::vector<DiagFactor>& fs, int NV) {
+  uint32_t out = 0;
+  for (int v = 0; v < NV; ++v) {
+    bool unit = true, neg = false;
+    for (const DiagFactor& f : fs) {
+      const int r = ((v >> f.a) & 1) | (f.k == 2 ? ((v >> f.b) & 1) << 1 : 0);
+      if ((f.negs >> r) & 1) neg = !neg;
+      else if (!((f.ones >> r) & 1)) unit = false;
+    }
+    if (unit) out |= neg ? 1u << (16 + v) : 1u << v;
+  }
+  return out;
+}
+
+// the items of one stage: permutations and their phases apart
+void stage_items(const PassPlan& pl, const StageDesc& sd, const std::vector<SchedOp>& ops, std::vector<StageItem>& out) {
+  for (int i = sd.op0; i < sd.op1; ++i) {
+    StageItem it;
+    it.od = pl.desc.ops[i];
+    it.src = pl.src[i];
+    const OpDesc& o = it.od;
+    it.mask = slot_mask(o);
+    const bool unit = o.flags & OPF_UNIT_PHASE;
+    if (o.kind == OP_M1R && !(o.perm & 1)) {
+      it.diag = true;
+      it.f.a = o.a;
+      it.f.k = 1;
+      it.f.ones = unit ? 3 : (o.urows & 3);
+      it.f.mat[0] = o.mat;
+      it.f.mat[1] = o.mat + 1;
+    } else if (o.kind == OP_M2R && (o.perm == kPermIdentity2 || !unit)) {
+      StageItem ph = it;
+      ph.diag = true;
+      ph.f.a = o.a;
+      ph.f.b = o.b;
+      ph.f.k = 2;
+      ph.f.negs = unit ? 0 : ops[it.src].nrows;
+      ph.f.ones = unit ? 15 : (uint8_t)(o.urows & 15 & ~ph.f.negs);
+      for (int r = 0; r < 4; ++r) ph.f.mat[r] = o.mat + r;
+      if (o.perm == kPermIdentity2) {
+        out.push_back(ph);
+        continue;
+      }
+      it.od.flags |= OPF_UNIT_PHASE;   // the permutation alone, then its phases by output row
+      it.od.urows = 15;
+      out.push_back(it);
+      ph.primary = false;
+      out.push_back(ph);
+      continue;
+    } else if (o.kind == OP_GRAD2 && o.perm == 2 && o.a == 0) {
+      it.diag = it.term = true;
+      it.f.a = o.b;
+      it.f.k = 1;
+      it.f.ones = o.flags == GRAD_PHASE ? 1 : 0;
+      it.f.mat[0] = o.mat;
+      it.f.mat[1] = o.mat + 3;
+    }
+    out.push_back(it);
+  }
+}
+
+}  // namespace
+
+// What it saves: FP64 work.  A phase costs 2 multiply-adds per amplitude, the
+// |11> phase of a carried CX 1, a CZ 1, a Z step 4; merged over a stage's four
+// slots they cost at most 4 x 15/16 together, CZ signs nothing, and the Z terms
+// share one product per (psi, lambda) pair.  30-qubit brick-wall of depth 20:
+// 2688 -> 1938 multiply-adds per amplitude, 325 -> 306 ms; 28-qubit gradient:
+// forward 898 -> 582, backward 1512 -> 1069, 177 -> 172 ms.
+void merge_stage_diagonals(std::vector<PassPlan>& plans, const std::vector<SchedOp>& ops) {
+  for (PassPlan& pl : plans) {
+    PassDesc& d = pl.desc;
+    if (d.R > 4) continue;
+    const int NV = 1 << d.R;
+    std::vector<OpDesc> nops;
+    std::vector<uint32_t> nsrc, nterm;
+    std::vector<std::vector<DiagFactor>> diag;
+    std::vector<std::pair<uint16_t, uint16_t>> range(d.nstages);
+    for (int s = 0; s < d.nstages; ++s) {
+      std::vector<StageItem> items;
+      stage_items(pl, d.st[s], ops, items);
+      range[s].first = (uint16_t)nops.size();
+      auto emit = [&](const OpDesc& o) {
+        nops.push_back(o);
+        if (o.kind == OP_GRAD2) {   // gradient rows are numbered in the order the operations run
+          nops.back().gidx = (uint32_t)nterm.size();
+          nterm.push_back(d.grad_term[o.gidx]);
+        }
+      };
+      size_t left = items.size();
+      std::vector<uint8_t> done(items.size(), 0);
+      while (left) {
+        // everything that is not a diagonal and waits for nothing before it
+        bool progress = true;
+        while (progress) {
+          progress = false;
+          uint32_t before = 0;
+          for (size_t i = 0; i < items.size(); ++i) {
+            if (done[i]) continue;
+            if (!items[i].diag && !(items[i].mask & before)) {
+              emit(items[i].od);
+              nsrc.push_back(items[i].src);
+              done[i] = 1;
+              --left;
+              progress = true;
+            } else {
+              before |= items[i].mask;
+            }
+          }
+        }
+        // then every diagonal with only diagonals before it on its slots
+        std::vector<int> group;
+        uint32_t blocked = 0;
+        for (size_t i = 0; i < items.size(); ++i) {
+          if (done[i]) continue;
+          if (!items[i].diag) blocked |= items[i].mask;
+          else if (!(items[i].mask & blocked)) group.push_back((int)i);
+        }
+        if (group.empty()) break;   // left == 0: the first item left waits for nothing
+        for (int i : group) {
+          done[i] = 1;
+          --left;
+        }
+        if (group.size() == 1 && items[group[0]].primary && !items[group[0]].f.negs) {
+          emit(items[group[0]].od);
+          nsrc.push_back(items[group[0]].src);
+          continue;
+        }
+        // gradient terms first (one OP_GDZ takes each slot once), then the phases
+        std::vector<int> terms;
+        for (int i : group)
+          if (items[i].term) terms.push_back(i);
+        while (!terms.empty()) {
+          int by_slot[kMaxK] = {-1, -1, -1, -1, -1};
+          std::vector<int> later;
+          for (int i : terms) {
+            if (by_slot[items[i].f.a] < 0) by_slot[items[i].f.a] = i;
+            else later.push_back(i);
+          }
+          OpDesc g{};
+          g.kind = OP_GDZ;
+          g.k = 1;
+          g.gidx = (uint32_t)nterm.size();
+          for (int sl = 0; sl < kMaxK; ++sl)
+            if (by_slot[sl] >= 0) {
+              g.flags |= (uint8_t)(1u << sl);
+              nterm.push_back(d.grad_term[items[by_slot[sl]].od.gidx]);
+              nsrc.push_back(items[by_slot[sl]].src);
+            }
+          nops.push_back(g);
+          terms.swap(later);
+        }
+        OpDesc m{};
+        m.kind = OP_DGR;
+        m.k = 1;
+        m.mat = (uint32_t)diag.size();
+        std::vector<DiagFactor> fs;
+        for (int i : group) {
+          fs.push_back(items[i].f);
+          m.flags |= (uint8_t)((1u << items[i].f.a) | (items[i].f.k == 2 ? 1u << items[i].f.b : 0u));
+          if (items[i].primary && !items[i].term) nsrc.push_back(items[i].src);
+        }
+        m.gidx = diag_units(fs, NV);
+        if ((m.gidx & 0xFFFFu) == (1u << NV) - 1u) continue;   // the identity
+        nops.push_back(m);
+        diag.push_back(fs);
+      }
+      range[s].second = (uint16_t)nops.size();
+    }
+    size_t elems = 0;
+    for (const OpDesc& o : nops) elems += pack_elems(o, d.R);
+    if (nops.size() > (size_t)kMaxPassOps || elems > (size_t)kSmemMatElems) continue;
+    std::copy(nops.begin(), nops.end(), d.ops);
+    d.nops = (uint32_t)nops.size();
+    for (int s = 0; s < d.nstages; ++s) {
+      d.st[s].op0 = range[s].first;
+      d.st[s].op1 = range[s].second;
+    }
+    std::copy(nterm.begin(), nterm.end(), d.grad_term);
+    pl.src = nsrc;
+    pl.diag = diag;
+  }
+}
+
+void pack_recipe(std::vector<PassPlan>& plans, PackRecipe& r) {
+  r.base.clear();
+  r.mults.clear();
   for (auto& pl : plans) {
     PassDesc& d = pl.desc;
-    const uint32_t base = (uint32_t)packed.size();
+    const uint32_t base = (uint32_t)r.base.size();
     for (uint32_t i = 0; i < d.nops; ++i) {
       OpDesc& od = d.ops[i];
-      const bool mono = od.kind == OP_M1R || od.kind == OP_M1L || od.kind == OP_M2R;
-      const uint32_t n = od.kind == OP_GRAD2 ? 4u : (mono ? (1u << od.k) : (1u << (2 * od.k)));
-      const uint32_t rel = (uint32_t)packed.size() - base;
-      packed.insert(packed.end(), pool + od.mat, pool + od.mat + n);
+      const uint32_t rel = (uint32_t)r.base.size() - base;
+      if (od.kind == OP_DGR) {
+        for (int v = 0; v < (1 << d.R); ++v) {
+          const uint32_t at = (uint32_t)r.base.size();
+          bool first = true, neg = false;
+          r.base.push_back(kPackOne);
+          for (const DiagFactor& f : pl.diag[od.mat]) {
+            const int row = ((v >> f.a) & 1) | (f.k == 2 ? ((v >> f.b) & 1) << 1 : 0);
+            if ((f.ones >> row) & 1) continue;
+            if ((f.negs >> row) & 1) { neg = !neg; continue; }
+            if (first) r.base[at] = f.mat[row];
+            else r.mults.push_back({at, f.mat[row]});
+            first = false;
+          }
+          if (neg) {
+            if (!first) r.mults.push_back({at, kPackMinusOne});
+            else r.base[at] = kPackMinusOne;
+          }
+        }
+      } else {
+        const uint32_t n = pack_elems(od, d.R);
+        for (uint32_t e = 0; e < n; ++e) r.base.push_back(od.mat + e);
+      }
       od.mat = rel;
     }
     d.mat_base = base;
-    d.mat_elems = (uint32_t)packed.size() - base;
+    d.mat_elems = (uint32_t)r.base.size() - base;
   }
+}
+
+void PackRecipe::fill(const cplx64* pool, cplx64* dst) const {
+  auto at = [&](uint32_t i) {
+    return i == kPackOne ? cplx64{1.0, 0.0} : (i == kPackMinusOne ? cplx64{-1.0, 0.0} : pool[i]);
+  };
+  for (size_t i = 0; i < base.size(); ++i) dst[i] = at(base[i]);
+  for (const auto& m : mults) dst[m.first] = cm(dst[m.first], at(m.second));
+}
+
+void pack_pass_matrices(std::vector<PassPlan>& plans, const cplx64* pool, std::vector<cplx64>& packed) {
+  PackRecipe r;
+  pack_recipe(plans, r);
+  packed.resize(r.base.size());
+  r.fill(pool, packed.data());
 }
 
 }  // namespace iqb

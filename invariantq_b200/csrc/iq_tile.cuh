@@ -488,6 +488,22 @@ __device__ __forceinline__ bool apply_op(const OpDesc& od, const double2 (&s)[1 
       grad_accumulate(acc, sgrad + od.gidx, lane8, omask);
       break;
     }
+    case OP_DGR:
+#pragma unroll
+      for (int v = 0; v < (1 << R); ++v) d[v] = cmul(ld_mat(m, v), s[v]);
+      break;
+    case OP_GDZ: {
+      double w[1 << (R - 1)];
+#pragma unroll
+      for (int v = 0; v < (1 << R); ++v) d[v] = s[v];
+#pragma unroll
+      for (int v = 0; v < (1 << (R - 1)); ++v) w[v] = z_product(s[2 * v], s[2 * v + 1]);
+      int at = 0;
+#pragma unroll
+      for (int b = 1; b < R; ++b)
+        if ((od.flags >> b) & 1) grad_accumulate(z_sum(w, b - 1), sgrad + od.gidx + at++, lane8, omask);
+      break;
+    }
     case OP_D1R: disp_d1r<R>(od.a, s, d, m, od.flags & OPF_REAL); break;
     case OP_N1R: disp_n1r<R>(od.a, od.perm, s, d, m); break;
     case OP_R1R: disp_r1r<R>(od.a, od.perm, s, d, m); break;
