@@ -466,9 +466,13 @@ __device__ __forceinline__ void set_tile_pass(const CUtensorMap& tm, const PassD
                                               int* status, int nbuf, double* grad_partials, unsigned char* smem_raw,
                                               Stages& stages);
 
-// 1024-byte aligned start of the dynamic shared memory (the tile buffers)
+// 1024-byte aligned start of the dynamic shared memory (the tile buffers).
+// An offset from smem_raw, not a rounded address: the compiler then still
+// knows the pointer as shared memory and the stages use shared loads and
+// stores, not generic ones, whose latency showed as the passes' first stall
+// (30 qubits, depth 20: 306 -> 291 ms; 28-qubit gradient 172 -> 164 ms).
 __device__ __forceinline__ double2* aligned_tiles(unsigned char* smem_raw) {
-  return reinterpret_cast<double2*>((reinterpret_cast<unsigned long long>(smem_raw) + 1023ull) & ~1023ull);
+  return reinterpret_cast<double2*>(smem_raw + ((0u - smem_u32(smem_raw)) & 1023u));
 }
 
 template <int NT, class Stages>
