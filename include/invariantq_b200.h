@@ -294,8 +294,10 @@ int iq_adjoint_gradient_c64(size_t num_qubits, size_t num_ops, const int* kinds,
  * kept for later calls unless they hold more than 8 GiB of device memory.
  * Returns 0, or -1 with iq_last_error set. */
 int iq_adjoint_gradient_batch(const iq_adjoint_circuit* circuits, size_t num_circuits, int num_streams);
-/* Free the device and pinned host memory the adjoint calls keep between calls;
- * returns the number of workspaces freed. */
+/* Free the device and pinned host memory the adjoint calls keep between calls
+ * (and what freed state-vector and density-matrix handles left for the next
+ * ones: at most four sets of streams and buffers, ~45 MiB of device memory
+ * each); returns the number of adjoint workspaces freed. */
 int iq_adjoint_release(void);
 /* Energies only (grad_out unused): the forward circuit and <psi|H|psi> for each
  * parameter set of one circuit, one set after another on one stream -- the

@@ -1275,6 +1275,7 @@ int iq_ansatz_energy(const iq_adjoint_circuit* circuit) { return run_circuits(ci
 
 int iq_adjoint_release(void) {
   resident_release();
+  release_handle_resources();
   std::vector<Workspace*> ws;
   {
     std::lock_guard<std::mutex> g(g_pool_mu);

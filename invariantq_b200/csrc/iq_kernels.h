@@ -174,6 +174,8 @@ size_t count_work_bytes(uint64_t shots);
 cudaError_t count_outcomes(const uint64_t* d_shots, uint64_t shots, void* work, uint64_t* d_vals, uint64_t* d_cnts,
                            uint64_t* d_nuniq, cudaStream_t st);
 
+// Free the streams and buffers that freed handles left for the next ones (iq_runtime.cu).
+void release_handle_resources();
 // Record an error for iq_last_error (defined in iq_runtime.cu).
 void record_error(int code, const char* msg);
 // Add to the iq_kernel_launches counter (defined in iq_runtime.cu).

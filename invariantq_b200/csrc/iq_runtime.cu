@@ -172,34 +172,173 @@ void jit_note(const std::string& why) {
 
 // ---------------------------------------------------------------- engine
 
-constexpr size_t kStageBytes = 64ull << 20;   // device/host staging for readbacks
+// Everything a handle works with besides its state: stream, events, small
+// device and pinned buffers, readback staging and scratch space, grown on
+// demand.  Creating and freeing these cost a circuit of a few qubits ~40 ms of
+// its ~45 (64 MiB of pinned staging first), so a freed handle leaves them to
+// the next one: at most kKeepHandles sets per process, each holding at most
+// ~45 MiB of device and ~12 MiB of pinned memory; iq_adjoint_release frees them.
+constexpr size_t kStageHalf = 4ull << 20;      // readbacks move in chunks of this size, two in flight
+constexpr size_t kSmallState = 1ull << 20;     // states up to this size live in a kept buffer
+constexpr size_t kKeepHandles = 4;
+constexpr size_t kKeepWork = 32ull << 20;
+constexpr size_t kKeepPool = 4ull << 20;
 
-struct Engine {
-  int kind = 0;            // 0 = state vector, 1 = density matrix
-  int nq = 0;              // qubits
-  int nbits = 0;           // index bits (SV: nq, DM: 2 nq)
-  uint64_t dim = 1;
+struct HandleRes {
   int device = 0;
-  int num_sms = 148;
-  double2* d_state = nullptr;
+  unsigned long long ctx = 0;        // the CUDA context all of it belongs to
   cudaStream_t stream = nullptr;
-
-  std::vector<SchedOp> ops;
-  std::vector<cplx64> pool;          // matrices of the queued ops (dense, plus phases of monomials)
-
   double2* d_pool = nullptr;
   size_t d_pool_cap = 0;
   double2* h_pool = nullptr;
   size_t h_pool_cap = 0;
   cudaEvent_t pool_ev = nullptr;
   bool pool_ev_recorded = false;
-
   double* d_scratch = nullptr;       // reduction partials and small results
   size_t scratch_bytes = 0;
   int* d_status = nullptr;
   double* h_small = nullptr;         // pinned small readback area
-  void* d_stage = nullptr;
-  void* h_stage = nullptr;
+  char* d_stage = nullptr;           // two halves of stage_cap bytes each
+  char* h_stage = nullptr;
+  size_t stage_cap = 0;
+  cudaEvent_t stage_ev[2] = {nullptr, nullptr};
+  char* d_work = nullptr;            // scratch space of sampling and entropies
+  size_t work_cap = 0;
+  double2* d_small = nullptr;        // kSmallState bytes
+
+  bool create(int dev) {
+    device = dev;
+    // the largest partials of any handle (34 index bits), so that a set serves every size
+    scratch_bytes = std::max<size_t>({zsums_partials_doubles(34) * 8, (size_t)kRedBlocks * 16, kHamPartials * 16}) + 4096;
+    return cuda_ok(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "cudaStreamCreate") &&
+           cuda_ok(cudaMalloc(&d_scratch, scratch_bytes), "cudaMalloc scratch") &&
+           cuda_ok(cudaMalloc(&d_status, sizeof(int)), "cudaMalloc status") &&
+           cuda_ok(cudaMallocHost(&h_small, 64 * 1024), "cudaMallocHost") &&
+           cuda_ok(cudaEventCreateWithFlags(&pool_ev, cudaEventDisableTiming), "cudaEventCreate") &&
+           cuda_ok(cudaEventCreateWithFlags(&stage_ev[0], cudaEventDisableTiming), "cudaEventCreate") &&
+           cuda_ok(cudaEventCreateWithFlags(&stage_ev[1], cudaEventDisableTiming), "cudaEventCreate");
+  }
+  void free_stage() {
+    if (d_stage) cudaFree(d_stage);
+    if (h_stage) cudaFreeHost(h_stage);
+    d_stage = h_stage = nullptr;
+    stage_cap = 0;
+  }
+  void free_work() {
+    if (d_work) cudaFree(d_work);
+    d_work = nullptr;
+    work_cap = 0;
+  }
+  void free_pool() {
+    if (d_pool) cudaFree(d_pool);
+    if (h_pool) cudaFreeHost(h_pool);
+    d_pool = h_pool = nullptr;
+    d_pool_cap = h_pool_cap = 0;
+  }
+  void destroy() {
+    free_stage();
+    free_work();
+    free_pool();
+    if (d_small) cudaFree(d_small);
+    if (d_scratch) cudaFree(d_scratch);
+    if (d_status) cudaFree(d_status);
+    if (h_small) cudaFreeHost(h_small);
+    for (cudaEvent_t e : {pool_ev, stage_ev[0], stage_ev[1]})
+      if (e) cudaEventDestroy(e);
+    if (stream) cudaStreamDestroy(stream);
+    *this = HandleRes{};
+  }
+  // at least `bytes` of scratch space (contents undefined); the stream's earlier users of it are done or ordered before
+  char* work(size_t bytes) {
+    if (bytes > work_cap) {
+      if (d_work) cudaStreamSynchronize(stream);
+      free_work();
+      if (!cuda_ok(cudaSetDevice(device), "cudaSetDevice") ||
+          !cuda_ok(cudaMalloc(&d_work, bytes), "cudaMalloc work space")) {
+        cudaGetLastError();
+        d_work = nullptr;
+        return nullptr;
+      }
+      work_cap = bytes;
+    }
+    return d_work;
+  }
+  // room for `bytes` of a readback's chunk (at most kStageHalf) in each half
+  bool ensure_stage(size_t bytes) {
+    if (bytes <= stage_cap) return true;
+    if (d_stage) cudaStreamSynchronize(stream);
+    free_stage();
+    if (!cuda_ok(cudaSetDevice(device), "cudaSetDevice") ||
+        !cuda_ok(cudaMalloc(&d_stage, 2 * bytes), "cudaMalloc staging") ||
+        !cuda_ok(cudaMallocHost(&h_stage, 2 * bytes), "cudaMallocHost staging")) {
+      cudaGetLastError();
+      free_stage();
+      return false;
+    }
+    stage_cap = bytes;
+    return true;
+  }
+};
+
+// id of the current CUDA context: sets of a context that was reset are not reused
+unsigned long long context_id() {
+  using Fn = CUresult (*)(CUcontext, unsigned long long*);
+  static const Fn fn = [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+      p = nullptr;
+    return reinterpret_cast<Fn>(p);
+  }();
+  unsigned long long id = 0;
+  if (!fn || fn(nullptr, &id) != CUDA_SUCCESS) return 0;
+  return id;
+}
+
+std::mutex g_res_mu;
+std::vector<HandleRes>* g_res = new std::vector<HandleRes>();   // never destroyed: handles may outlive static objects
+
+bool res_take(int dev, unsigned long long ctx, HandleRes& out) {
+  std::lock_guard<std::mutex> g(g_res_mu);
+  for (size_t i = 0; i < g_res->size(); ++i)
+    if ((*g_res)[i].device == dev && (*g_res)[i].ctx == ctx && ctx) {
+      out = (*g_res)[i];
+      g_res->erase(g_res->begin() + i);
+      return true;
+    }
+  return false;
+}
+
+// the stream is idle and its work succeeded
+void res_give(HandleRes& r) {
+  if (r.work_cap > kKeepWork) r.free_work();
+  if (std::max(r.d_pool_cap, r.h_pool_cap) * sizeof(double2) > kKeepPool) r.free_pool();
+  r.pool_ev_recorded = false;
+  {
+    std::lock_guard<std::mutex> g(g_res_mu);
+    // sets of contexts that are gone: their memory went with the context
+    for (size_t i = g_res->size(); i-- > 0;)
+      if ((*g_res)[i].device == r.device && (*g_res)[i].ctx != r.ctx) g_res->erase(g_res->begin() + i);
+    if (r.ctx && g_res->size() < kKeepHandles) {
+      g_res->push_back(r);
+      r = HandleRes{};
+      return;
+    }
+  }
+  r.destroy();
+}
+
+struct Engine : HandleRes {
+  int kind = 0;            // 0 = state vector, 1 = density matrix
+  int nq = 0;              // qubits
+  int nbits = 0;           // index bits (SV: nq, DM: 2 nq)
+  uint64_t dim = 1;
+  int num_sms = 148;
+  double2* d_state = nullptr;
+
+  std::vector<SchedOp> ops;
+  std::vector<cplx64> pool;          // matrices of the queued ops (dense, plus phases of monomials)
 
   SchedParams sp{};
   TileLaunch tl{};
@@ -271,18 +410,23 @@ struct Engine {
       return false;
     }
     cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, device);
-    if (!cuda_ok(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "cudaStreamCreate")) return false;
-    if (cudaMalloc(&d_state, dim * sizeof(double2)) != cudaSuccess) {
+    if (!cuda_ok(cudaFree(nullptr), "CUDA context")) return false;
+    const unsigned long long id = context_id();
+    const int dev = device;
+    if (!res_take(dev, id, *this)) {
+      if (!create(dev)) return false;
+      ctx = id;
+    }
+    const size_t bytes = dim * sizeof(double2);
+    if (bytes <= kSmallState) {
+      if (!d_small && !cuda_ok(cudaMalloc(&d_small, kSmallState), "cudaMalloc small state")) return false;
+      d_state = d_small;
+    } else if (cudaMalloc(&d_state, bytes) != cudaSuccess) {
       cudaGetLastError();
       set_error(E_MEM, "cannot allocate %.3f GiB of device memory for %d qubits", dim * 16.0 / (1 << 30), nq);
       d_state = nullptr;
       return false;
     }
-    scratch_bytes = std::max<size_t>({zsums_partials_doubles(nbits) * 8, (size_t)kRedBlocks * 16, kHamPartials * 16}) + 4096;
-    if (!cuda_ok(cudaMalloc(&d_scratch, scratch_bytes), "cudaMalloc scratch")) return false;
-    if (!cuda_ok(cudaMalloc(&d_status, sizeof(int)), "cudaMalloc status")) return false;
-    if (!cuda_ok(cudaMallocHost(&h_small, 64 * 1024), "cudaMallocHost")) return false;
-    if (!cuda_ok(cudaEventCreateWithFlags(&pool_ev, cudaEventDisableTiming), "cudaEventCreate")) return false;
     cudaMemsetAsync(d_status, 0, sizeof(int), stream);
     sp.nbits = nbits;
     tl.consumers = 128;
@@ -303,24 +447,17 @@ struct Engine {
   }
 
   void release() {
-    if (stream) cudaStreamSynchronize(stream);
+    const bool ok = stream && cudaStreamSynchronize(stream) == cudaSuccess;
     for (auto& pe : prof) {
       cudaEventDestroy(pe.first);
       cudaEventDestroy(pe.second);
     }
     prof.clear();
-    if (d_state) cudaFree(d_state);
-    if (d_pool) cudaFree(d_pool);
-    if (h_pool) cudaFreeHost(h_pool);
-    if (d_scratch) cudaFree(d_scratch);
-    if (d_status) cudaFree(d_status);
-    if (h_small) cudaFreeHost(h_small);
-    if (d_stage) cudaFree(d_stage);
-    if (h_stage) cudaFreeHost(h_stage);
-    if (pool_ev) cudaEventDestroy(pool_ev);
-    if (stream) cudaStreamDestroy(stream);
+    if (d_state && d_state != d_small) cudaFree(d_state);
     d_state = nullptr;
-    stream = nullptr;
+    HandleRes& r = *this;
+    if (ok) res_give(r);
+    else r.destroy();
   }
 
   bool select() { return cuda_ok(cudaSetDevice(device), "cudaSetDevice"); }
@@ -330,13 +467,6 @@ struct Engine {
     ++st_launches;
     ++g_launches;
     return cuda_ok(launch_set_basis(d_state, dim, stream), "reset");
-  }
-
-  bool ensure_stage() {
-    if (d_stage) return true;
-    if (!cuda_ok(cudaMalloc(&d_stage, kStageBytes), "cudaMalloc staging")) return false;
-    if (!cuda_ok(cudaMallocHost(&h_stage, kStageBytes), "cudaMallocHost staging")) return false;
-    return true;
   }
 
   // -------------------------------------------------------------- queue
@@ -626,22 +756,31 @@ struct Engine {
     return read_doubles(result_slot(), 1, out);
   }
 
-  // copy count elements produced chunk by chunk by `produce(offset, n, dst_device)`
+  // copy `count` elements of each of nout arrays to the host: `produce(offset, n, dst)`
+  // writes elements [offset, offset + n) of every array, one after the other, to
+  // dst on the device.  Two chunks are in flight: while the host copies one out
+  // of the pinned half, the next is produced and transferred.
   template <class F>
   bool chunked_readback(uint64_t count, size_t elem_bytes, int nout, double** outs, F produce) {
-    if (!ensure_stage()) return false;
-    const uint64_t per = kStageBytes / (elem_bytes * nout);
-    for (uint64_t off = 0; off < count; off += per) {
-      const uint64_t n = std::min<uint64_t>(per, count - off);
-      if (!produce(off, n)) return false;
-      for (int j = 0; j < nout; ++j) {
-        if (!cuda_ok(cudaMemcpyAsync(h_stage, reinterpret_cast<char*>(d_stage) + (size_t)j * n * elem_bytes,
-                                     n * elem_bytes, cudaMemcpyDeviceToHost, stream),
-                     "D2H"))
+    const size_t row = elem_bytes * nout;
+    const uint64_t per = std::min<uint64_t>(kStageHalf / row, count);
+    if (!ensure_stage(per * row)) return false;
+    const uint64_t chunks = (count + per - 1) / per;
+    auto len = [&](uint64_t i) { return std::min<uint64_t>(per, count - i * per); };
+    for (uint64_t i = 0; i <= chunks; ++i) {
+      if (i < chunks) {
+        char* const d = d_stage + (i & 1) * stage_cap;
+        if (!produce(i * per, len(i), d)) return false;
+        if (!cuda_ok(cudaMemcpyAsync(h_stage + (i & 1) * stage_cap, d, len(i) * row, cudaMemcpyDeviceToHost, stream),
+                     "D2H") ||
+            !cuda_ok(cudaEventRecord(stage_ev[i & 1], stream), "event"))
           return false;
-        if (!cuda_ok(cudaStreamSynchronize(stream), "stream sync")) return false;
-        memcpy(outs[j] + off, h_stage, n * elem_bytes);
       }
+      if (i == 0) continue;
+      const uint64_t k = i - 1;
+      if (!cuda_ok(cudaEventSynchronize(stage_ev[k & 1]), "stream sync")) return false;
+      for (int j = 0; j < nout; ++j)
+        memcpy(outs[j] + k * per, h_stage + (k & 1) * stage_cap + (size_t)j * len(k) * elem_bytes, len(k) * elem_bytes);
     }
     return true;
   }
@@ -649,8 +788,8 @@ struct Engine {
   bool get_split(double* re, double* im) {
     if (!sync()) return false;
     double* outs[2] = {re, im};
-    return chunked_readback(dim, sizeof(double), 2, outs, [&](uint64_t off, uint64_t n) {
-      double* dre = reinterpret_cast<double*>(d_stage);
+    return chunked_readback(dim, sizeof(double), 2, outs, [&](uint64_t off, uint64_t n, char* dst) {
+      double* dre = reinterpret_cast<double*>(dst);
       ++g_launches;
       ++st_launches;
       return cuda_ok(launch_split(d_state + off, n, dre, dre + n, stream), "split kernel");
@@ -660,10 +799,10 @@ struct Engine {
   bool get_probs(double* out) {
     if (!sync()) return false;
     double* outs[1] = {out};
-    return chunked_readback(dim, sizeof(double), 1, outs, [&](uint64_t off, uint64_t n) {
+    return chunked_readback(dim, sizeof(double), 1, outs, [&](uint64_t off, uint64_t n, char* dst) {
       ++g_launches;
       ++st_launches;
-      return cuda_ok(launch_probs(d_state + off, n, reinterpret_cast<double*>(d_stage), stream), "probs kernel");
+      return cuda_ok(launch_probs(d_state + off, n, reinterpret_cast<double*>(dst), stream), "probs kernel");
     });
   }
 };
@@ -724,6 +863,19 @@ struct CpuCore {
 
 }  // namespace
 
+void iqb::release_handle_resources() {
+  std::vector<HandleRes> r;
+  {
+    std::lock_guard<std::mutex> g(g_res_mu);
+    r.swap(*g_res);
+  }
+  int dev = 0;
+  const bool back = !r.empty() && cudaGetDevice(&dev) == cudaSuccess;
+  for (HandleRes& x : r) {
+    if (cudaSetDevice(x.device) == cudaSuccess && context_id() == x.ctx) x.destroy();
+  }
+  if (back) cudaSetDevice(dev);
+}
 void iqb::record_error(int code, const char* msg) { set_error(code, "%s", msg); }
 void iqb::count_launches(uint64_t n) { g_launches += n; }
 
@@ -903,15 +1055,13 @@ void iq_statevector_sample(void* sv, size_t num_shots, uint64_t seed, uint64_t* 
   // everything on the device (iq_sampling.cu): block sums, their prefix, the
   // mt19937_64 stream (statevector.cpp:244-245), per-shot search
   const size_t wbytes = sample_work_bytes(e->nbits, num_shots);
-  void* dbuf = nullptr;
-  if (!cuda_ok(cudaMallocAsync(&dbuf, wbytes + num_shots * 8 + 256, e->stream), "cudaMallocAsync sampling")) return;
-  uint64_t* d_out = reinterpret_cast<uint64_t*>(static_cast<char*>(dbuf) + ((wbytes + 255) & ~(size_t)255));
+  char* dbuf = e->work(wbytes + num_shots * 8 + 256);
+  if (!dbuf) return;
+  uint64_t* d_out = reinterpret_cast<uint64_t*>(dbuf + ((wbytes + 255) & ~(size_t)255));
   ++e->st_launches;
   cuda_ok(sample_on_device(e->d_state, e->nbits, num_shots, seed, dbuf, d_out, e->stream), "sampling") &&
       cuda_ok(cudaMemcpyAsync(results_out, d_out, num_shots * 8, cudaMemcpyDeviceToHost, e->stream), "D2H") &&
       cuda_ok(cudaStreamSynchronize(e->stream), "sync");
-  cudaFreeAsync(dbuf, e->stream);
-  cudaStreamSynchronize(e->stream);
 }
 
 int iq_statevector_sample_counts(void* sv, size_t num_shots, uint64_t seed, uint64_t* values_out,
@@ -927,10 +1077,8 @@ int iq_statevector_sample_counts(void* sv, size_t num_shots, uint64_t seed, uint
   }
   const size_t wbytes = (std::max(sample_work_bytes(e->nbits, num_shots), count_work_bytes(num_shots)) + 255) & ~(size_t)255;
   const size_t obytes = (num_shots * 8 + 255) & ~(size_t)255;
-  char* dbuf = nullptr;
-  if (!cuda_ok(cudaMallocAsync(reinterpret_cast<void**>(&dbuf), wbytes + 3 * obytes + 256, e->stream),
-               "cudaMallocAsync sampling"))
-    return -1;
+  char* dbuf = e->work(wbytes + 3 * obytes + 256);
+  if (!dbuf) return -1;
   uint64_t* d_shots = reinterpret_cast<uint64_t*>(dbuf + wbytes);
   uint64_t* d_vals = reinterpret_cast<uint64_t*>(dbuf + wbytes + obytes);
   uint64_t* d_cnts = reinterpret_cast<uint64_t*>(dbuf + wbytes + 2 * obytes);
@@ -944,8 +1092,6 @@ int iq_statevector_sample_counts(void* sv, size_t num_shots, uint64_t seed, uint
     ok = cuda_ok(cudaMemcpyAsync(values_out, d_vals, nu * 8, cudaMemcpyDeviceToHost, e->stream), "D2H") &&
          cuda_ok(cudaMemcpyAsync(counts_out, d_cnts, nu * 8, cudaMemcpyDeviceToHost, e->stream), "D2H") &&
          cuda_ok(cudaStreamSynchronize(e->stream), "sync");
-  cudaFreeAsync(dbuf, e->stream);
-  cudaStreamSynchronize(e->stream);
   if (!ok) return -1;
   *num_unique = (size_t)nu;
   return 0;
@@ -1008,8 +1154,8 @@ double iq_statevector_entropy(void* sv, const size_t* qubits, size_t num_subsys_
     return entropy_from(w);
   }
   const size_t kd = (size_t)1 << kk;
-  double2* d_rho = nullptr;
-  if (!cuda_ok(cudaMallocAsync(&d_rho, kd * kd * sizeof(double2), e->stream), "cudaMallocAsync")) return kNaN;
+  double2* d_rho = reinterpret_cast<double2*>(e->work(kd * kd * sizeof(double2)));
+  if (!d_rho) return kNaN;
   std::vector<cd> rho(kd * kd);
   ++g_launches;
   ++e->st_launches;
@@ -1017,7 +1163,6 @@ double iq_statevector_entropy(void* sv, const size_t* qubits, size_t num_subsys_
             cuda_ok(cudaMemcpyAsync(rho.data(), d_rho, kd * kd * sizeof(double2), cudaMemcpyDeviceToHost, e->stream),
                     "D2H") &&
             cuda_ok(cudaStreamSynchronize(e->stream), "sync");
-  cudaFreeAsync(d_rho, e->stream);
   if (!ok) return kNaN;
   std::vector<double> w;
   if (!hermitian_eigenvalues(rho, (int)kd, w)) {
@@ -1179,14 +1324,17 @@ int iq_statevector_set_amplitudes(void* sv, const double* real_in, const double*
   if (!e || !real_in || !imag_in) return -1;
   if (!e->select()) return -1;
   e->clear_queue();
-  if (!e->ensure_stage()) return -1;
-  const uint64_t per = kStageBytes / 16;
-  for (uint64_t off = 0; off < e->dim; off += per) {
+  const uint64_t per = std::min<uint64_t>(kStageHalf / 16, e->dim);
+  if (!e->ensure_stage(per * 16)) return -1;
+  for (uint64_t off = 0, i = 0; off < e->dim; off += per, ++i) {
     const uint64_t n = std::min<uint64_t>(per, e->dim - off);
-    double2* h = reinterpret_cast<double2*>(e->h_stage);
-    if (!cuda_ok(cudaStreamSynchronize(e->stream), "sync")) return -1;
-    for (uint64_t i = 0; i < n; ++i) h[i] = make_double2(real_in[off + i], imag_in[off + i]);
-    if (!cuda_ok(cudaMemcpyAsync(e->d_state + off, h, n * 16, cudaMemcpyHostToDevice, e->stream), "H2D")) return -1;
+    double2* h = reinterpret_cast<double2*>(e->h_stage + (i & 1) * e->stage_cap);
+    // the half's previous copy has left it
+    if (i >= 2 && !cuda_ok(cudaEventSynchronize(e->stage_ev[i & 1]), "sync")) return -1;
+    for (uint64_t j = 0; j < n; ++j) h[j] = make_double2(real_in[off + j], imag_in[off + j]);
+    if (!cuda_ok(cudaMemcpyAsync(e->d_state + off, h, n * 16, cudaMemcpyHostToDevice, e->stream), "H2D") ||
+        !cuda_ok(cudaEventRecord(e->stage_ev[i & 1], e->stream), "event"))
+      return -1;
   }
   return cuda_ok(cudaStreamSynchronize(e->stream), "sync") ? 0 : -1;
 }
