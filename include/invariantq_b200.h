@@ -296,7 +296,7 @@ int iq_adjoint_gradient_c64(size_t num_qubits, size_t num_ops, const int* kinds,
 int iq_adjoint_gradient_batch(const iq_adjoint_circuit* circuits, size_t num_circuits, int num_streams);
 /* Free the device and pinned host memory the adjoint calls keep between calls
  * (and what freed state-vector and density-matrix handles left for the next
- * ones: at most four sets of streams and buffers, ~45 MiB of device memory
+ * ones: at most four sets of streams and buffers, ~80 MiB of device memory
  * each); returns the number of adjoint workspaces freed. */
 int iq_adjoint_release(void);
 /* Energies only (grad_out unused): the forward circuit and <psi|H|psi> for each

@@ -153,10 +153,12 @@ cudaError_t launch_init_joint_c64(float2* s, int n, uint64_t jdim, int nsets, cu
 cudaError_t launch_row_sums(const double* in, int rows, int cols, double* out, cudaStream_t st);
 
 // Eigenvalues (ascending) of the reduced state on the kept qubits keep[0..k) of
-// the 2^nbits state psi, computed on the device (iq_entropy.cu); k is at most
-// reduced_spectrum_max_bits() and below nbits.  Synchronises `st`.
+// the 2^nbits state psi, computed on the device (iq_entropy.cu); 7 <= k <=
+// reduced_spectrum_max_bits(), k < nbits.  work: reduced_spectrum_bytes(nbits, k)
+// bytes of device memory, 256-byte aligned.  Synchronises `st`.
 int reduced_spectrum_max_bits();
-cudaError_t reduced_spectrum(const double2* psi, int nbits, const int* keep, int k, std::vector<double>& eig,
+size_t reduced_spectrum_bytes(int nbits, int k);
+cudaError_t reduced_spectrum(const double2* psi, int nbits, const int* keep, int k, std::vector<double>& eig, void* work,
                              cudaStream_t st);
 
 // Measurement shots on the device (iq_sampling.cu): `shots` outcome indices

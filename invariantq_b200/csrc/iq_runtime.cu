@@ -177,11 +177,11 @@ void jit_note(const std::string& why) {
 // demand.  Creating and freeing these cost a circuit of a few qubits ~40 ms of
 // its ~45 (64 MiB of pinned staging first), so a freed handle leaves them to
 // the next one: at most kKeepHandles sets per process, each holding at most
-// ~45 MiB of device and ~12 MiB of pinned memory; iq_adjoint_release frees them.
+// ~80 MiB of device and ~12 MiB of pinned memory; iq_adjoint_release frees them.
 constexpr size_t kStageHalf = 4ull << 20;      // readbacks move in chunks of this size, two in flight
 constexpr size_t kSmallState = 1ull << 20;     // states up to this size live in a kept buffer
 constexpr size_t kKeepHandles = 4;
-constexpr size_t kKeepWork = 32ull << 20;
+constexpr size_t kKeepWork = 64ull << 20;
 constexpr size_t kKeepPool = 4ull << 20;
 
 struct HandleRes {
@@ -1150,8 +1150,21 @@ double iq_statevector_entropy(void* sv, const size_t* qubits, size_t num_subsys_
   if (kk >= 7) {
     // reduced state, tridiagonalisation and eigenvalues on the device (iq_entropy.cu)
     std::vector<double> w;
-    if (!cuda_ok(reduced_spectrum(e->d_state, n, keep.data(), kk, w, e->stream), "reduced spectrum")) return kNaN;
-    return entropy_from(w);
+    const size_t bytes = reduced_spectrum_bytes(n, kk);
+    void* buf = nullptr;
+    const bool kept = bytes <= kKeepWork;   // larger than that (from 11 qubits): for this call only
+    if (kept) {
+      buf = e->work(bytes);
+      if (!buf) return kNaN;
+    } else if (!cuda_ok(cudaMallocAsync(&buf, bytes, e->stream), "cudaMallocAsync entropy")) {
+      return kNaN;
+    }
+    const bool ok = cuda_ok(reduced_spectrum(e->d_state, n, keep.data(), kk, w, buf, e->stream), "reduced spectrum");
+    if (!kept) {
+      cudaFreeAsync(buf, e->stream);
+      cudaStreamSynchronize(e->stream);
+    }
+    return ok ? entropy_from(w) : kNaN;
   }
   const size_t kd = (size_t)1 << kk;
   double2* d_rho = reinterpret_cast<double2*>(e->work(kd * kd * sizeof(double2)));
