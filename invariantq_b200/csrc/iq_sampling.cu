@@ -19,9 +19,9 @@
 //      that round up to 1 replaced by the largest double below 1;
 //   4. per shot a binary search for its block, then the warp search inside
 //      the block (launch_block_search);
-//   5. for counts: the shot indices sorted (bitonic network in global memory,
-//      padded to a power of two), run-length encoded into ascending outcomes
-//      and their counts.
+//   5. for counts: the shot indices sorted (bitonic network, in shared memory
+//      where partners are near, padded to a power of two), run-length encoded
+//      into ascending outcomes and their counts.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -89,26 +89,45 @@ __global__ void __launch_bounds__(kMtM) mt64_uniform_kernel(uint64_t seed, uint6
   }
 }
 
-// One CTA: inclusive prefix of in[0..n) into out (contiguous runs per thread).
+// exclusive prefix of one value per thread over a CTA of 1024 (warp scans, then
+// the warp totals); *total gets the sum
+template <class T>
+__device__ __forceinline__ T block_exclusive(T v, T* warp_tot, T* total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  T inc = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const T u = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += u;
+  }
+  if (lane == 31) warp_tot[warp] = inc;
+  __syncthreads();
+  if (warp == 0) {
+    T w = warp_tot[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const T u = __shfl_up_sync(0xffffffffu, w, o);
+      if (lane >= o) w += u;
+    }
+    warp_tot[lane] = w;
+  }
+  __syncthreads();
+  *total = warp_tot[31];
+  return (warp ? warp_tot[warp - 1] : T(0)) + inc - v;
+}
+
+// One CTA of 1024: inclusive prefix of in[0..n) into out (contiguous runs per
+// thread; the scan of the runs' sums took one thread 1024 steps before: 9.3 ->
+// 3 us for one block).
 __global__ void __launch_bounds__(1024) prefix_kernel(const double* __restrict__ in, uint64_t n, double* __restrict__ out) {
-  __shared__ double tot[1024];
+  __shared__ double warp_tot[32];
   const int t = threadIdx.x, T = blockDim.x;
   const uint64_t per = (n + T - 1) / T;
   const uint64_t b = (uint64_t)t * per, e = (b + per < n) ? b + per : n;
   double s = 0.0;
   for (uint64_t i = b; i < e; ++i) s += in[i];
-  tot[t] = s;
-  __syncthreads();
-  if (t == 0) {
-    double run = 0.0;
-    for (int k = 0; k < T; ++k) {
-      const double v = tot[k];
-      tot[k] = run;
-      run += v;
-    }
-  }
-  __syncthreads();
-  double run = tot[t];
+  double total;
+  double run = block_exclusive(s, warp_tot, &total);
   for (uint64_t i = b; i < e; ++i) {
     run += in[i];
     out[i] = run;
@@ -132,55 +151,140 @@ __global__ void find_block_kernel(const double* __restrict__ incl, uint64_t nblk
   base[k] = lo ? incl[lo - 1] : 0.0;
 }
 
-__global__ void pad_kernel(const uint64_t* __restrict__ in, int n, uint64_t* __restrict__ out, int npow) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < npow) out[i] = i < n ? in[i] : ~0ULL;
+// ---- counts: the shots sorted by a bitonic network, then run-length encoded
+//
+// Launches bound the small cases: one per network step was 91 launches for 8192
+// shots.  Steps whose partners lie within kSortTile run in shared memory, all
+// of them in one launch; up to kSortTile shots the whole count is one launch.
+constexpr int kSortTile = 8192;        // 64 KiB of shared memory, 1024 threads
+
+// network steps j = j0, j0/2, .. 1 of merge size k on the tile's elements (global index base + i)
+__device__ __forceinline__ void tile_steps(uint64_t* s, uint64_t base, int len, uint64_t k, int j0) {
+  for (int j = j0; j > 0; j >>= 1) {
+    for (int q = threadIdx.x; q < len / 2; q += blockDim.x) {
+      const int i = ((q & ~(j - 1)) << 1) | (q & (j - 1)), p = i | j;
+      const uint64_t x = s[i], y = s[p];
+      if ((x > y) == (((base + i) & k) == 0)) {
+        s[i] = y;
+        s[p] = x;
+      }
+    }
+    __syncthreads();
+  }
 }
 
-// one compare-exchange step (k, j) of the bitonic network, ascending
-__global__ void bitonic_step_kernel(uint64_t* __restrict__ a, int npow, int k, int j) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= npow) return;
-  const int p = i ^ j;
-  if (p <= i) return;
+// tiles of in[0..n) (padded with the largest value) sorted, alternating in direction
+__global__ void __launch_bounds__(1024) sort_tiles_kernel(const uint64_t* __restrict__ in, uint64_t n,
+                                                          uint64_t* __restrict__ out) {
+  extern __shared__ uint64_t sort_smem[];
+  const uint64_t base = (uint64_t)blockIdx.x * kSortTile;
+  for (int i = threadIdx.x; i < kSortTile; i += blockDim.x) sort_smem[i] = base + i < n ? in[base + i] : ~0ULL;
+  __syncthreads();
+  for (int k = 2; k <= kSortTile; k <<= 1) tile_steps(sort_smem, base, kSortTile, (uint64_t)k, k >> 1);
+  for (int i = threadIdx.x; i < kSortTile; i += blockDim.x) out[base + i] = sort_smem[i];
+}
+
+// the steps of merge size k > kSortTile whose partners lie within a tile
+__global__ void __launch_bounds__(1024) merge_tiles_kernel(uint64_t* __restrict__ a, uint64_t k) {
+  extern __shared__ uint64_t sort_smem[];
+  const uint64_t base = (uint64_t)blockIdx.x * kSortTile;
+  for (int i = threadIdx.x; i < kSortTile; i += blockDim.x) sort_smem[i] = a[base + i];
+  __syncthreads();
+  tile_steps(sort_smem, base, kSortTile, k, kSortTile >> 1);
+  for (int i = threadIdx.x; i < kSortTile; i += blockDim.x) a[base + i] = sort_smem[i];
+}
+
+// one compare-exchange step (k, j) in global memory, one pair per thread
+__global__ void bitonic_step_kernel(uint64_t* __restrict__ a, uint64_t pairs, uint64_t k, uint64_t j) {
+  const uint64_t q = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  if (q >= pairs) return;
+  const uint64_t i = ((q & ~(j - 1)) << 1) | (q & (j - 1)), p = i | j;
   const uint64_t x = a[i], y = a[p];
-  const bool up = (i & k) == 0;
-  if ((x > y) == up) {
+  if ((x > y) == ((i & k) == 0)) {
     a[i] = y;
     a[p] = x;
   }
 }
 
-// One CTA: run-length encoding of the sorted a[0..n) into ascending outcomes and counts.
-__global__ void __launch_bounds__(1024) rle_kernel(const uint64_t* __restrict__ a, int n, uint64_t* __restrict__ vals,
-                                                   uint64_t* __restrict__ cnts, uint64_t* __restrict__ nuniq) {
-  __shared__ int heads[1024];
-  const int t = threadIdx.x, T = blockDim.x;
-  const int per = (n + T - 1) / T;
-  const int b = t * per, e = (b + per < n) ? b + per : n;
-  int h = 0;
-  for (int i = b; i < e; ++i) h += (i == 0 || a[i] != a[i - 1]);
-  heads[t] = h;
+// a run starts at sorted position i
+__device__ __forceinline__ bool run_head(const uint64_t* a, uint64_t i) { return i == 0 || a[i] != a[i - 1]; }
+
+// One CTA, at most kSortTile shots: sort, run heads, values and counts.
+__global__ void __launch_bounds__(1024) count_small_kernel(const uint64_t* __restrict__ in, int n, int npow,
+                                                           uint64_t* __restrict__ vals, uint64_t* __restrict__ cnts,
+                                                           uint64_t* __restrict__ nuniq) {
+  extern __shared__ uint64_t sort_smem[];
+  uint32_t* const pos = reinterpret_cast<uint32_t*>(sort_smem + npow);   // run heads, then n
+  __shared__ uint32_t warp_tot[32];
+  for (int i = threadIdx.x; i < npow; i += blockDim.x) sort_smem[i] = i < n ? in[i] : ~0ULL;
   __syncthreads();
-  if (t == 0) {
-    int run = 0;
-    for (int k = 0; k < T; ++k) {
-      const int v = heads[k];
-      heads[k] = run;
-      run += v;
+  for (int k = 2; k <= npow; k <<= 1) tile_steps(sort_smem, 0, npow, (uint64_t)k, k >> 1);
+  const int per = (n + 1023) / 1024, b = threadIdx.x * per, e = b + per < n ? b + per : n;
+  uint32_t h = 0, total;
+  for (int i = b; i < e; ++i) h += run_head(sort_smem, i);
+  uint32_t u = block_exclusive(h, warp_tot, &total);
+  for (int i = b; i < e; ++i)
+    if (run_head(sort_smem, i)) {
+      vals[u] = sort_smem[i];
+      pos[u++] = (uint32_t)i;
     }
-    *nuniq = (uint64_t)run;
+  if (threadIdx.x == 0) {
+    pos[total] = (uint32_t)n;
+    *nuniq = total;
   }
   __syncthreads();
-  int u = heads[t];   // index of the first run this thread's range starts
-  for (int i = b; i < e; ++i)
-    if (i == 0 || a[i] != a[i - 1]) {
-      int j = i + 1;
-      while (j < n && a[j] == a[i]) ++j;
-      vals[u] = a[i];
-      cnts[u] = (uint64_t)(j - i);
-      ++u;
-    }
+  for (uint32_t r = threadIdx.x; r < total; r += blockDim.x) cnts[r] = pos[r + 1] - pos[r];
+}
+
+// more shots: heads per block of 1024, their prefix, the heads' positions, the counts
+__global__ void __launch_bounds__(1024) head_count_kernel(const uint64_t* __restrict__ a, uint64_t n,
+                                                          uint32_t* __restrict__ blocks) {
+  const uint64_t i = blockIdx.x * 1024ull + threadIdx.x;
+  const int h = __syncthreads_count(i < n && run_head(a, i));
+  if (threadIdx.x == 0) blocks[blockIdx.x] = (uint32_t)h;
+}
+
+__global__ void __launch_bounds__(1024) head_prefix_kernel(uint32_t* __restrict__ blocks, uint64_t nblk,
+                                                           uint64_t* __restrict__ nuniq) {
+  __shared__ uint32_t warp_tot[32];
+  const uint64_t per = (nblk + 1023) / 1024;
+  const uint64_t b = threadIdx.x * per, e = b + per < nblk ? b + per : nblk;
+  uint32_t s = 0, total;
+  for (uint64_t i = b; i < e; ++i) s += blocks[i];
+  uint32_t run = block_exclusive(s, warp_tot, &total);
+  for (uint64_t i = b; i < e; ++i) {
+    const uint32_t v = blocks[i];
+    blocks[i] = run;
+    run += v;
+  }
+  if (threadIdx.x == 0) *nuniq = total;
+}
+
+__global__ void __launch_bounds__(1024) head_write_kernel(const uint64_t* __restrict__ a, uint64_t n,
+                                                          const uint32_t* __restrict__ blocks,
+                                                          uint64_t* __restrict__ vals, uint32_t* __restrict__ pos) {
+  __shared__ uint32_t warp_tot[32];
+  const uint64_t i = blockIdx.x * 1024ull + threadIdx.x;
+  const bool head = i < n && run_head(a, i);
+  uint32_t total;
+  const uint32_t u = blocks[blockIdx.x] + block_exclusive((uint32_t)head, warp_tot, &total);
+  if (head) {
+    vals[u] = a[i];
+    pos[u] = (uint32_t)i;
+  }
+}
+
+__global__ void run_counts_kernel(const uint32_t* __restrict__ pos, const uint64_t* __restrict__ nuniq, uint64_t n,
+                                  uint64_t* __restrict__ cnts) {
+  const uint64_t runs = *nuniq;
+  for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < runs; r += (uint64_t)gridDim.x * blockDim.x)
+    cnts[r] = (r + 1 < runs ? pos[r + 1] : (uint32_t)n) - pos[r];
+}
+
+uint64_t sort_size(uint64_t shots) {   // power of two; whole tiles above one
+  uint64_t npow = 1;
+  while (npow < shots) npow <<= 1;
+  return npow;
 }
 
 }  // namespace
@@ -218,26 +322,46 @@ size_t sample_work_bytes(int nbits, uint64_t shots) {
 
 cudaError_t count_outcomes(const uint64_t* d_shots, uint64_t shots, void* work, uint64_t* d_vals, uint64_t* d_cnts,
                            uint64_t* d_nuniq, cudaStream_t st) {
-  int npow = 1;
-  while ((uint64_t)npow < shots) npow <<= 1;
+  const uint64_t npow = sort_size(shots);
+  if (npow <= (uint64_t)kSortTile) {
+    const size_t smem = npow * 8 + (shots + 1) * 4;
+    cudaError_t e = cudaFuncSetAttribute(count_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         kSortTile * 8 + (kSortTile + 1) * 4);
+    if (e != cudaSuccess) return e;
+    count_small_kernel<<<1, 1024, smem, st>>>(d_shots, (int)shots, (int)npow, d_vals, d_cnts, d_nuniq);
+    count_launches(1);
+    return cudaGetLastError();
+  }
   uint64_t* a = static_cast<uint64_t*>(work);
-  const unsigned g = (unsigned)((npow + 255) / 256);
-  pad_kernel<<<g, 256, 0, st>>>(d_shots, (int)shots, a, npow);
-  uint64_t launches = 2;
-  for (int k = 2; k <= npow; k <<= 1)
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      bitonic_step_kernel<<<g, 256, 0, st>>>(a, npow, k, j);
+  uint32_t* pos = reinterpret_cast<uint32_t*>(a + npow);
+  uint32_t* blocks = pos + ((shots + 63) & ~(uint64_t)63);
+  const size_t smem = kSortTile * 8;
+  cudaError_t e = cudaFuncSetAttribute(sort_tiles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(merge_tiles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  const unsigned tiles = (unsigned)(npow / kSortTile);
+  sort_tiles_kernel<<<tiles, 1024, smem, st>>>(d_shots, shots, a);
+  uint64_t launches = 1;
+  for (uint64_t k = 2ull * kSortTile; k <= npow; k <<= 1) {
+    for (uint64_t j = k >> 1; j >= (uint64_t)kSortTile; j >>= 1) {
+      bitonic_step_kernel<<<(unsigned)(npow / 2 / 256), 256, 0, st>>>(a, npow / 2, k, j);
       ++launches;
     }
-  rle_kernel<<<1, 1024, 0, st>>>(a, (int)shots, d_vals, d_cnts, d_nuniq);
-  count_launches(launches);
+    merge_tiles_kernel<<<tiles, 1024, smem, st>>>(a, k);
+    ++launches;
+  }
+  const uint64_t nblk = (shots + 1023) / 1024;
+  head_count_kernel<<<(unsigned)nblk, 1024, 0, st>>>(a, shots, blocks);
+  head_prefix_kernel<<<1, 1024, 0, st>>>(blocks, nblk, d_nuniq);
+  head_write_kernel<<<(unsigned)nblk, 1024, 0, st>>>(a, shots, blocks, d_vals, pos);
+  run_counts_kernel<<<(unsigned)std::min<uint64_t>(nblk, 148 * 4), 256, 0, st>>>(pos, d_nuniq, shots, d_cnts);
+  count_launches(launches + 4);
   return cudaGetLastError();
 }
 
 size_t count_work_bytes(uint64_t shots) {
-  uint64_t npow = 1;
-  while (npow < shots) npow <<= 1;
-  return npow * 8 + 256;
+  const uint64_t npow = sort_size(shots);
+  return npow * 8 + ((shots + 63) & ~(uint64_t)63) * 4 + ((shots + 1023) / 1024) * 4 + 256;
 }
 
 }  // namespace iqb
