@@ -70,8 +70,8 @@ struct Cfg {
   // complex64 states: every pass a specialised kernel that widens the loaded
   // amplitudes to FP64 and rounds to FP32 at its stage boundaries (jit_launch_narrow)
   bool c64 = false;
-  // a circuit with one parameter set: forward and backward in the forms that
-  // depend on its angles (fewer FP64 operations; adjoint_ops' single_set)
+  // a circuit with one parameter set: forward and backward in the cheap forms,
+  // in a Pauli frame (adjoint_ops' single_set and framed)
   bool single_forms = true;
   static Cfg from_env() {
     Cfg c;
@@ -260,14 +260,17 @@ struct Circuit {
   std::unique_ptr<Shape> fw, bw;
 };
 
-// fused forward / backward operation lists and matrix pools of one parameter
-// set.  A circuit with a single parameter set takes the angle-dependent forms
-// (rotation + phase forward, scaled adjoint steps: adjoint_ops' single_set):
-// its plans serve no other set.
+// Forward / backward operation lists and matrix pools of one parameter set.  A
+// circuit with a single parameter set takes the cheap forms (rotation + phase
+// forward, tan-form adjoint steps: adjoint_ops' single_set) in the set's Pauli
+// frame, which makes their structure the same for every set of angles: the next
+// call with new angles finds its kernels compiled (the first gradient of 20
+// qubits with new angles took 1.1 s, compiling).
 using JobOps = AdjointOps;
 
 void job_ops(const Cfg& cfg, const Circuit& c, const double* theta, bool backward, JobOps& j) {
-  adjoint_ops(c.n, c.ops, theta, backward, cfg.fuse != 0, cfg.single_forms && c.nsets == 1, j);
+  const bool single = cfg.single_forms && c.nsets == 1;
+  adjoint_ops(c.n, c.ops, theta, backward, cfg.fuse != 0, single, j, single);
 }
 
 int joint_bits(int n) { return std::max(n + 1, 7); }
@@ -576,7 +579,7 @@ bool launch_sets(Workspace& w, const Cfg& cfg, Circuit& c, const std::vector<siz
   if (!finish(w, k, err)) return false;
   const size_t nf = fw->pack.base.size(), nb = want_grad ? bw->pack.base.size() : 0;
   const size_t per = nf + nb;
-  if (!w.hmats[k].ensure(per * S, err) || !w.hout[k].ensure(S + (size_t)S * ngrads, err) || !w.hstat[k].ensure(1, err))
+  if (!w.hmats[k].ensure((per + 1) * S, err) || !w.hout[k].ensure(S + (size_t)S * ngrads, err) || !w.hstat[k].ensure(1, err))
     return false;
   double2* hm = w.hmats[k].p;
   const auto tg = std::chrono::steady_clock::now();
@@ -584,6 +587,8 @@ bool launch_sets(Workspace& w, const Cfg& cfg, Circuit& c, const std::vector<siz
     const JobOps& o = jo[j];
     fw->pack.fill(o.fpool.data(), reinterpret_cast<cplx64*>(hm + (size_t)j * nf));
     if (want_grad) bw->pack.fill(o.bpool.data(), reinterpret_cast<cplx64*>(hm + (size_t)S * nf + (size_t)j * nb));
+    const uint64_t f[2] = {o.frame.x, o.frame.z};   // the sets' frames follow their matrices
+    std::memcpy(hm + per * S + j, f, sizeof(f));
   }
   st.host_ns += (uint64_t)std::chrono::duration_cast<std::chrono::nanoseconds>(std::chrono::steady_clock::now() - tg)
                     .count();
@@ -594,7 +599,7 @@ bool launch_sets(Workspace& w, const Cfg& cfg, Circuit& c, const std::vector<siz
   // tensor maps hold the state buffers' addresses, so they are dropped if one moves
   const double2* psi0 = w.psi.p;
   const double2* joint0 = w.joint.p;
-  if (!w.mats.ensure(2 * per * S, err, "matrices", w.stream) ||
+  if (!w.mats.ensure(2 * (per + 1) * S, err, "matrices", w.stream) ||
       !w.red.ensure((size_t)S * (kHamPartials + 1), err, "reduction partials", w.stream) ||
       (!want_grad && !w.psi.ensure(dim * S, err, "the states", w.stream)))
     return false;
@@ -617,19 +622,20 @@ bool launch_sets(Workspace& w, const Cfg& cfg, Circuit& c, const std::vector<siz
   // matrices go to the half of the device buffer this slot owns, so the copy for
   // the next job cannot overwrite matrices this job's passes still read
   double2* dm = w.mats.p + (size_t)k * (w.mats.cap / 2);
-  if (!cuda_ok(cudaMemcpyAsync(dm, hm, per * S * sizeof(double2), cudaMemcpyHostToDevice, w.stream), "H2D matrices",
+  if (!cuda_ok(cudaMemcpyAsync(dm, hm, (per + 1) * S * sizeof(double2), cudaMemcpyHostToDevice, w.stream), "H2D matrices",
                err))
     return false;
 
   double* partials = w.red.p;
   double* energy_dev = w.red.p + (size_t)S * kHamPartials;
   const HamTables ht = c.ham.plan.tables(w.ham.p);
+  const ulonglong2* frames = reinterpret_cast<const ulonglong2*>(dm + per * S);
   if (!want_grad) {
     // forward from |0> for every set on the state buffer, then the energies
     if (!cuda_ok(launch_set_basis_sets(w.psi.p, dim, (int)S, w.stream), "reset", err)) return false;
     if (!run_shape(w, cfg, *fw, fw_cached, w.psi.p, S, dm, (uint32_t)nf, nullptr, 0, nullptr, st, err)) return false;
     st.fw_passes += (fw->tiled ? fw->plans.size() : fw->sops.size()) * S;
-    if (!cuda_ok(launch_hamiltonian(c.ham.plan, ht, w.psi.p, dim, (int)S, nullptr, 0, partials, energy_dev, nullptr,
+    if (!cuda_ok(launch_hamiltonian(c.ham.plan, ht, frames, w.psi.p, dim, (int)S, nullptr, 0, partials, energy_dev, nullptr,
                                     w.stream),
                  "energy kernel", err))
       return false;
@@ -647,10 +653,10 @@ bool launch_sets(Workspace& w, const Cfg& cfg, Circuit& c, const std::vector<siz
     if (!run_shape(w, cfg, *fw, fw_cached, w.joint.p, S, dm, (uint32_t)nf, nullptr, 0, nullptr, st, err, jdim))
       return false;
     st.fw_passes += (fw->tiled ? fw->plans.size() : fw->sops.size()) * S;
-    if (cfg.c64 ? !cuda_ok(launch_hamiltonian_c64(c.ham.plan, ht, J64, jdim, (int)S, J64 + dim, jdim, partials,
+    if (cfg.c64 ? !cuda_ok(launch_hamiltonian_c64(c.ham.plan, ht, frames, J64, jdim, (int)S, J64 + dim, jdim, partials,
                                                   energy_dev, w.stream),
                            "Hamiltonian kernel", err)
-                : !cuda_ok(launch_hamiltonian(c.ham.plan, ht, w.joint.p, jdim, (int)S, w.joint.p + dim, jdim, partials,
+                : !cuda_ok(launch_hamiltonian(c.ham.plan, ht, frames, w.joint.p, jdim, (int)S, w.joint.p + dim, jdim, partials,
                                               energy_dev, nullptr, w.stream),
                            "Hamiltonian kernel", err))
       return false;
@@ -689,11 +695,14 @@ bool launch_sets(Workspace& w, const Cfg& cfg, Circuit& c, const std::vector<siz
   bool unit_scales = true;
   for (uint32_t j = 0; j < S && want_grad; ++j)
     for (double f : jo[j].grad_scale) unit_scales = unit_scales && f == 1.0;
+  for (uint32_t j = 0; j < S && want_grad; ++j)
+    for (int8_t f : jo[j].grad_sign) unit_scales = unit_scales && f == 1;
   if (!unit_scales)   // scaled adjoint steps: each term's scale in the order the backward passes run them
     for (uint32_t j = 0; j < S; ++j) {
       std::vector<double> sc;
       exec_grad_scales(bw->tiled ? &bw->plans : nullptr, jo[j].bw, sc);
-      if ((int)sc.size() != ngrads) { err = "internal: gradient scales"; return false; }
+      if ((int)sc.size() != ngrads || (int)jo[j].grad_sign.size() != ngrads) { err = "internal: gradient scales"; return false; }
+      for (int t = 0; t < ngrads; ++t) sc[t] *= jo[j].grad_sign[t];   // the frame's sign of the rotation
       p.grad_scale.insert(p.grad_scale.end(), sc.begin(), sc.end());
     }
   st.jobs += S;
@@ -878,7 +887,7 @@ int run_batch(std::vector<std::unique_ptr<Circuit>>& circs, int nstreams, bool w
       if (!want_grad) bd.psi_amps = std::max<uint64_t>(bd.psi_amps, (uint64_t)ns << c->n);
       if (want_grad)
         bd.joint_amps = std::max<uint64_t>(bd.joint_amps, ((uint64_t)ns << joint_bits(c->n)) >> (c64 ? 1 : 0));
-      bd.mats = std::max(bd.mats, ns * 96 * nops);
+      bd.mats = std::max(bd.mats, ns * (96 * nops + 1));
       bd.sets = std::max(bd.sets, ns);
       if (want_grad) bd.grads = std::max(bd.grads, ns * 3 * nops);
     }

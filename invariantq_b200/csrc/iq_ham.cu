@@ -91,9 +91,9 @@ size_t ham_smem_bytes(const HamSweep& s, size_t amp) {
 template <class T>
 __global__ void __launch_bounds__(kHamThreads, 2)
 ham_sweep_kernel(const T* __restrict__ psi, uint64_t pstride, const __grid_constant__ HamSweep P,
-                 const HamItem* __restrict__ g_items, const uint64_t* __restrict__ tz, const double* __restrict__ tc,
-                 T* __restrict__ lam, uint64_t lstride, double* __restrict__ re, double* __restrict__ im,
-                 uint32_t rstride) {
+                 const HamItem* __restrict__ g_items, const uint64_t* __restrict__ tz, const uint64_t* __restrict__ txm,
+                 const double* __restrict__ tc, const ulonglong2* __restrict__ frames, T* __restrict__ lam,
+                 uint64_t lstride, double* __restrict__ re, double* __restrict__ im, uint32_t rstride) {
   extern __shared__ __align__(16) unsigned char ham_smem[];
   T* const tile = reinterpret_cast<T*>(ham_smem);
   const int nterms = ham_smem_terms(P);
@@ -104,6 +104,9 @@ ham_sweep_kernel(const T* __restrict__ psi, uint64_t pstride, const __grid_const
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   psi += blockIdx.y * pstride;
   if (lam) lam += blockIdx.y * lstride;
+  // the set's Pauli frame X^x Z^z: strings that do not commute with it change sign
+  const ulonglong2 frame = frames ? frames[blockIdx.y] : make_ulonglong2(0, 0);
+  auto flips = [&](uint64_t x, int k) { return (__popcll((x ^ frame.x) & tz[k]) + __popcll(txm[k] & frame.y)) & 1; };
   uint64_t tphys = 0;                  // physical bits of the thread's tile-local bits
   for (int j = 0; j < kHamTidBits; ++j)
     if ((tid >> j) & 1) tphys |= 1ULL << P.bit[j];
@@ -151,7 +154,7 @@ ham_sweep_kernel(const T* __restrict__ psi, uint64_t pstride, const __grid_const
     }
     for (int k = tid; k < nterms; k += kHamThreads) {
       const double c = tc[P.term0 + k];
-      sc[k] = (__popcll(base & tz[P.term0 + k]) & 1) ? -c : c;
+      sc[k] = flips(base, P.term0 + k) ? -c : c;
     }
     __syncthreads();
     // sum of the strings [k0, k1) at the thread's amplitude 0
@@ -163,7 +166,7 @@ ham_sweep_kernel(const T* __restrict__ psi, uint64_t pstride, const __grid_const
           f += ((words[k * (kHamThreads / 32) + warp] >> lane) & 1) ? -c : c;
         }
       } else {
-        for (int k = k0; k < k1; ++k) f += (__popcll(tx & tz[k]) & 1) ? -tc[k] : tc[k];
+        for (int k = k0; k < k1; ++k) f += flips(tx, k) ? -tc[k] : tc[k];
       }
       return f;
     };
@@ -251,8 +254,8 @@ constexpr size_t ham_smem_limit() {
 }
 
 template <class T>
-cudaError_t run_sweeps(const HamPlan& hp, const HamTables& tb, const T* psi, uint64_t pstride, int nsets, T* lam,
-                       uint64_t lstride, double* partials, double* energy, double* energy_im, cudaStream_t st) {
+cudaError_t run_sweeps(const HamPlan& hp, const HamTables& tb, const ulonglong2* frames, const T* psi,
+                       uint64_t pstride, int nsets, T* lam, uint64_t lstride, double* partials, double* energy, double* energy_im, cudaStream_t st) {
   if (nsets < 1) nsets = 1;
   size_t smem_max = 0;
   for (const HamSweep& w : hp.sweeps) smem_max = std::max(smem_max, ham_smem_bytes(w, sizeof(T)));
@@ -274,7 +277,7 @@ cudaError_t run_sweeps(const HamPlan& hp, const HamTables& tb, const T* psi, uin
     const bool sums = !lam || i == np - 1;
     const size_t at = lam ? 0 : (size_t)i * grid;
     ham_sweep_kernel<T><<<dim3(grid, nsets), kHamThreads, ham_smem_bytes(s, sizeof(T)), st>>>(
-        psi, pstride, s, tb.items, tb.z, tb.c, lam, lstride, sums ? partials + at : nullptr,
+        psi, pstride, s, tb.items, tb.z, tb.x, tb.c, frames, lam, lstride, sums ? partials + at : nullptr,
         (sums && im) ? im + at : nullptr, rstride);
   }
   cudaError_t e = launch_row_sums(partials, nsets, (int)rstride, energy, st);
@@ -289,6 +292,7 @@ void plan_hamiltonian(int n, const HamTerms& h, const uint64_t* zmask, const dou
   hp.sweeps.clear();
   hp.items.clear();
   hp.z.clear();
+  hp.x.clear();
   hp.c.clear();
   const uint64_t low = (1ULL << kHamChunk) - 1;
   std::vector<uint8_t> done(h.ngroups, 0);
@@ -347,6 +351,7 @@ void plan_hamiltonian(int n, const HamTerms& h, const uint64_t* zmask, const dou
             if (pat != p) continue;
             if (p) I.flags &= ~HAM_FLAT;
             hp.z.push_back(zmask[t]);
+            hp.x.push_back(h.xmask[g]);
             // the sign is that of the partner index x ^ xmask
             hp.c.push_back((__builtin_popcountll(h.xmask[g] & zmask[t]) & 1) ? -c : c);
           }
@@ -367,7 +372,7 @@ void plan_hamiltonian(int n, const HamTerms& h, const uint64_t* zmask, const dou
 }
 
 size_t HamPlan::table_bytes() const {
-  return items.size() * sizeof(HamItem) + z.size() * sizeof(uint64_t) + c.size() * sizeof(double);
+  return items.size() * sizeof(HamItem) + (z.size() + x.size()) * sizeof(uint64_t) + c.size() * sizeof(double);
 }
 
 void HamPlan::pack(void* dst) const {
@@ -376,6 +381,8 @@ void HamPlan::pack(void* dst) const {
   p += items.size() * sizeof(HamItem);
   std::memcpy(p, z.data(), z.size() * sizeof(uint64_t));
   p += z.size() * sizeof(uint64_t);
+  std::memcpy(p, x.data(), x.size() * sizeof(uint64_t));
+  p += x.size() * sizeof(uint64_t);
   std::memcpy(p, c.data(), c.size() * sizeof(double));
 }
 
@@ -386,20 +393,22 @@ HamTables HamPlan::tables(const void* dev) const {
   p += items.size() * sizeof(HamItem);
   t.z = reinterpret_cast<const uint64_t*>(p);
   p += z.size() * sizeof(uint64_t);
+  t.x = reinterpret_cast<const uint64_t*>(p);
+  p += x.size() * sizeof(uint64_t);
   t.c = reinterpret_cast<const double*>(p);
   return t;
 }
 
-cudaError_t launch_hamiltonian(const HamPlan& hp, const HamTables& tb, const double2* psi, uint64_t pstride, int nsets,
-                               double2* lam, uint64_t lstride, double* partials, double* energy, double* energy_im,
+cudaError_t launch_hamiltonian(const HamPlan& hp, const HamTables& tb, const ulonglong2* frames, const double2* psi,
+                               uint64_t pstride, int nsets, double2* lam, uint64_t lstride, double* partials, double* energy, double* energy_im,
                                cudaStream_t st) {
-  return run_sweeps(hp, tb, psi, pstride, nsets, lam, lstride, partials, energy, energy_im, st);
+  return run_sweeps(hp, tb, frames, psi, pstride, nsets, lam, lstride, partials, energy, energy_im, st);
 }
 
-cudaError_t launch_hamiltonian_c64(const HamPlan& hp, const HamTables& tb, const float2* psi, uint64_t pstride,
-                                   int nsets, float2* lam, uint64_t lstride, double* partials, double* energy,
+cudaError_t launch_hamiltonian_c64(const HamPlan& hp, const HamTables& tb, const ulonglong2* frames, const float2* psi,
+                                   uint64_t pstride, int nsets, float2* lam, uint64_t lstride, double* partials, double* energy,
                                    cudaStream_t st) {
-  return run_sweeps(hp, tb, psi, pstride, nsets, lam, lstride, partials, energy, (double*)nullptr, st);
+  return run_sweeps(hp, tb, frames, psi, pstride, nsets, lam, lstride, partials, energy, (double*)nullptr, st);
 }
 
 }  // namespace iqb

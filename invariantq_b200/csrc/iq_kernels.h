@@ -120,13 +120,14 @@ struct HamSweep {
 };
 struct HamTables {
   const HamItem* items;
-  const uint64_t* z;
+  const uint64_t* z;                   // per string: Z mask, X mask, coefficient
+  const uint64_t* x;
   const double* c;
 };
 struct HamPlan {
   std::vector<HamSweep> sweeps;
   std::vector<HamItem> items;
-  std::vector<uint64_t> z;
+  std::vector<uint64_t> z, x;
   std::vector<double> c;
   size_t table_bytes() const;
   void pack(void* dst) const;          // table_bytes() bytes, 8-byte aligned
@@ -138,12 +139,13 @@ void plan_hamiltonian(int n, const HamTerms& h, const uint64_t* zmask, const dou
 // For each of nsets states psi_s = psi + s * pstride (2^n amplitudes):
 // lambda_s = H psi_s written to lam + s * lstride (when lam is not null), and
 // energy[s] = Re <psi_s|H|psi_s> (energy_im: the imaginary part, if not null).
-cudaError_t launch_hamiltonian(const HamPlan& hp, const HamTables& tb, const double2* psi, uint64_t pstride, int nsets,
-                               double2* lam, uint64_t lstride, double* partials, double* energy, double* energy_im,
+// frames (device, or null): set s's Pauli frame, X mask and Z mask; H is then F H F.
+cudaError_t launch_hamiltonian(const HamPlan& hp, const HamTables& tb, const ulonglong2* frames, const double2* psi,
+                               uint64_t pstride, int nsets, double2* lam, uint64_t lstride, double* partials, double* energy, double* energy_im,
                                cudaStream_t st);
 // complex64 (float2) storage, products and sums in FP64; a plan of one sweep, so lambda is rounded once
-cudaError_t launch_hamiltonian_c64(const HamPlan& hp, const HamTables& tb, const float2* psi, uint64_t pstride,
-                                   int nsets, float2* lam, uint64_t lstride, double* partials, double* energy,
+cudaError_t launch_hamiltonian_c64(const HamPlan& hp, const HamTables& tb, const ulonglong2* frames, const float2* psi,
+                                   uint64_t pstride, int nsets, float2* lam, uint64_t lstride, double* partials, double* energy,
                                    cudaStream_t st);
 // nsets joint arrays [psi | lambda | zero padding] of jdim amplitudes end to
 // end: psi halves (2^n amplitudes) set to e_0, padding above 2^(n+1) zeroed.

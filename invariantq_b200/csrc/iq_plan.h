@@ -426,7 +426,19 @@ void normalize_one_qubit_ops(std::vector<SchedOp>& ops, std::vector<cplx64>& poo
 // diag(1, p) (2 FMAs per amplitude).  Scalars collect into runs of at most
 // kNormSegment rotations, each ended by a scalar operation.  Non-unitary
 // one-qubit matrices are left dense.
-void decompose_one_qubit_ops(std::vector<SchedOp>& ops, std::vector<cplx64>& pool);
+//
+// The emitted structure normally follows the angles: a rotation is divided by
+// the larger of |c| and |s|, X is emitted where a gate or a pending diagonal
+// makes one, and scalars where their magnitude asks for it.  Kernels compiled
+// for one circuit's structure then do not fit the next circuit of the same
+// gates, so two steadier forms exist: DECOMP_STEADY_SCALARS emits the scalar
+// after a fixed number of rotations; DECOMP_STEADY also pulls an X out of every
+// gate with |c| < |s| (the tan form always), carries pending X operators
+// through the later gates as it does diagonals, and writes each qubit's last
+// rotation as a plain real 2x2 that absorbs the pending X (2 multiply-adds per
+// amplitude more, once per qubit).
+enum DecompMode { DECOMP_BY_ANGLE = 0, DECOMP_STEADY_SCALARS = 1, DECOMP_STEADY = 2 };
+void decompose_one_qubit_ops(std::vector<SchedOp>& ops, std::vector<cplx64>& pool, DecompMode mode = DECOMP_BY_ANGLE);
 // Re-pack the matrix data each pass references (absolute offsets into `pool`)
 // into one contiguous block per pass: sets desc.mat_base / mat_elems and makes
 // every op's `mat` relative to its pass block, which the kernel stages in
@@ -470,7 +482,22 @@ int ansatz_check(int n, const std::vector<AnsatzOp>& ops, std::string& err);
 // Forward circuit on an n-bit state vector: ops appended to `out` (matrices to `pool`).
 // phase_free: RZ (and P) as diag(1, e^{i theta}), the global phase dropped.
 void ansatz_forward(int n, const std::vector<AnsatzOp>& ops, const double* params, std::vector<SchedOp>& out,
-                    std::vector<cplx64>& pool, bool phase_free = false);
+                    std::vector<cplx64>& pool, bool phase_free = false, const struct PauliFrame* frame = nullptr);
+// A circuit in a Pauli frame: its state is X^x Z^z (up to a phase) times the
+// state of the same circuit with every rotation's angle th replaced by
+// sign th - k pi, |c| >= |s| for X and Y rotations.  exp(-i k pi P / 2) is a
+// Pauli operator, which every fixed gate maps to another one and which flips
+// the sign of the rotations it does not commute with.  X and Y rotations then
+// always take the tan form, so operation lists (and the kernels compiled for
+// their plans) do not depend on the angles; <H> and its gradient come from the
+// frame's state with the signs of H's strings flipped where they do not
+// commute with the frame, and each term times its rotation's sign.
+struct PauliFrame {
+  struct Rot { double c, s; int sign; };   // cos and sin of half the reduced angle (Z: of half sign th)
+  std::vector<Rot> rot;                    // in forward order, gate by gate
+  uint64_t x = 0, z = 0;
+};
+void pauli_frame(const std::vector<AnsatzOp>& ops, const double* params, PauliFrame& f);
 // Backward sweep on the joint array of n + 1 bits (bit 0 selects psi (0) or
 // lambda = H psi (1), bit q + 1 is qubit q): for every gate from last to first,
 // an adjoint step (gradient term + inverse rotation) per rotation angle, or the
@@ -484,7 +511,8 @@ void ansatz_forward(int n, const std::vector<AnsatzOp>& ops, const double* param
 // angles, so `scaled` suits a parameter set that shares its plans with no other.
 void ansatz_backward(int n, const std::vector<AnsatzOp>& ops, const double* params, std::vector<SchedOp>& out,
                      std::vector<cplx64>& pool, std::vector<int>& grad_param, int select_bit = 0,
-                     bool scaled = false, std::vector<double>* grad_scale = nullptr);
+                     bool scaled = false, std::vector<double>* grad_scale = nullptr,
+                     const PauliFrame* frame = nullptr, std::vector<int8_t>* grad_sign = nullptr);
 // One parameter set's operation lists as the adjoint executor runs them.
 // single_set: the forward goes through decompose_one_qubit_ops and
 // normalize_one_qubit_ops (two-qubit monomials kept apart) and the backward
@@ -496,9 +524,12 @@ struct AdjointOps {
   std::vector<cplx64> fpool, bpool;
   std::vector<int> grad_param;
   std::vector<double> grad_scale;
+  PauliFrame frame;                  // with `framed` only
+  std::vector<int8_t> grad_sign;
 };
+// framed: with single_set, in a Pauli frame -- one structure for every parameter set
 void adjoint_ops(int n, const std::vector<AnsatzOp>& ops, const double* params, bool backward, bool fuse,
-                 bool single_set, AdjointOps& j);
+                 bool single_set, AdjointOps& j, bool framed = false);
 // The scale factors of a backward sweep's gradient terms in the order the
 // operations run: the planner moves adjoint steps on different qubits past
 // each other, so the scale each term sees is the product of the factors

@@ -594,7 +594,7 @@ struct Engine : HandleRes {
     pg.tl = launch_params(spec);
     std::vector<SchedOp> fused = fuse ? fuse_two_qubit_blocks(ops, pool, spec) : ops;
     if (spec && normalize) {
-      decompose_one_qubit_ops(fused, pool);
+      decompose_one_qubit_ops(fused, pool, DECOMP_STEADY);
       normalize_one_qubit_ops(fused, pool);
     }
     int maxk = 1;
@@ -1320,7 +1320,7 @@ int iq_statevector_expval_pauli_sum(void* sv, size_t nterms, const double* coeff
     e->st_launches += (double)launches;
     double* res = e->result_slot();
     double out[2];
-    if (!cuda_ok(launch_hamiltonian(hp, hp.tables(e->d_pool), e->d_state, 0, 1, nullptr, 0, e->partials(), res, res + 1,
+    if (!cuda_ok(launch_hamiltonian(hp, hp.tables(e->d_pool), nullptr, e->d_state, 0, 1, nullptr, 0, e->partials(), res, res + 1,
                                     e->stream),
                  "pauli sum") ||
         !e->read_doubles(res, 2, out))

@@ -757,7 +757,7 @@ std::vector<SchedOp> fuse_two_qubit_blocks(const std::vector<SchedOp>& ops, std:
 void normalize_one_qubit_ops(std::vector<SchedOp>& ops, std::vector<cplx64>& pool) {
   std::vector<int> dense1;
   for (size_t i = 0; i < ops.size(); ++i)
-    if (ops[i].k == 1 && !ops[i].mono && !ops[i].grad && !ops[i].rot) dense1.push_back((int)i);
+    if (ops[i].k == 1 && !ops[i].mono && !ops[i].grad && !ops[i].rot && !ops[i].realm) dense1.push_back((int)i);
   for (size_t s0 = 0; s0 < dense1.size(); s0 += kNormSegment) {
     const size_t s1 = std::min(dense1.size(), s0 + kNormSegment);
     if (s1 - s0 < 2) break;
@@ -797,10 +797,22 @@ struct Decomposer {
   std::vector<SchedOp>& out;
   std::vector<cplx64>& pool;
   std::vector<cplx64> pa, pb;   // pending output diagonal diag(pa[q], pb[q]) of each qubit
+  std::vector<uint8_t> px;      // DECOMP_STEADY: a pending X of the qubit, before that diagonal
   cplx64 G{1.0, 0.0};           // scalar factored out of the emitted operations
+  DecompMode mode;
+  int rotations = 0;            // since the last scalar
+  // a tan form divides by c >= 1/sqrt 2: this many keep the scale above 2^-96
+  static constexpr int kScalarEvery = 192;
 
-  Decomposer(std::vector<SchedOp>& o, std::vector<cplx64>& p) : out(o), pool(p), pa(64, {1.0, 0.0}), pb(64, {1.0, 0.0}) {}
+  Decomposer(std::vector<SchedOp>& o, std::vector<cplx64>& p, DecompMode m)
+      : out(o), pool(p), pa(64, {1.0, 0.0}), pb(64, {1.0, 0.0}), px(64, 0), mode(m) {}
 
+  // exactly 1 -- in the steady modes also 1 up to rounding, so that a phase that
+  // cancels does not come and go with the angles
+  bool unit_phase(cplx64 a) const {
+    if (is_one(a)) return true;
+    return mode != DECOMP_BY_ANGLE && std::fabs(a.re - 1.0) <= 2e-15 && std::fabs(a.im) <= 2e-15;
+  }
   uint32_t put(std::initializer_list<cplx64> v) {
     const uint32_t at = (uint32_t)pool.size();
     for (const cplx64& x : v) pool.push_back(x);
@@ -810,7 +822,7 @@ struct Decomposer {
   void emit_phase(int q, cplx64 a, cplx64 b) {
     const cplx64 r = cdiv(b, a);
     G = cm(G, a);
-    if (is_one(r)) return;
+    if (unit_phase(r)) return;
     SchedOp o{};
     o.k = 1;
     o.q[0] = (uint8_t)q;
@@ -821,7 +833,13 @@ struct Decomposer {
     o.dense = put({{1.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}, r});
     out.push_back(o);
   }
+  void flush_x(int q) {
+    if (!px[q]) return;
+    emit_x(q);
+    px[q] = 0;
+  }
   void flush(int q) {
+    flush_x(q);
     if (is_one(pa[q]) && is_one(pb[q])) return;
     emit_phase(q, pa[q], pb[q]);
     pa[q] = pb[q] = {1.0, 0.0};
@@ -850,12 +868,12 @@ struct Decomposer {
     o.dense = put({{0.0, 0.0}, {1.0, 0.0}, {1.0, 0.0}, {0.0, 0.0}});
     out.push_back(o);
   }
-  // real rotation [[c, -s], [s, c]] (c^2 + s^2 = 1), normalised by max(c, s)
+  // real rotation [[c, -s], [s, c]] (c > 0, c^2 + s^2 = 1), normalised by max(c, |s|)
   void emit_rotation(int q, double c, double s) {
     SchedOp o{};
     o.k = 1;
     o.q[0] = (uint8_t)q;
-    if (c >= s) {
+    if (c >= std::fabs(s)) {
       const double t = s / c;
       G = cm(G, {c, 0.0});
       o.rot = 1;
@@ -870,13 +888,32 @@ struct Decomposer {
     out.push_back(o);
     // keep the scale of the intermediate state within 2^+-100
     const double g2 = cabs2(G);
-    if (g2 < 0x1p-200 || g2 > 0x1p200) emit_scalar(q);
+    ++rotations;
+    if (g2 < 0x1p-200 || g2 > 0x1p200 || (mode != DECOMP_BY_ANGLE && rotations >= kScalarEvery)) {
+      emit_scalar(q);
+      rotations = 0;
+    }
+  }
+  void emit_real(int q, double c, double s) {   // [[c, -s], [s, c]] as it is
+    SchedOp o{};
+    o.k = 1;
+    o.q[0] = (uint8_t)q;
+    o.realm = 1;
+    o.dense = o.mat = put({{c, 0.0}, {-s, 0.0}, {s, 0.0}, {c, 0.0}});
+    out.push_back(o);
   }
   // dense one-qubit U (row-major) on q, after the pending diagonal of q
-  void dense1(const SchedOp& src) {
+  // (`last`: no dense one-qubit operation on q follows)
+  void dense1(const SchedOp& src, bool last) {
     const int q = src.q[0];
+    const bool steady = mode == DECOMP_STEADY;
     const cplx64* U0 = pool.data() + src.dense;
-    const cplx64 A = cm(U0[0], pa[q]), B = cm(U0[1], pb[q]), C = cm(U0[2], pa[q]), D = cm(U0[3], pb[q]);
+    cplx64 A = cm(U0[0], pa[q]), B = cm(U0[1], pb[q]), C = cm(U0[2], pa[q]), D = cm(U0[3], pb[q]);
+    if (px[q]) {   // the pending X swaps the columns
+      std::swap(A, B);
+      std::swap(C, D);
+      px[q] = 0;
+    }
     const double n0 = cabs2(A) + cabs2(C), n1 = cabs2(B) + cabs2(D);
     const cplx64 ip{A.re * B.re + A.im * B.im + C.re * D.re + C.im * D.im,
                     A.re * B.im - A.im * B.re + C.re * D.im - C.im * D.re};   // conj(A) B + conj(C) D
@@ -888,23 +925,43 @@ struct Decomposer {
       return;
     }
     if (unitary && c0 == 0.0 && cabs2(D) == 0.0) {     // anti-diagonal: X, then diag(B, C)
-      emit_x(q);
+      if (steady) px[q] = 1;
+      else emit_x(q);
       pa[q] = B;
       pb[q] = C;
       return;
     }
     if (unitary && c0 > 0.0 && s0 > 0.0) {
+      // steady: U = X (X U) where |c| < |s|, so the rotation is always of the tan form
+      const bool swap = steady && !last && c0 < s0;
+      if (swap) {
+        std::swap(A, C);
+        std::swap(B, D);
+      }
       const double r = std::hypot(c0, s0);
-      const double c = c0 / r, s = s0 / r;
-      const cplx64 d0 = cdiv(A, {c, 0.0}), d1 = cdiv(C, {s, 0.0});
-      const cplx64 e1 = cdiv({-B.re, -B.im}, cm(d0, {s, 0.0}));
+      const double c = (swap ? s0 : c0) / r;
+      double s = (swap ? c0 : s0) / r;
+      const cplx64 d0 = cdiv(A, {c, 0.0});
+      cplx64 d1 = cdiv(C, {s, 0.0});
+      cplx64 e1 = cdiv({-B.re, -B.im}, cm(d0, {s, 0.0}));
+      if (mode != DECOMP_BY_ANGLE && e1.re < 0.0) {   // the sign goes to s: a real gate has no phase, whatever its angle
+        s = -s;
+        d1 = {-d1.re, -d1.im};
+        e1 = {-e1.re, -e1.im};
+      }
       const cplx64 Dr = cm(cm(d1, {c, 0.0}), e1);           // the rebuilt entry D
       if (cabs2({Dr.re - D.re, Dr.im - D.im}) < 1e-28) {
         emit_phase(q, {1.0, 0.0}, e1);
-        emit_rotation(q, c, s);
-        pa[q] = d0;
-        pb[q] = d1;
+        if (steady && last) emit_real(q, c, s);
+        else emit_rotation(q, c, s);
+        pa[q] = swap ? d1 : d0;
+        pb[q] = swap ? d0 : d1;
+        px[q] = swap ? 1 : 0;
         return;
+      }
+      if (swap) {
+        std::swap(A, C);
+        std::swap(B, D);
       }
     }
     // not unitary (or not rebuilt exactly enough): dense, with the pending diagonal in its columns
@@ -922,11 +979,19 @@ struct Decomposer {
     const int q0 = src.q[0], q1 = src.q[1];
     cplx64 ph[4];
     for (int r = 0; r < 4; ++r) ph[r] = src.unit ? cplx64{1.0, 0.0} : pool[src.mat + r];
-    cplx64 Dp[4];
-    for (int r = 0; r < 4; ++r) {
-      const int col = (src.perm >> (2 * r)) & 3;
+    // pending X operators X^m in front of the permutation P are X^mo behind it
+    // (every permutation of four is affine: P(r ^ mo) = P(r) ^ m); rows are
+    // numbered before X^mo
+    auto column = [&](int r) { return (src.perm >> (2 * r)) & 3; };
+    const int m = (px[q0] ? 1 : 0) | (px[q1] ? 2 : 0);
+    int mo = 0;
+    while ((column(mo) ^ column(0)) != m) ++mo;
+    cplx64 Dp[4], php[4];
+    for (int z = 0; z < 4; ++z) {
+      const int r = z ^ mo, col = column(r);
       const cplx64 dl = cm((col & 1) ? pb[q0] : pa[q0], (col & 2) ? pb[q1] : pa[q1]);
-      Dp[r] = cm(ph[r], dl);
+      Dp[z] = cm(ph[r], dl);
+      php[z] = ph[r];
     }
     bool unit_modulus = true;
     for (int r = 0; r < 4; ++r) unit_modulus = unit_modulus && std::fabs(cabs2(ph[r]) - 1.0) < 1e-12;
@@ -937,6 +1002,9 @@ struct Decomposer {
       SchedOp o = src;
       o.unit = 0;
       o.urows = 0;
+      o.nrows = 0;
+      px[q0] = (uint8_t)(mo & 1);
+      px[q1] = (uint8_t)(mo >> 1);
       o.mat = put({Dp[0], Dp[1], Dp[2], Dp[3]});
       o.dense = (uint32_t)pool.size();
       for (int r = 0; r < 4; ++r)
@@ -949,13 +1017,17 @@ struct Decomposer {
     const cplx64 s0 = Dp[0];
     const cplx64 x1 = cdiv(Dp[1], s0), y1 = cdiv(Dp[2], s0);
     // a diagonal gate's own part does not depend on the pending diagonals (CZ: exactly -1)
-    const cplx64 gamma = src.perm == 0xE4 ? cdiv(cm(ph[0], ph[3]), cm(ph[1], ph[2])) : cdiv(Dp[3], cm(s0, cm(x1, y1)));
+    const cplx64 gamma = src.perm == 0xE4 ? cdiv(cm(php[0], php[3]), cm(php[1], php[2])) : cdiv(Dp[3], cm(s0, cm(x1, y1)));
     G = cm(G, s0);
+    px[q0] = (uint8_t)(mo & 1);
+    px[q1] = (uint8_t)(mo >> 1);
     pa[q0] = pa[q1] = {1.0, 0.0};
     pb[q0] = x1;
     pb[q1] = y1;
+    if (px[q0]) std::swap(pa[q0], pb[q0]);   // the diagonal comes after the X
+    if (px[q1]) std::swap(pa[q1], pb[q1]);
     SchedOp o = src;
-    const bool unit = is_one(gamma);
+    const bool unit = unit_phase(gamma);
     o.unit = unit ? 1 : 0;
     o.urows = unit ? 15 : 7;
     o.nrows = (gamma.re == -1.0 && gamma.im == 0.0) ? 8 : 0;
@@ -969,17 +1041,32 @@ struct Decomposer {
     out.push_back(o);
   }
   // dense k-qubit operation: the pending diagonals scale its columns
+  // (and a pending X swaps them)
   void dense_k(const SchedOp& src) {
     const int d = 1 << src.k;
+    int m = 0, keep = 0;
+    for (int j = 0; j < src.k; ++j) m |= px[src.q[j]] ? 1 << j : 0;
+    if (src.xpat && m) {
+      // a channel's shape survives X (x) X on both sides only: those stay pending behind it
+      if (m == 3) keep = 3;
+      else for (int j = 0; j < src.k; ++j) flush_x(src.q[j]);
+      if (m != 3) m = 0;
+    }
     SchedOp o = src;
     o.dense = o.mat = (uint32_t)pool.size();
+    // column c of the operation acting on X^m x reads column c ^ m, scaled by the diagonal there; rows
+    // keep their X^keep in front
     for (int r = 0; r < d; ++r)
       for (int c = 0; c < d; ++c) {
+        const int col = c ^ m;
         cplx64 f{1.0, 0.0};
-        for (int j = 0; j < src.k; ++j) f = cm(f, ((c >> j) & 1) ? pb[src.q[j]] : pa[src.q[j]]);
-        pool.push_back(cm(pool[src.dense + r * d + c], f));
+        for (int j = 0; j < src.k; ++j) f = cm(f, ((col >> j) & 1) ? pb[src.q[j]] : pa[src.q[j]]);
+        pool.push_back(cm(pool[src.dense + (r ^ keep) * d + col], f));
       }
-    for (int j = 0; j < src.k; ++j) pa[src.q[j]] = pb[src.q[j]] = {1.0, 0.0};
+    for (int j = 0; j < src.k; ++j) {
+      pa[src.q[j]] = pb[src.q[j]] = {1.0, 0.0};
+      px[src.q[j]] = (uint8_t)((keep >> j) & 1);
+    }
     if (src.xpat)   // the diagonal scales columns: same shape, entries maybe complex now
       o.xpat = (uint8_t)classify_xpattern(reinterpret_cast<const double*>(pool.data() + o.dense));
     out.push_back(o);
@@ -988,22 +1075,27 @@ struct Decomposer {
 
 }  // namespace
 
-void decompose_one_qubit_ops(std::vector<SchedOp>& ops, std::vector<cplx64>& pool) {
+void decompose_one_qubit_ops(std::vector<SchedOp>& ops, std::vector<cplx64>& pool, DecompMode mode) {
   std::vector<SchedOp> out;
   out.reserve(ops.size() * 2);
-  Decomposer dc(out, pool);
+  Decomposer dc(out, pool, mode);
+  std::vector<size_t> last(64, 0);   // index past each qubit's last dense one-qubit operation
+  for (size_t i = 0; i < ops.size(); ++i)
+    if (ops[i].k == 1 && !ops[i].mono && !ops[i].grad) last[ops[i].q[0]] = i + 1;
   int last_q = 0;
-  for (const SchedOp& o : ops) {
+  for (size_t i = 0; i < ops.size(); ++i) {
+    const SchedOp& o = ops[i];
     if (o.grad) {
       for (int j = 0; j < o.k; ++j) dc.flush(o.q[j]);
       out.push_back(o);
     } else if (o.k == 1 && !o.mono) {
-      dc.dense1(o);
+      dc.dense1(o, last[o.q[0]] == i + 1);
     } else if (o.k == 1) {             // one-qubit monomial: diagonal, or X with phases
       const int q = o.q[0];
       const cplx64 p0 = o.unit ? cplx64{1.0, 0.0} : pool[o.mat], p1 = o.unit ? cplx64{1.0, 0.0} : pool[o.mat + 1];
       if (o.perm & 1) {
-        dc.emit_x(q);
+        if (mode == DECOMP_STEADY) dc.px[q] ^= 1;
+        else dc.emit_x(q);
         const cplx64 a = cm(p0, dc.pb[q]), b = cm(p1, dc.pa[q]);
         dc.pa[q] = a;
         dc.pb[q] = b;
@@ -1069,6 +1161,14 @@ void rotation(int g, double th, cdd* m) {
   else { m[0] = std::exp(-I * (th / 2.0)); m[1] = 0.0; m[2] = 0.0; m[3] = std::exp(I * (th / 2.0)); }
 }
 
+// the same from c = cos(th/2), s = sin(th/2)
+void rotation_cs(int g, double c, double s, cdd* m) {
+  const cdd I(0.0, 1.0);
+  if (g == 0) { m[0] = c; m[1] = -I * s; m[2] = -I * s; m[3] = c; }
+  else if (g == 1) { m[0] = c; m[1] = -s; m[2] = s; m[3] = c; }
+  else { m[0] = cdd(c, -s); m[1] = 0.0; m[2] = 0.0; m[3] = cdd(c, s); }
+}
+
 void dagger2(const cdd* m, cdd* o) {
   o[0] = std::conj(m[0]); o[1] = std::conj(m[2]); o[2] = std::conj(m[1]); o[3] = std::conj(m[3]);
 }
@@ -1120,21 +1220,79 @@ int ansatz_check(int n, const std::vector<AnsatzOp>& ops, std::string& err) {
   return np;
 }
 
+void pauli_frame(const std::vector<AnsatzOp>& ops, const double* params, PauliFrame& f) {
+  f.rot.clear();
+  f.x = f.z = 0;
+  for (const AnsatzOp& o : ops) {
+    int gen[3], par[3];
+    const int nr = rotations_of(o, gen, par);
+    const uint64_t b = 1ULL << o.q0;
+    for (int r = 0; r < nr; ++r) {
+      const bool fx = f.x & b, fz = f.z & b;
+      // X, Y, Z anticommute with the frame's Pauli operator on the qubit
+      const bool anti = gen[r] == 0 ? fz : (gen[r] == 1 ? fx != fz : fx);
+      PauliFrame::Rot t;
+      t.sign = anti ? -1 : 1;
+      const double th = params[par[r]];
+      t.c = std::cos(th / 2.0);
+      t.s = t.sign * std::sin(th / 2.0);
+      if (gen[r] != 2 && std::fabs(t.s) > std::fabs(t.c)) {
+        // th' = th - pi: cos(th'/2) = sin(th/2), sin(th'/2) = -cos(th/2); exp(-i pi P / 2) joins the frame
+        const double c = t.c;
+        t.c = t.s;
+        t.s = -c;
+        f.x ^= b;
+        if (gen[r] == 1) f.z ^= b;
+      }
+      if (gen[r] != 2 && t.c < 0.0) {   // an overall sign
+        t.c = -t.c;
+        t.s = -t.s;
+      }
+      f.rot.push_back(t);
+    }
+    if (nr) continue;
+    const uint64_t c = o.q1 >= 0 ? 1ULL << o.q1 : 0;
+    switch (o.kind) {
+      case GATE_CZ:
+        if (f.x & b) f.z ^= c;
+        if (f.x & c) f.z ^= b;
+        break;
+      case GATE_CX:   // control q0, target q1
+        if (f.x & b) f.x ^= c;
+        if (f.z & c) f.z ^= b;
+        break;
+      case GATE_H: {
+        const bool fx = f.x & b, fz = f.z & b;
+        f.x = (f.x & ~b) | (fz ? b : 0);
+        f.z = (f.z & ~b) | (fx ? b : 0);
+        break;
+      }
+      case GATE_SX:   // Z to -Y
+        if (f.z & b) f.x ^= b;
+        break;
+      default: break;
+    }
+  }
+}
+
 void ansatz_forward(int n, const std::vector<AnsatzOp>& ops, const double* params, std::vector<SchedOp>& out,
-                    std::vector<cplx64>& pool, bool phase_free) {
+                    std::vector<cplx64>& pool, bool phase_free, const PauliFrame* frame) {
   (void)n;
+  size_t rot = 0;
   for (const AnsatzOp& o : ops) {
     int gen[3], par[3];
     const int nr = rotations_of(o, gen, par);
     if (nr) {
       for (int r = 0; r < nr; ++r) {
         cdd m[4];
-        rotation(gen[r], params[par[r]], m);
+        if (frame) rotation_cs(gen[r], frame->rot[rot].c, frame->rot[rot].s, m);
+        else rotation(gen[r], params[par[r]], m);
         if (phase_free && gen[r] == 2) {   // e^{-i th/2} diag(1, e^{i th}): the common phase dropped
           const double th = params[par[r]];
           m[0] = 1.0;
-          m[3] = cdd(std::cos(th), std::sin(th));
+          m[3] = cdd(std::cos(th), frame ? frame->rot[rot].sign * std::sin(th) : std::sin(th));
         }
+        ++rot;
         const int q[1] = {o.q0};
         push_op(out, pool, 1, q, m);
       }
@@ -1149,10 +1307,13 @@ void ansatz_forward(int n, const std::vector<AnsatzOp>& ops, const double* param
 
 void ansatz_backward(int n, const std::vector<AnsatzOp>& ops, const double* params, std::vector<SchedOp>& out,
                      std::vector<cplx64>& pool, std::vector<int>& grad_param, int select_bit, bool scaled,
-                     std::vector<double>* grad_scale) {
+                     std::vector<double>* grad_scale, const PauliFrame* frame, std::vector<int8_t>* grad_sign) {
   if (select_bit < 0) select_bit = n;
   auto bit = [&](int q) { return q + (q >= select_bit ? 1 : 0); };   // index bit of qubit q in the joint array
   double sigma = 1.0;   // stored amplitudes = true amplitudes / sigma
+  size_t rot = frame ? frame->rot.size() : 0;
+  int since = 0;        // scaled steps since the last scalar; in a frame each divides by 1/sqrt 2 or more
+  constexpr int kScalarEvery = 120;
   for (size_t i = ops.size(); i-- > 0;) {
     const AnsatzOp& o = ops[i];
     int gen[3], par[3];
@@ -1160,15 +1321,16 @@ void ansatz_backward(int n, const std::vector<AnsatzOp>& ops, const double* para
     if (nr) {
       for (int r = nr - 1; r >= 0; --r) {   // last rotation of the gate first
         const double th = params[par[r]];
+        const PauliFrame::Rot* fr = frame ? &frame->rot[--rot] : nullptr;
         cdd md[4];
         uint8_t form = GRAD_PLAIN;
         double kappa = 1.0;
         if (gen[r] == 2) {
           // exp(+i th Z / 2) divided by its row-0 phase: diag(1, e^{-i th})
           form = GRAD_PHASE;
-          md[0] = 1.0; md[1] = 0.0; md[2] = 0.0; md[3] = cdd(std::cos(th), -std::sin(th));
+          md[0] = 1.0; md[1] = 0.0; md[2] = 0.0; md[3] = cdd(std::cos(th), fr ? -fr->sign * std::sin(th) : -std::sin(th));
         } else if (scaled) {
-          const double c = std::cos(th / 2.0), s = std::sin(th / 2.0);
+          const double c = fr ? fr->c : std::cos(th / 2.0), s = fr ? fr->s : std::sin(th / 2.0);
           const cdd j = gen[r] == 0 ? cdd(0.0, 1.0) : cdd(1.0, 0.0);   // X: i s off the diagonal; Y: +s, -s
           const cdd jl = gen[r] == 0 ? cdd(0.0, 1.0) : cdd(-1.0, 0.0);
           if (std::fabs(c) >= std::fabs(s)) {
@@ -1201,8 +1363,11 @@ void ansatz_backward(int n, const std::vector<AnsatzOp>& ops, const double* para
         out.push_back(g);
         grad_param.push_back(par[r]);
         if (grad_scale) grad_scale->push_back(sigma * sigma);
+        if (grad_sign) grad_sign->push_back(fr ? (int8_t)fr->sign : (int8_t)1);
         sigma *= kappa;
-        if (std::fabs(sigma) < 0x1p-64 || std::fabs(sigma) > 0x1p64) {
+        if (scaled && gen[r] != 2) ++since;
+        if (frame ? since >= kScalarEvery : (std::fabs(sigma) < 0x1p-64 || std::fabs(sigma) > 0x1p64)) {
+          since = 0;
           // back to the true scale: every amplitude of both halves times sigma
           const cdd sc[4] = {sigma, 0.0, 0.0, sigma};
           const int q[1] = {bit(o.q0)};
@@ -1225,14 +1390,18 @@ void ansatz_backward(int n, const std::vector<AnsatzOp>& ops, const double* para
 }
 
 void adjoint_ops(int n, const std::vector<AnsatzOp>& ops, const double* params, bool backward, bool fuse,
-                 bool single_set, AdjointOps& j) {
+                 bool single_set, AdjointOps& j, bool framed) {
   j.fw.clear(); j.bw.clear(); j.fpool.clear(); j.bpool.clear(); j.grad_param.clear(); j.grad_scale.clear();
+  j.grad_sign.clear();
+  framed = framed && single_set;
+  if (framed) pauli_frame(ops, params, j.frame);
+  const PauliFrame* const frame = framed ? &j.frame : nullptr;
   std::vector<SchedOp> raw;
   // a global phase of psi changes neither the energy nor any Im<lambda|P|psi>
-  ansatz_forward(n, ops, params, raw, j.fpool, /*phase_free=*/!single_set);
+  ansatz_forward(n, ops, params, raw, j.fpool, /*phase_free=*/!single_set, frame);
   if (single_set) {
     j.fw = fuse_two_qubit_blocks(raw, j.fpool, true);
-    decompose_one_qubit_ops(j.fw, j.fpool);
+    decompose_one_qubit_ops(j.fw, j.fpool, framed ? DECOMP_STEADY_SCALARS : DECOMP_BY_ANGLE);
     normalize_one_qubit_ops(j.fw, j.fpool);
   } else {
     // forms that do not depend on the angles, every gate alone: RY (and any
@@ -1250,7 +1419,7 @@ void adjoint_ops(int n, const std::vector<AnsatzOp>& ops, const double* params, 
   }
   if (!backward) return;
   raw.clear();
-  ansatz_backward(n, ops, params, raw, j.bpool, j.grad_param, n, single_set, &j.grad_scale);   // [psi | lambda]
+  ansatz_backward(n, ops, params, raw, j.bpool, j.grad_param, n, single_set, &j.grad_scale, frame, &j.grad_sign);   // [psi | lambda]
   j.bw = fuse ? fuse_two_qubit_blocks(raw, j.bpool, single_set) : raw;
 }
 
