@@ -291,7 +291,8 @@ int iq_adjoint_gradient_c64(size_t num_qubits, size_t num_ops, const int* kinds,
  * the parameter sets of one circuit run together, through the same tile-pass
  * launches, in groups that fit IQ_ADJOINT_JOB_BYTES (4 GiB) of states.  Fewer
  * streams when the workspaces would not fit in device memory.  Workspaces are
- * kept for later calls unless they hold more than 8 GiB of device memory.
+ * kept for later calls unless they hold more than 12 GiB of device memory (24
+ * GiB for all that are kept).
  * Returns 0, or -1 with iq_last_error set. */
 int iq_adjoint_gradient_batch(const iq_adjoint_circuit* circuits, size_t num_circuits, int num_streams);
 /* Free the device and pinned host memory the adjoint calls keep between calls

@@ -796,10 +796,13 @@ int current_device(std::string& err) {
 thread_local double t_stats[10] = {0};
 
 // Workspaces kept between calls (streams, events and buffers are costly to
-// create and allocation synchronises the device).  A workspace holding more
-// than kPoolKeepBytes of device memory is freed at the end of its call;
-// iq_adjoint_release frees the rest.  Never freed at process exit.
-constexpr double kPoolKeepBytes = 8.0 * (1ull << 30);
+// create and allocation synchronises the device; 8 GiB for a 28-qubit gradient:
+// ~4 ms of 160, with outliers of hundreds).  A workspace holding more than
+// kPoolKeepBytes of device memory, or that would take the pool past
+// kPoolTotalBytes, is freed at the end of its call; iq_adjoint_release frees the
+// rest.  Never freed at process exit.
+constexpr double kPoolKeepBytes = 12.0 * (1ull << 30);
+constexpr double kPoolTotalBytes = 24.0 * (1ull << 30);
 std::mutex g_pool_mu;
 std::vector<Workspace*>* g_pool = new std::vector<Workspace*>();
 
@@ -821,8 +824,17 @@ void pool_give(Workspace* w, bool ok) {
     return;
   }
   cudaStreamSynchronize(w->stream);
-  std::lock_guard<std::mutex> g(g_pool_mu);
-  g_pool->push_back(w);
+  {
+    std::lock_guard<std::mutex> g(g_pool_mu);
+    double kept = w->device_bytes();
+    for (const Workspace* o : *g_pool) kept += o->device_bytes();
+    if (kept <= kPoolTotalBytes) {
+      g_pool->push_back(w);
+      return;
+    }
+  }
+  w->release();
+  delete w;
 }
 
 // Run all jobs of `circs` (every parameter set of every circuit) on `nstreams` workers.
