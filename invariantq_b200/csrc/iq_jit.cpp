@@ -30,6 +30,7 @@ namespace {
 #include "iq_jit_headers.inc"
 
 constexpr int kMaxBufJit = 4;
+constexpr int kPairCtaThreads = 2 * 256 + 32, kPairTileBufs = 3;   // iq_pipe.cuh's pair pipeline
 // Kernels kept per process.  Modules stay loaded for the process's life (a
 // launch may still use one), so past this many distinct pass structures new
 // passes run on the interpreting kernel.
@@ -196,6 +197,7 @@ struct JitKernel {
   int nt = 128;
   bool sets = false;     // shared-memory matrices per parameter set (interpreting kernel's arguments)
   bool narrow = false;   // complex64 array, direct global loads and stores (jit_launch_narrow)
+  bool pair = false;     // the pair pipeline: one CTA per SM, three tile buffers
   std::atomic<int> smem_limit_set{0};
 };
 
@@ -279,6 +281,8 @@ bool install(int dev, const std::string& key, const std::string& src, const std:
   k->nt = source_NT(src);
   k->sets = src.find(" sets=1 ") != std::string::npos;
   k->narrow = src.find(" narrow=1 ") != std::string::npos;
+  k->pair = src.find(" pair=1 ") != std::string::npos;
+  if (k->pair) k->nt = kPairCtaThreads;
   JitState& S = state();
   std::lock_guard<std::mutex> lk(S.mu);
   S.cache.emplace(std::make_pair(dev, key), std::move(k));   // keeps the first if two raced
@@ -432,6 +436,7 @@ cudaError_t jit_launch(const JitKernel* kc, const CUtensorMap& tm, const PassDes
   JitKernel* k = const_cast<JitKernel*>(kc);
   const Driver& dr = driver();
   int nbuf = tl.nbuf < 1 ? 1 : (tl.nbuf > kMaxBufJit ? kMaxBufJit : tl.nbuf);
+  if (k->pair) nbuf = kPairTileBufs;
   const size_t smem = 1024 + (size_t)nbuf * ((size_t)16 << d.M);
   if (!k->smem_limit_set.load(std::memory_order_acquire)) {
     int dev = 0, optin = 0;
@@ -446,7 +451,7 @@ cudaError_t jit_launch(const JitKernel* kc, const CUtensorMap& tm, const PassDes
   const double2* mats = d.mat_elems ? host_mats : zero_mat;
   void* args[] = {const_cast<CUtensorMap*>(&tm), const_cast<PassDesc*>(&d), const_cast<double2*>(mats), &dev_status,
                   &nbuf};
-  const unsigned grid = tile_pass_grid(d, tl, num_sms);
+  const unsigned grid = k->pair ? (unsigned)std::min<uint64_t>((uint64_t)num_sms, d.ntiles) : tile_pass_grid(d, tl, num_sms);
   const CUresult r = dr.launch(k->fn, grid, 1, 1, (unsigned)k->nt, 1, 1, (unsigned)smem, (CUstream)st, args, nullptr);
   return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorLaunchFailure;
 }

@@ -30,7 +30,10 @@ std::string mat(uint32_t i) { return (g_set_mode ? "smat[" : "Mt.m[") + std::to_
 // global memory (gst + tile base tb + physical offsets) instead of the tile;
 // bit 1: it stores them there; bit 2: the shared-memory tile is complex64
 // (float2 `ftile`: values widened to FP64 on load, rounded on store).
-bool gen_stage(Gen& g, const PassDesc& d, int s, int NT, std::string& err, int gmode = 0) {
+// `sync`: what separates the stage from the next one.  NT = 0: the pair
+// pipeline's groups, whose threads hold one row each (no loop over rows).
+bool gen_stage(Gen& g, const PassDesc& d, int s, int NT, std::string& err, int gmode = 0,
+               const char* sync = "__syncthreads();") {
   const StageDesc& sd = d.st[s];
   const int R = d.R, NV = 1 << R;
   const bool gload = gmode & 1, gstore = gmode & 2, use_smem = !(gload && gstore), ftile = gmode & 4;
@@ -55,7 +58,8 @@ bool gen_stage(Gen& g, const PassDesc& d, int s, int NT, std::string& err, int g
       if ((v >> i) & 1) x += " | q" + std::to_string(i);
     return "gst + (" + x + ")";
   };
-  o << "      for (int u = octet; u < " << (1 << sd.nt) << "; u += " << NT / 8 << ") {\n";
+  if (NT) o << "      for (int u = octet; u < " << (1 << sd.nt) << "; u += " << NT / 8 << ") {\n";
+  else o << "      {\n        const int u = octet;\n";
   o << "        unsigned base = lo";
   for (int i = 0; i < sd.nt; ++i) o << " | ((((unsigned)u >> " << i << ") & 1u) << " << (int)sd.tb[i] << ")";
   o << ";\n";
@@ -304,7 +308,7 @@ bool gen_stage(Gen& g, const PassDesc& d, int s, int NT, std::string& err, int g
     else if (ftile) o << "        stn(" << atp(v) << ", " << cur[v] << ");\n";
     else o << "        " << at(v) << " = " << cur[v] << ";\n";
   }
-  o << "      }\n    }\n    __syncthreads();\n";
+  o << "      }\n    }\n    " << sync << "\n";
   return true;
 }
 
@@ -361,13 +365,18 @@ std::string jit_pass_source(const PassDesc& d, std::string& err, int min_blocks,
     err = "register slots out of range";
     return "";
   }
+  const bool pair = threads == kPairForm;
+  if (pair && (set_mode || !pair_form_fits(d))) {
+    err = "the pass does not fit the pair pipeline";
+    return "";
+  }
   const int NT = (threads == 128 || threads == 256) ? threads : tile_pass_threads(d.R);
   const int MINB = d.R == 5 ? 1 : (min_blocks >= 1 && min_blocks <= 4 ? min_blocks : 2);
   const uint32_t nmat = d.mat_elems ? d.mat_elems : 1;
   Gen g;
   std::ostringstream& o = g.o;
   o << "// generated by iq_jitgen (iq-jit-3): NT=" << NT << " sets=" << (set_mode ? 1 : 0)
-    << " narrow=" << (narrow ? 1 : 0) << " M=" << (int)d.M
+    << " narrow=" << (narrow ? 1 : 0) << " pair=" << (pair ? 1 : 0) << " M=" << (int)d.M
     << " c=" << (int)d.c << " R=" << (int)d.R
     << " stages=" << (int)d.nstages << " ops=" << d.nops << "\n";
   o << "#include \"iq_pipe.cuh\"\nusing namespace iqb;\n";
@@ -410,6 +419,22 @@ std::string jit_pass_source(const PassDesc& d, std::string& err, int min_blocks,
     return o.str();
   }
   o << "struct JitMats { double2 m[" << nmat << "]; };\n";
+  if (pair) {
+    o << "struct JitBody {\n  const JitMats& Mt;\n";
+    o << "  __device__ __forceinline__ void operator()(double2* tile, unsigned long long, int grp, int gtid) {\n";
+    o << "    const int lane8 = gtid & 7, octet = gtid >> 3;\n    const unsigned omask = 0xFFu << (gtid & 24);\n"
+      << "    (void)omask;\n";
+    for (int s = 0; s < d.nstages; ++s)
+      if (!gen_stage(g, d, s, 0, err, 0, s + 1 < d.nstages ? "group_sync(grp);" : "")) return "";
+    o << "  }\n};\n";
+    o << "extern \"C\" __global__ void __launch_bounds__(kPairThreads, 1)\n"
+      << "iq_jit_pass(const __grid_constant__ CUtensorMap tm, const __grid_constant__ PassDesc P,\n"
+      << "            const __grid_constant__ JitMats Mt, int* __restrict__ status, int nbuf) {\n"
+      << "  extern __shared__ __align__(1024) unsigned char smem_raw[];\n"
+      << "  JitBody body{Mt};\n"
+      << "  pair_pipeline(tm, P, aligned_tiles(smem_raw), status, body);\n}\n";
+    return o.str();
+  }
   o << "struct JitBody {\n  const JitMats& Mt;\n  int lane8, octet;\n  unsigned omask;\n";
   o << "  __device__ __forceinline__ void operator()(double2* tile, unsigned long long, bool work) {\n";
   o << "    if (!work) return;\n";

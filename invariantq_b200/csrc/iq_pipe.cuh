@@ -416,6 +416,129 @@ __device__ __forceinline__ void tile_pipeline(const CUtensorMap& tm, const PassD
   bulk_wait_all();
 }
 
+// ---- the pair pipeline: one CTA per SM, two groups of 256 threads that each
+// compute a tile, and a producer warp that moves tiles through three buffers.
+//
+// What bounds heavy passes is the sum of a tile's memory time and its FP64 time
+// when every CTA loads, computes and stores its one buffer in turn: three CTAs
+// of 128 threads per SM fall into step and leave either HBM or the FP64 pipe
+// idle.  Here two tiles are always being computed, by 16 warps instead of 12,
+// while the third buffer's store and next load run behind them.  A thread holds
+// one row of 16 amplitudes per stage, so a stage has no loop.  Used for tiles
+// of 2^12 amplitudes in 4 register slots.
+constexpr int kPairGroup = 256;
+constexpr int kPairThreads = 2 * kPairGroup + 32;
+constexpr int kPairBufs = 3;
+
+__device__ __forceinline__ void group_sync(int grp) {
+  asm volatile("barrier.cta.sync %0, %1;" ::"r"(grp + 1), "n"(kPairGroup) : "memory");
+}
+__device__ __forceinline__ bool group_and(int grp, bool v) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %1, 0;\n\t"
+      "barrier.cta.red.and.pred q, %2, %3, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(r)
+      : "r"((uint32_t)v), "r"(grp + 1), "n"(kPairGroup)
+      : "memory");
+  return r != 0;
+}
+
+// body(buf, t, grp, gtid) runs the pass's stages on the resident tile buf
+// (global tile index t) with the 256 threads of group grp (gtid: the thread in
+// it), a group_sync(grp) between stages.  Every wait is bounded; after one gives
+// up, both groups leave their loops, and the producer lets loads in flight land.
+template <class Body>
+__device__ __forceinline__ void pair_pipeline(const CUtensorMap& tm, const PassDesc& P, double2* tiles,
+                                              int* __restrict__ status, Body&& body) {
+  // The tile is loaded (one arrival: the producer's).  A buffer's tiles alternate
+  // between the groups, and a group that skipped phases of a shared barrier could
+  // take an older phase of the same parity for its own, so each group has its own.
+  __shared__ __align__(8) uint64_t bar_full[2 * kPairBufs];
+  __shared__ __align__(8) uint64_t bar_done[kPairBufs];   // the tile is computed (one arrival per warp of its group)
+  __shared__ volatile int abort_flag;
+  const int tid = threadIdx.x;
+  const int lane = tid & 31;
+  if (tid == 0) {
+    for (int b = 0; b < 2 * kPairBufs; ++b) mbar_init(&bar_full[b], 1);
+    for (int b = 0; b < kPairBufs; ++b) mbar_init(&bar_done[b], kPairGroup / 32);
+    abort_flag = 0;
+    fence_mbar_init();
+  }
+  __syncthreads();
+  const uint32_t tile_elems = 1u << P.M;
+  const uint64_t first = blockIdx.x;
+  const uint64_t cnt = (first < P.ntiles) ? (P.ntiles - 1 - first) / gridDim.x + 1 : 0;
+  auto full = [&](uint64_t i) { return &bar_full[i % (2 * kPairBufs)]; };   // tile i: group i % 2, buffer i % 3
+  auto full_phase = [&](uint64_t i) { return (uint32_t)((i / (2 * kPairBufs)) & 1); };
+  if (tid < 2 * kPairGroup) {
+    const int grp = tid / kPairGroup, gtid = tid % kPairGroup;
+    for (uint64_t i = grp; i < cnt; i += 2) {
+      const int b = (int)(i % kPairBufs);
+      const bool ok = bounded_wait(full(i), full_phase(i), &abort_flag, status, DEV_WAIT_LOADED);
+      if (!group_and(grp, ok && !abort_flag)) return;
+      body(tiles + (size_t)b * tile_elems, first + i * gridDim.x, grp, gtid);
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bar_done[b]);
+    }
+    return;
+  }
+  // the producer warp: a tile moves in nissue boxes, dealt to the lanes
+  const int nissue = 1 << (P.nH - P.nbox);
+  const uint32_t box_elems = 1u << (P.c + P.nbox);
+  constexpr int kPer = 4;                                  // nissue <= 128
+  int jc1[kPer], jc3[kPer], jc4[kPer];
+#pragma unroll
+  for (int r = 0; r < kPer; ++r) {
+    const int j = lane + 32 * r;
+    int c2;
+    jc1[r] = jc3[r] = jc4[r] = 0;
+    if (j < nissue) chunk_coords(issue_offset(j, P), P, jc1[r], c2, jc3[r], jc4[r]);
+  }
+  TileCoordMap cmap;
+  tile_coord_map(P, cmap);
+  auto load = [&](uint64_t i) {
+    const int b = (int)(i % kPairBufs);
+    int c1, c2, c3, c4;
+    tile_coords((uint32_t)(first + i * gridDim.x), cmap, c1, c2, c3, c4);
+    if (lane == 0) mbar_arrive_expect_tx(full(i), 16u << P.M);
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < kPer; ++r)
+      if (lane + 32 * r < nissue)
+        tma_load_5d(tiles + (size_t)b * tile_elems + (size_t)(lane + 32 * r) * box_elems, &tm, 0, c1 + jc1[r], 0,
+                    c3 + jc3[r], c4 + jc4[r], full(i));
+  };
+  uint64_t issued = 0;
+  for (; issued < kPairBufs && issued < cnt; ++issued) load(issued);
+  uint64_t j = 0;
+  for (; j < cnt; ++j) {
+    const int b = (int)(j % kPairBufs);
+    const bool ok = bounded_wait(&bar_done[b], (uint32_t)((j / kPairBufs) & 1), &abort_flag, status, DEV_WAIT_COMPUTED);
+    if (!__all_sync(0xffffffffu, ok)) break;
+    int c1, c2, c3, c4;
+    tile_coords((uint32_t)(first + j * gridDim.x), cmap, c1, c2, c3, c4);
+#pragma unroll
+    for (int r = 0; r < kPer; ++r)
+      if (lane + 32 * r < nissue)
+        tma_store_5d(&tm, 0, c1 + jc1[r], 0, c3 + jc3[r], c4 + jc4[r],
+                     tiles + (size_t)b * tile_elems + (size_t)(lane + 32 * r) * box_elems);
+    bulk_commit();
+    if (issued < cnt) {
+      bulk_wait_read_all();
+      __syncwarp();
+      load(issued);
+      ++issued;
+    }
+  }
+  // after an abort: loads issued for tiles not computed land before the CTA exits
+  for (uint64_t i = j; i < issued; ++i) drain_wait(full(i), full_phase(i));
+  bulk_wait_all();
+}
+
 // A pass over nsets arrays laid end to end (one per parameter set), each with
 // its own matrix block and gradient terms (PassDesc::nsets, set_shift,
 // set_mat_stride, grad_stride).  Dynamic shared memory: [tile buffers]

@@ -142,7 +142,7 @@ struct PassDesc {
   // bit the pass touches), so the pass runs over the lower half of each
   // 2^(gap + 1)-amplitude block -- e.g. the psi half of a [psi | lambda] array.
   uint8_t gap;
-  uint8_t pad1;
+  uint8_t run1;                  // length of the first run of adjacent bits in H (see pass_tmap_layout)
   uint8_t H[kMaxTileBits + 3];   // physical bit of tile-local bit c + i (ascending)
   uint64_t ntiles;
   uint32_t nops, pad2;
@@ -254,13 +254,18 @@ IQ_HD uint64_t issue_offset(int j, const PassDesc& P) {
 IQ_HD uint32_t swz(uint32_t j) { return j ^ ((j >> 3) & 7u); }
 
 // 5-D view of the array used by the pass tensor map (dimension 0 innermost,
-// counted in doubles; strides in bytes for dimensions 1..4).  The bits of the
-// amplitude index are cut at the first two tile bits H[0], H[1]:
+// counted in doubles; strides in bytes for dimensions 1..4).  The high tile
+// bits H start with a run of run1 adjacent bits [H0, H0 + run1); the next nbox -
+// run1 are a second run of adjacent bits from H1 = H[run1] (none if nbox ==
+// run1).  The bits of the amplitude index are cut at the runs:
 //   dim0 = 8 amplitudes (128 B, the swizzle span), dim1 = bits [3, H0),
-//   dim2 = bit H0, dim3 = bits (H0, H1), dim4 = bits [H1, nbits).
-// The box takes 2^(c-3) rows of dim1 (the rest of the 2^c chunk) and both
-// values of H0 and H1, so one copy moves 2^(c + nbox) amplitudes; the other
-// tile bits are enumerated by issues.
+//   dim2 = the first run, dim3 = the bits between the runs (without a second
+//   run: all above the first), dim4 = bits [H1, nbits).
+// The box takes 2^(c-3) rows of dim1 (the rest of the 2^c chunk) and every
+// value of both runs, so one copy moves 2^(c + nbox) amplitudes; the other tile
+// bits are enumerated by issues.  The bits a pass works on mostly form one or
+// two runs, so a tile of 2^12 moves in 1 to 8 copies where two bits per box took
+// 64, whose issue bound the light passes of a producer warp.
 IQ_HD void pass_tmap_layout(const PassDesc& d, int nbits, uint64_t gd[5], uint64_t gs[4], uint32_t box[5]) {
   if (d.gap) nbits = d.gap + 1;   // the map covers the whole 2^(gap + 1) block of each array
   const int c = d.c;
@@ -271,57 +276,64 @@ IQ_HD void pass_tmap_layout(const PassDesc& d, int nbits, uint64_t gd[5], uint64
   box[0] = 16;
   box[1] = 1u << (c - 3);
   const uint64_t sets = d.nsets > 1 ? d.nsets : 1;   // sets extend the top dimension
-  if (d.nbox == 2) {
-    const int h0 = d.H[0], h1 = d.H[1];
-    gd[1] = 1ull << (h0 - 3); gd[2] = 2; gd[3] = 1ull << (h1 - h0 - 1); gd[4] = (1ull << (nbits - h1)) * sets;
-    gs[1] = (1ull << h0) * E; gs[2] = (1ull << (h0 + 1)) * E; gs[3] = (1ull << h1) * E;
-    box[2] = 2; box[3] = 1; box[4] = 2;
-  } else if (d.nbox == 1) {
-    const int h0 = d.H[0];
-    gd[1] = 1ull << (h0 - 3); gd[2] = (1ull << (nbits - h0)) * sets; gd[3] = 1; gd[4] = 1;
-    gs[1] = (1ull << h0) * E; gs[2] = top; gs[3] = top;
-    box[2] = 2; box[3] = 1; box[4] = 1;
-  } else {
+  if (d.nbox == 0) {
     gd[1] = (1ull << (nbits - 3)) * sets; gd[2] = 1; gd[3] = 1; gd[4] = 1;
     gs[1] = top; gs[2] = top; gs[3] = top;
     box[2] = 1; box[3] = 1; box[4] = 1;
+    return;
+  }
+  const int h0 = d.H[0], k1 = d.run1, k2 = d.nbox - k1;
+  gd[1] = 1ull << (h0 - 3);
+  gs[1] = (1ull << h0) * E;
+  gd[2] = 1ull << k1;
+  box[2] = 1u << k1;
+  gs[2] = (1ull << (h0 + k1)) * E;
+  box[3] = 1;
+  if (k2) {
+    const int h1 = d.H[k1];
+    gd[3] = 1ull << (h1 - h0 - k1); gd[4] = (1ull << (nbits - h1)) * sets;
+    gs[3] = (1ull << h1) * E;
+    box[4] = 1u << k2;
+  } else {
+    gd[3] = (1ull << (nbits - h0 - k1)) * sets; gd[4] = 1;
+    gs[3] = top;
+    box[4] = 1;
   }
 }
 
 // Tensor-map coordinates (dims 1..4) of the copy whose first amplitude is A
 // (A has zeros in bits [0, c) and at the box bits).
 IQ_HD void chunk_coords(uint64_t A, const PassDesc& P, int& c1, int& c2, int& c3, int& c4) {
-  if (P.nbox == 2) {
-    const int h0 = P.H[0], h1 = P.H[1];
-    c1 = (int)((A >> 3) & ((1ULL << (h0 - 3)) - 1));
-    c2 = 0;
-    c3 = (int)((A >> (h0 + 1)) & ((1ULL << (h1 - h0 - 1)) - 1));
-    c4 = (int)(A >> h1);
-  } else if (P.nbox == 1) {
-    const int h0 = P.H[0];
-    c1 = (int)((A >> 3) & ((1ULL << (h0 - 3)) - 1));
-    c2 = (int)(A >> h0);
-    c3 = 0;
-    c4 = 0;
-  } else {
+  c2 = c3 = c4 = 0;
+  if (P.nbox == 0) {
     c1 = (int)(A >> 3);
-    c2 = c3 = c4 = 0;
+    return;
+  }
+  const int h0 = P.H[0], k1 = P.run1;
+  c1 = (int)((A >> 3) & ((1ULL << (h0 - 3)) - 1));
+  if (P.nbox > k1) {
+    const int h1 = P.H[k1];
+    c3 = (int)((A >> (h0 + k1)) & ((1ULL << (h1 - h0 - k1)) - 1));
+    c4 = (int)(A >> h1);
+  } else {
+    c3 = (int)(A >> (h0 + k1));
   }
 }
 
 // Tensor-map coordinates of tile t's first copy, computed from t directly
 // (equal to chunk_coords(tile_base(t, P), P)).  The tile index's bits fill the
-// non-tile bit positions in order; cut at H[0] and H[1] they give: the low
-// n1 = H0 - c bits -> dim 1 (above the chunk's 2^(c-3) rows), the next
-// n3 = H1 - H0 - 1 bits -> dim 3, the rest -> the top dimension with the
-// higher tile bits as zero gaps.  Built once per thread; 32-bit arithmetic.
+// non-tile bit positions in order; cut at the runs they give: the low n1 = H0 -
+// c bits -> dim 1 (above the chunk's 2^(c-3) rows), the next n3 -> dim 3 (the
+// bits between the runs, or all the rest), the rest -> dim 4 with the second
+// run's and the higher tile bits as zero gaps.  Built once per thread; 32-bit
+// arithmetic.
 struct TileCoordMap {
   int nbox;
   int n1, sh1;            // dim 1: (t & ((1 << n1) - 1)) << sh1
-  int n3;                 // dim 3 (nbox 2): (t >> n1) & ((1 << n3) - 1)
-  int shhi;               // top-dimension bits start at t >> shhi
+  int n3;                 // dim 3: (t >> n1) & ((1 << n3) - 1); -1: (t >> n1) with the gap
+  int shhi;               // dim 4's bits start at t >> shhi
   int ngap;
-  uint8_t gap[kMaxTileBits + 1];   // ascending zero positions in the top coordinate
+  uint8_t gap[kMaxTileBits + 1];   // ascending zero positions in dim 4 (n3 = -1: in dim 3)
   int gap1;               // nbox 0: zero position in dim 1 (-1: none)
 };
 
@@ -334,14 +346,14 @@ IQ_HD void tile_coord_map(const PassDesc& P, TileCoordMap& m) {
     if (P.gap) m.gap1 = P.gap - 3;
     return;
   }
-  const int h0 = P.H[0];
+  const int h0 = P.H[0], k1 = P.run1;
   m.n1 = h0 - P.c;
   m.sh1 = P.c - 3;
-  const int lo = (P.nbox == 2) ? P.H[1] : h0;   // the top dimension starts at this bit
-  m.n3 = (P.nbox == 2) ? P.H[1] - h0 - 1 : 0;
-  m.shhi = m.n1 + m.n3;
-  m.gap[m.ngap++] = 0;                          // bit `lo` itself is a tile bit
-  for (int i = P.nbox; i < P.nH; ++i) m.gap[m.ngap++] = (uint8_t)(P.H[i] - lo);
+  const bool two = P.nbox > k1;
+  const int lo = two ? P.H[k1] : h0 + k1;       // dim 4 (or dim 3) starts at this bit
+  m.n3 = two ? lo - h0 - k1 : -1;
+  m.shhi = m.n1 + (two ? m.n3 : 0);
+  for (int i = k1; i < P.nH; ++i) m.gap[m.ngap++] = (uint8_t)(P.H[i] - lo);
   if (P.gap) m.gap[m.ngap++] = (uint8_t)(P.gap - lo);   // above every tile bit: last
 }
 
@@ -361,11 +373,11 @@ IQ_HD void tile_coords(uint32_t t, const TileCoordMap& m, int& c1, int& c2, int&
       const int g = m.gap[i];
       x = ((x >> g) << (g + 1)) | (x & ((1u << g) - 1u));
     }
-  if (m.nbox == 2) {
+  if (m.n3 >= 0) {
     c3 = (int)((t >> m.n1) & ((1u << m.n3) - 1u));
     c4 = (int)x;
   } else {
-    c2 = (int)x;
+    c3 = (int)x;
   }
 }
 
@@ -383,7 +395,8 @@ int plan_passes(const SchedParams& p, const std::vector<SchedOp>& ops, std::vect
 // that is not specialised (adjoint steps, several parameter sets).
 // min_blocks: resident CTAs per SM the kernel's register budget is sized for
 // (launch bounds; 2 when out of 1..4; always 1 for R = 5); threads: CTA size
-// (128 or 256; otherwise tile_pass_threads(R)).
+// (128 or 256; kPairForm: the pair pipeline, for passes pair_form_fits takes;
+// otherwise tile_pass_threads(R)).
 // set_mode: the form for passes over several parameter sets and adjoint steps
 // (matrices staged per set in shared memory, gradient accumulators; the
 // interpreting kernel's launch arguments); otherwise matrices are a kernel
@@ -392,6 +405,13 @@ int plan_passes(const SchedParams& p, const std::vector<SchedOp>& ops, std::vect
 // widening to FP64, and the stages exchange through a float2 shared tile
 // (arguments: pass, matrices, state, gradient partials; launched with
 // jit_launch_narrow).
+constexpr int kPairForm = 512;
+// Time of a pass of the pair pipeline on a large array, in milliseconds at 2^30
+// amplitudes: the larger of its HBM traffic and 0.78 times the sum of its FP64
+// multiply-adds (0.065 ms each per amplitude) and its shared-memory round trips
+// (1.02 ms per stage and for the copies) -- within 8 % of passes of 2 to 6 stages.
+double pass_time_model(const PassDesc& d);
+inline bool pair_form_fits(const PassDesc& d) { return d.M == 12 && d.R == 4 && d.nH - d.nbox <= 7; }
 std::string jit_pass_source(const PassDesc& d, std::string& err, int min_blocks = 2, int threads = 0,
                             bool set_mode = false, bool narrow = false);
 // Compact byte string of everything jit_pass_source's output depends on

@@ -362,7 +362,7 @@ struct Engine : HandleRes {
   // measured: 78 passes, ~627 ms, against 110 passes and ~776 ms with the
   // interpreting kernel's 11 / 5 / 120 / 4 CTAs).  Interpreting kernel: tiles of
   // 2^11 holding 5, budget 120, 2 CTAs per SM with three buffers.
-  bool set_M = false, set_c = false, set_budget = false, set_nbuf = false, set_ctas = false;
+  bool set_M = false, set_c = false, set_budget = false, set_nbuf = false, set_ctas = false, set_stages = false;
 
   bool spec_style() const {
     return plan_style == 2 || (plan_style == 0 && jit && (jit >= 2 || nbits >= kJitMinBits) && !eager && nbits >= 7);
@@ -442,6 +442,7 @@ struct Engine : HandleRes {
     set_budget = getenv("IQ_PASS_BUDGET") != nullptr;
     set_nbuf = getenv("IQ_NBUF") != nullptr;
     set_ctas = getenv("IQ_CTAS_PER_SM") != nullptr;
+    set_stages = getenv("IQ_MAX_STAGES") != nullptr;
     eager = env_int("IQ_EAGER", 0);
     return reset_state();
   }
@@ -565,12 +566,54 @@ struct Engine : HandleRes {
     TileLaunch tl{};                     // launch settings of the passes
   };
 
+  // The pair pipeline unless an option asks for another CTA shape.  26 qubits,
+  // three CTAs of one buffer -> pair pipeline: passes of 3 stages 0.377 -> 0.350
+  // ms, 4 stages 0.478 -> 0.412, a 30-qubit circuit of depth 20 289 -> 273 ms.
+  bool may_pair() const { return jit_threads == 0 && !set_ctas && !set_nbuf; }
+
+  // Stage limits tried for arrays whose passes are long enough to pay for the
+  // planning (2^kPlanTrialBits amplitudes: ~0.6 ms a pass, a plan ~1 ms): below
+  // four stages a pass of the pair pipeline is bound by HBM, so circuits with
+  // much work per pass run faster as more passes of fewer stages (30 qubits,
+  // depth 20: 273 ms at up to 8 stages, 249 at 5, 253 at 4; depth 6: 87, 86, 79).
+  // Which limit wins depends on the circuit: the cheapest by pass_time_model.
+  static constexpr int kPlanTrialBits = 27;
+  bool plan_program(SchedParams p, const std::vector<SchedOp>& fused, bool spec, std::vector<PassPlan>& plans,
+                    std::string& err) {
+    std::vector<int> limits{p.max_stages};
+    if (spec && nbits >= kPlanTrialBits && may_pair() && !set_stages && jit)
+      for (int ms : {4, 5})
+        if (ms < p.max_stages) limits.push_back(ms);
+    double best = 0.0;
+    for (size_t i = 0; i < limits.size(); ++i) {
+      std::vector<PassPlan> trial;
+      p.max_stages = limits[i];
+      if (plan_passes(p, fused, trial, err) < 0) {
+        if (i == 0) return false;
+        continue;
+      }
+      if (spec) merge_stage_diagonals(trial, fused);
+      double t = 0.0;
+      for (const PassPlan& pl : trial) t += pass_time_model(pl.desc);
+      if (i == 0 || t < best) {
+        best = t;
+        plans.swap(trial);
+      }
+    }
+    return true;
+  }
+
   // kernels specialised to the program's passes: compiled now (recorded
   // programs, jit 2) or taken from those already compiled (flushes)
   void attach_jit(Program& pg, bool own, std::vector<cplx64>& packed) {
     if (!jit || (jit == 1 && nbits < kJitMinBits) || pg.plans.empty()) return;
     std::vector<const PassDesc*> ds;
-    for (auto& pl : pg.plans) ds.push_back(&pl.desc);
+    bool pair = may_pair();
+    for (auto& pl : pg.plans) {
+      ds.push_back(&pl.desc);
+      pair = pair && pair_form_fits(pl.desc);
+    }
+    const int jit_threads = pair ? kPairForm : this->jit_threads;
     if (own || jit >= 2) {
       std::string err;
       if (!jit_prepare(ds, pg.jit, err, pg.tl.ctas_per_sm, jit_threads)) {
@@ -616,11 +659,10 @@ struct Engine : HandleRes {
       p.nbits = nbits;
       p.R = std::min(5, std::max(sp.R, maxk));
       std::string err;
-      if (plan_passes(p, fused, pg.plans, err) < 0) {
+      if (!plan_program(p, fused, spec, pg.plans, err)) {
         set_error(E_STATE, "scheduler: %s", err.c_str());
         return false;
       }
-      if (spec) merge_stage_diagonals(pg.plans, fused);
       pack_pass_matrices(pg.plans, pool.data(), packed);
       src = packed.data();
       nsrc = packed.size();
@@ -1401,7 +1443,7 @@ int iq_handle_set_option(void* h, const char* key, double v) {
   const int iv = (int)v;
   if (!strcmp(key, "tile_bits")) { if (iv < 7 || iv > kMaxTileBits) return -1; e->sp.M = iv; e->set_M = true; }
   else if (!strcmp(key, "chunk_bits")) { if (iv < 3 || iv > 7) return -1; e->sp.c = iv; e->set_c = true; }
-  else if (!strcmp(key, "max_stages")) { if (iv < 1 || iv > kMaxStages) return -1; e->sp.max_stages = iv; }
+  else if (!strcmp(key, "max_stages")) { if (iv < 1 || iv > kMaxStages) return -1; e->sp.max_stages = iv; e->set_stages = true; }
   else if (!strcmp(key, "budget")) { if (v <= 0) return -1; e->sp.budget = v; e->set_budget = true; }
   else if (!strcmp(key, "nbuf")) { if (iv < 1 || iv > 4) return -1; e->tl.nbuf = iv; e->set_nbuf = true; }
   else if (!strcmp(key, "reg_slots")) { if (iv < 3 || iv > 5) return -1; e->sp.R = iv; }

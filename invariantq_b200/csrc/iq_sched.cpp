@@ -428,8 +428,15 @@ int plan_passes(const SchedParams& p, const std::vector<SchedOp>& ops, std::vect
     d.c = (uint8_t)c;
     d.R = (uint8_t)p.R;
     d.nH = (uint8_t)H.size();
-    d.nbox = (uint8_t)std::min<int>(2, (int)H.size());
     for (size_t i = 0; i < H.size(); ++i) d.H[i] = (uint8_t)H[i];
+    // the copies' boxes span the first two runs of adjacent high bits (at most 256 entries per dimension)
+    auto run = [&](size_t from) {
+      size_t k = 0;
+      while (from + k < H.size() && k < 8 && H[from + k] == H[from] + (int)k) ++k;
+      return (int)k;
+    };
+    d.run1 = (uint8_t)run(0);
+    d.nbox = (uint8_t)(d.run1 + run(d.run1));
     d.ntiles = 1ULL << (nb - M);
     d.nstages = (uint8_t)pb.stages.size();
     d.ngrad = 0;
@@ -1660,6 +1667,30 @@ void merge_stage_diagonals(std::vector<PassPlan>& plans, const std::vector<Sched
     pl.src = nsrc;
     pl.diag = diag;
   }
+}
+
+double pass_time_model(const PassDesc& d) {
+  double f = 0.0;   // real multiply-adds per amplitude
+  for (uint32_t i = 0; i < d.nops; ++i) {
+    const OpDesc& o = d.ops[i];
+    const bool unit = o.flags & OPF_UNIT_PHASE;
+    const int rows = 1 << o.k;
+    switch (o.kind) {
+      case OP_M1R: case OP_M2R:
+        if (!unit) f += 4.0 * (rows - __builtin_popcount(o.urows & ((1u << rows) - 1))) / rows;
+        break;
+      case OP_M1L: f += unit ? 0.0 : 4.0; break;
+      case OP_R1R: case OP_R1L: f += 2.0; break;
+      case OP_D1R: case OP_D1L: f += (o.flags & OPF_REAL) ? 4.0 : 8.0; break;
+      case OP_N1R: f += 6.0; break;
+      case OP_X2R: f += ((o.flags & 1) ? 2.0 : 4.0) + ((o.flags & 2) ? 1.0 : 2.0); break;
+      case OP_DGR: f += 4.0 * ((1 << d.R) - __builtin_popcount(o.gidx)) / (1 << d.R); break;
+      case OP_GDZ: f += 1.4; break;
+      case OP_GRAD2: f += (o.perm == 2 || o.flags) ? 4.0 : 6.0; break;
+      default: f += 4.0 * rows; break;
+    }
+  }
+  return std::max(5.75, 0.78 * (0.065 * f + 1.02 * (d.nstages + 1)));
 }
 
 void pack_recipe(std::vector<PassPlan>& plans, PackRecipe& r) {
