@@ -242,6 +242,74 @@ bool make_shape(const Cfg& cfg, int nbits, const std::vector<SchedOp>& fused, si
   return true;
 }
 
+// Shapes outlive a call: a variational loop plans its circuit once (20 qubits, 8
+// layers: ~0.3 ms of a 1.6 ms gradient).  Found by the whole operation structure
+// and the settings, so any circuit of the same gates shares them; at most
+// kMaxShapes, the least recently used goes first; iq_adjoint_release drops them.
+constexpr size_t kMaxShapes = 64;
+struct ShapeEntry {
+  uint64_t key;
+  uint64_t used;
+  std::shared_ptr<const Shape> shape;
+};
+std::mutex g_shape_mu;
+std::vector<ShapeEntry>* g_shapes = new std::vector<ShapeEntry>();
+uint64_t g_shape_clock = 0;
+
+uint64_t shape_key(const Cfg& cfg, int dev, int nbits, const std::vector<SchedOp>& ops, size_t pool_size, int num_sms) {
+  uint64_t h = 1469598103934665603ull;
+  auto put = [&](uint64_t v) { h = (h ^ v) * 1099511628211ull; };
+  for (uint64_t v : {(uint64_t)dev, (uint64_t)nbits, (uint64_t)pool_size, (uint64_t)num_sms, (uint64_t)cfg.sp.M,
+                     (uint64_t)cfg.sp.c, (uint64_t)cfg.sp.R, (uint64_t)cfg.sp.max_stages, (uint64_t)cfg.tl.nbuf,
+                     (uint64_t)cfg.tl.ctas_per_sm, (uint64_t)cfg.jit, (uint64_t)cfg.c64, (uint64_t)ops.size()})
+    put(v);
+  for (double v : {cfg.sp.budget, cfg.sp.grad_cost}) {
+    uint64_t b;
+    std::memcpy(&b, &v, 8);
+    put(b);
+  }
+  for (const SchedOp& o : ops) {
+    put(o.k | (uint64_t)o.mono << 8 | (uint64_t)o.perm << 16 | (uint64_t)o.unit << 24 | (uint64_t)o.norm << 32 |
+        (uint64_t)o.rot << 40 | (uint64_t)o.urows << 48 | (uint64_t)o.nrows << 56);
+    put(o.grad | (uint64_t)o.xpat << 8 | (uint64_t)o.realm << 16 | (uint64_t)o.gen << 24 | (uint64_t)o.gidx << 32);
+    put(o.mat | (uint64_t)o.dense << 32);
+    for (int i = 0; i < o.k; ++i) put(o.q[i]);
+  }
+  return h;
+}
+
+std::shared_ptr<const Shape> shape_for(const Cfg& cfg, int dev, int nbits, const std::vector<SchedOp>& ops,
+                                       size_t pool_size, int num_sms, int ngrads, std::string& err) {
+  const uint64_t key = shape_key(cfg, dev, nbits, ops, pool_size, num_sms);
+  auto find = [&]() -> std::shared_ptr<const Shape> {   // g_shape_mu held; the key's whole structure is compared
+    for (ShapeEntry& e : *g_shapes)
+      if (e.key == key && e.shape->nbits == nbits && matches(*e.shape, ops, pool_size)) {
+        e.used = ++g_shape_clock;
+        return e.shape;
+      }
+    return nullptr;
+  };
+  {
+    std::lock_guard<std::mutex> g(g_shape_mu);
+    if (auto s = find()) return s;
+  }
+  auto s = std::make_shared<Shape>();
+  if (!make_shape(cfg, nbits, ops, pool_size, num_sms, *s, err)) return nullptr;
+  s->ngrads = ngrads;
+  if (cfg.jit || cfg.c64) {   // kernels that could not be had this time are tried again at the next call
+    bool all = s->jit.size() == s->plans.size();
+    for (const JitKernel* k : s->jit) all = all && k;
+    if (!all) return s;
+  }
+  std::lock_guard<std::mutex> g(g_shape_mu);
+  if (auto other = find()) return other;   // another thread planned it meanwhile
+  if (g_shapes->size() >= kMaxShapes)
+    g_shapes->erase(std::min_element(g_shapes->begin(), g_shapes->end(),
+                                     [](const ShapeEntry& a, const ShapeEntry& b) { return a.used < b.used; }));
+  g_shapes->push_back({key, ++g_shape_clock, s});
+  return s;
+}
+
 // ---------------------------------------------------------------- circuits
 
 struct Circuit {
@@ -257,7 +325,7 @@ struct Circuit {
   std::mutex mu;
   bool planned = false;
   std::string plan_err;
-  std::unique_ptr<Shape> fw, bw;
+  std::shared_ptr<const Shape> fw, bw;
 };
 
 // Forward / backward operation lists and matrix pools of one parameter set.  A
@@ -729,13 +797,10 @@ bool launch_job(Workspace& w, const Cfg& cfg, Circuit& c, size_t set0, size_t ns
     t0 = std::chrono::steady_clock::now();
     if (!c.planned) {
       c.planned = true;
-      c.fw.reset(new Shape);
-      if (!make_shape(cfg, c.n, jo[0].fw, jo[0].fpool.size(), w.num_sms, *c.fw, c.plan_err)) c.fw.reset();
-      if (c.fw && want_grad) {
-        c.bw.reset(new Shape);
-        if (!make_shape(cfg, joint_bits(c.n), jo[0].bw, jo[0].bpool.size(), w.num_sms, *c.bw, c.plan_err)) c.bw.reset();
-        else c.bw->ngrads = (int)jo[0].grad_param.size();
-      }
+      c.fw = shape_for(cfg, w.device, c.n, jo[0].fw, jo[0].fpool.size(), w.num_sms, 0, c.plan_err);
+      if (c.fw && want_grad)
+        c.bw = shape_for(cfg, w.device, joint_bits(c.n), jo[0].bw, jo[0].bpool.size(), w.num_sms,
+                         (int)jo[0].grad_param.size(), c.plan_err);
     }
     st.host_ns += since(t0);
     if (!c.fw || (want_grad && !c.bw)) {
@@ -885,7 +950,7 @@ int run_batch(std::vector<std::unique_ptr<Circuit>>& circs, int nstreams, bool w
       resident_sets += c->nsets;
       continue;
     }
-    plan_hamiltonian(c->n, c->ham.groups, c->ham.zmask.data(), c->ham.coef.data(), c64 ? 1 : kHamMaxSweeps, c->ham.plan);
+    plan_hamiltonian(c->n, c->ham.groups, c->ham.zmask.data(), c->ham.coef.data(), (c64 || c->n <= kHamOneSweepBits) ? 1 : kHamMaxSweeps, c->ham.plan);
     c->ham.tables.resize(c->ham.plan.table_bytes() / 8 + 1);
     c->ham.plan.pack(c->ham.tables.data());
     const double per_set = (c64 ? 8.0 : 16.0) * std::ldexp(1.0, joint_bits(c->n));
@@ -1297,6 +1362,10 @@ int iq_ansatz_energy(const iq_adjoint_circuit* circuit) { return run_circuits(ci
 int iq_adjoint_release(void) {
   resident_release();
   release_handle_resources();
+  {
+    std::lock_guard<std::mutex> g(g_shape_mu);
+    g_shapes->clear();
+  }
   std::vector<Workspace*> ws;
   {
     std::lock_guard<std::mutex> g(g_pool_mu);

@@ -64,14 +64,15 @@ __device__ __forceinline__ double block_total(double v, double* red) {
   return t;
 }
 
-// Shared memory of a sweep: [tile][strings' signed coefficients][strings' sign words: one bit per thread][items].
+// Shared memory of a sweep: [tile][strings: signed coefficients, coefficients, Z and X masks][items][strings' sign
+// words: one bit per thread].
 // Strings past kHamSmemTerms are summed from global memory, sign by sign.
 constexpr int kHamSmemTerms = 512;
 __host__ __device__ inline int ham_smem_terms(const HamSweep& s) {
   return s.term1 - s.term0 <= kHamSmemTerms ? s.term1 - s.term0 : 0;
 }
 size_t ham_smem_bytes(const HamSweep& s, size_t amp) {
-  return (amp << kHamM) + (size_t)ham_smem_terms(s) * (8 + kHamThreads / 8) + (size_t)(s.item1 - s.item0) * sizeof(HamItem);
+  return (amp << kHamM) + (size_t)ham_smem_terms(s) * (32 + kHamThreads / 8) + (size_t)(s.item1 - s.item0) * sizeof(HamItem);
 }
 
 // One sweep.  blockIdx.y = set: psi + set * pstride, lam + set * lstride.
@@ -98,7 +99,10 @@ ham_sweep_kernel(const T* __restrict__ psi, uint64_t pstride, const __grid_const
   T* const tile = reinterpret_cast<T*>(ham_smem);
   const int nterms = ham_smem_terms(P);
   double* const sc = reinterpret_cast<double*>(ham_smem + (sizeof(T) << kHamM));
-  HamItem* const items = reinterpret_cast<HamItem*>(sc + nterms);
+  double* const c0 = sc + nterms;                      // the strings' coefficients and masks
+  uint64_t* const sz = reinterpret_cast<uint64_t*>(c0 + nterms);
+  uint64_t* const sx = sz + nterms;
+  HamItem* const items = reinterpret_cast<HamItem*>(sx + nterms);
   uint32_t* const words = reinterpret_cast<uint32_t*>(items + (P.item1 - P.item0));
   __shared__ double red[kHamThreads / 32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -123,8 +127,14 @@ ham_sweep_kernel(const T* __restrict__ psi, uint64_t pstride, const __grid_const
     const int words_of = (int)(sizeof(HamItem) / 4) * (P.item1 - P.item0);
     const uint32_t* src = reinterpret_cast<const uint32_t*>(g_items + P.item0);
     for (int i = tid; i < words_of; i += kHamThreads) reinterpret_cast<uint32_t*>(items)[i] = src[i];
+    for (int k = tid; k < nterms; k += kHamThreads) {
+      sz[k] = tz[P.term0 + k];
+      sx[k] = txm[P.term0 + k];
+      c0[k] = tc[P.term0 + k];
+    }
+    __syncthreads();
     for (int k = 0; k < nterms; ++k) {
-      const uint32_t w = __ballot_sync(0xffffffffu, __popcll(tphys & tz[P.term0 + k]) & 1);
+      const uint32_t w = __ballot_sync(0xffffffffu, __popcll(tphys & sz[k]) & 1);
       if (lane == 0) words[k * (kHamThreads / 32) + warp] = w;
     }
   }
@@ -153,8 +163,8 @@ ham_sweep_kernel(const T* __restrict__ psi, uint64_t pstride, const __grid_const
       acc[v] = (P.add && x < dim) ? wide(lam[x]) : make_double2(0.0, 0.0);
     }
     for (int k = tid; k < nterms; k += kHamThreads) {
-      const double c = tc[P.term0 + k];
-      sc[k] = flips(base, P.term0 + k) ? -c : c;
+      const bool neg = (__popcll((base ^ frame.x) & sz[k]) + __popcll(sx[k] & frame.y)) & 1;
+      sc[k] = neg ? -c0[k] : c0[k];
     }
     __syncthreads();
     // sum of the strings [k0, k1) at the thread's amplitude 0
@@ -250,7 +260,7 @@ ham_sweep_kernel(const T* __restrict__ psi, uint64_t pstride, const __grid_const
 // the largest sweep: 64 groups of two items, kHamSmemTerms strings
 template <class T>
 constexpr size_t ham_smem_limit() {
-  return (sizeof(T) << kHamM) + (size_t)kHamSmemTerms * (8 + kHamThreads / 8) + 2 * kMaxHamGroups * sizeof(HamItem);
+  return (sizeof(T) << kHamM) + (size_t)kHamSmemTerms * (32 + kHamThreads / 8) + 2 * kMaxHamGroups * sizeof(HamItem);
 }
 
 template <class T>

@@ -100,6 +100,8 @@ struct HamTerms {
 };
 // The Hamiltonian sweeps of iq_ham.cu: a plan (host), its tables (device) and the launch.
 constexpr int kHamMaxSweeps = 6;
+// up to this size the state stays in the caches: the few flips beyond a tile gather in the one sweep
+constexpr int kHamOneSweepBits = 18;
 constexpr int kHamBlocks = 2 * 148;    // CTAs per set and sweep: two tiles of 64 KiB fit an SM
 // partial sums a launch needs per set (twice that with the imaginary part)
 constexpr size_t kHamPartials = (size_t)kHamMaxSweeps * kHamBlocks;

@@ -86,11 +86,13 @@ int classify_xpattern(const double* m) {
 
 namespace {
 
-struct Stage {
+struct StageBits {                 // what placing an operation reads and changes (copied for each trial)
   int S[kMaxK];
   int nS = 0;
   uint64_t lanereq = 0;            // bits that 1q lane operations of this stage act on
   bool dk = false;                 // holds one dense k>=3 block; closed
+};
+struct Stage : StageBits {
   std::vector<int> ops;
 };
 
@@ -101,12 +103,12 @@ struct PassBuilder {
   bool allow_new = true;   // false: an operation joins the current stage or waits
   explicit PassBuilder(const SchedParams& pp, int cc) : p(pp), c(cc) {}
 
-  static bool inS(const Stage& s, int b) {
+  static bool inS(const StageBits& s, int b) {
     for (int i = 0; i < s.nS; ++i)
       if (s.S[i] == b) return true;
     return false;
   }
-  int lowcount(const Stage& s) const {
+  int lowcount(const StageBits& s) const {
     int n = 0;
     for (int i = 0; i < s.nS; ++i) n += s.S[i] < c;
     return n;
@@ -116,7 +118,7 @@ struct PassBuilder {
   // lanes can then use the first tile bit above the chunk, whose swizzled
   // image also has a low bit set, so the octet's accesses can stay on eight
   // bank groups (the lane choice below takes the best rank it finds).
-  int lowlimit(const Stage& s, bool no_lanes_after) const {
+  int lowlimit(const StageBits& s, bool no_lanes_after) const {
     return c - kLaneBits + ((no_lanes_after && s.lanereq == 0) ? 1 : 0);
   }
   // Whether a stage without lane operations whose slots also take the nn bits
@@ -126,7 +128,7 @@ struct PassBuilder {
   // slots.  Tile-local bits >= c are high tile bits chosen when the pass is
   // finalised; physical bit j stands in for them (it is the one they are when
   // it is local in the pass).
-  bool lanes_feasible(const Stage& s, const int* add, int nn) const {
+  bool lanes_feasible(const StageBits& s, const int* add, int nn) const {
     for (int k = 0; k < 3; ++k) {
       bool free_member = false;
       for (int j = k; j < 6 && !free_member; j += 3) {
@@ -142,7 +144,7 @@ struct PassBuilder {
   }
   // Register slots take at most c - 3 of the chunk bits [0, c), so three lane
   // bits always remain inside the chunk; lane operations name up to 3 of them.
-  bool tryAdd(Stage& s, const SchedOp& op) const {
+  bool tryAdd(StageBits& s, const SchedOp& op) const {
     if (s.dk) return false;
     if (op.k == 1) {
       const int b = op.q[0];
@@ -181,7 +183,7 @@ struct PassBuilder {
       // current stage can take the select bit into slot 0 (swapped there, or
       // inserted when a slot is free and the chunk-bit limit allows)
       if (!stages.empty() && !stages.back().dk) {
-        Stage trial = stages.back();
+        StageBits trial = stages.back();
         const int sel = op.q[0];
         bool ready = trial.nS > 0 && trial.S[0] == sel;
         if (!ready && inS(trial, sel)) {
@@ -196,8 +198,8 @@ struct PassBuilder {
           ready = true;
         }
         if (ready && tryAdd(trial, op)) {
-          trial.ops.push_back(idx);
-          stages.back() = trial;
+          static_cast<StageBits&>(stages.back()) = trial;
+          stages.back().ops.push_back(idx);
           return true;
         }
       }
@@ -206,7 +208,7 @@ struct PassBuilder {
       s.S[s.nS++] = op.q[0];
       if (!tryAdd(s, op)) return false;
       s.ops.push_back(idx);
-      stages.push_back(s);
+      stages.push_back(std::move(s));
       return true;
     }
     if (op.k >= 3) {
@@ -216,14 +218,14 @@ struct PassBuilder {
       s.dk = true;
       for (int i = 0; i < op.k; ++i) s.S[s.nS++] = op.q[i];
       s.ops.push_back(idx);
-      stages.push_back(s);
+      stages.push_back(std::move(s));
       return true;
     }
     if (!stages.empty()) {
-      Stage trial = stages.back();
+      StageBits trial = stages.back();
       if (tryAdd(trial, op)) {
-        trial.ops.push_back(idx);
-        stages.back() = trial;
+        static_cast<StageBits&>(stages.back()) = trial;
+        stages.back().ops.push_back(idx);
         return true;
       }
     }
@@ -231,7 +233,7 @@ struct PassBuilder {
     Stage s;
     if (!tryAdd(s, op)) return false;
     s.ops.push_back(idx);
-    stages.push_back(s);
+    stages.push_back(std::move(s));
     return true;
   }
 };
@@ -327,6 +329,9 @@ int plan_passes(const SchedParams& p, const std::vector<SchedOp>& ops, std::vect
   for (int i = 0; i < nops; ++i)
     for (int j = dep_first(i); j < ops[i].k; ++j) q[ops[i].q[j]].push_back(i);
   std::vector<int> headcnt(nops, 0);
+  struct Facts { uint64_t mask; double cost; int elems; };   // looked up once per pass and operation below
+  std::vector<Facts> facts(nops);
+  for (int i = 0; i < nops; ++i) facts[i] = {opmask(ops[i]), op_cost(ops[i], p.grad_cost), op_mat_elems(ops[i])};
   std::set<int> ready;
   for (int b = 0; b < nb; ++b)
     if (!q[b].empty()) {
@@ -374,13 +379,13 @@ int plan_passes(const SchedParams& p, const std::vector<SchedOp>& ops, std::vect
           for (auto it = ready.begin(); it != ready.end();) {
             const int i = *it;
             const SchedOp& o = ops[i];
-            const double oc = op_cost(o, p.grad_cost);
-            if ((opmask(o) & ~local) == 0 && (int)taken.size() < kMaxPassOps &&
-                mat_elems + op_mat_elems(o) <= kSmemMatElems && (taken.empty() || cost + oc <= p.budget) &&
+            const double oc = facts[i].cost;
+            if ((facts[i].mask & ~local) == 0 && (int)taken.size() < kMaxPassOps &&
+                mat_elems + facts[i].elems <= kSmemMatElems && (taken.empty() || cost + oc <= p.budget) &&
                 (!o.grad || ngrad < kMaxPassGrads) && pb.place(i, o)) {
               taken.push_back(i);
               cost += oc;
-              mat_elems += op_mat_elems(o);
+              mat_elems += facts[i].elems;
               ngrad += o.grad ? 1 : 0;
               it = ready.erase(it);
               retire(i);
@@ -396,15 +401,15 @@ int plan_passes(const SchedParams& p, const std::vector<SchedOp>& ops, std::vect
       if (free_slots == 0 || (int)taken.size() >= kMaxPassOps) break;
       int best = -1, bestmiss = 0;
       for (int i : ready) {
-        const int miss = __builtin_popcountll(opmask(ops[i]) & ~local);
-        if (miss > 0 && miss <= free_slots && (taken.empty() || cost + op_cost(ops[i], p.grad_cost) <= p.budget)) {
+        const int miss = __builtin_popcountll(facts[i].mask & ~local);
+        if (miss > 0 && miss <= free_slots && (taken.empty() || cost + facts[i].cost <= p.budget)) {
           best = i;
           bestmiss = miss;
           break;
         }
       }
       if (best < 0) break;
-      local |= opmask(ops[best]);
+      local |= facts[best].mask;
       free_slots -= bestmiss;
     }
     if (taken.empty()) { err = "scheduler could not place an operation"; return -1; }
@@ -530,7 +535,7 @@ int plan_passes(const SchedParams& p, const std::vector<SchedOp>& ops, std::vect
     d.grad_base = 0;
     plan.nsrc = (int)taken.size();
     plan.cost = cost;
-    out.push_back(plan);
+    out.push_back(std::move(plan));
   }
   return (int)out.size();
 }
@@ -591,6 +596,7 @@ std::vector<SchedOp> fuse_two_qubit_blocks(const std::vector<SchedOp>& ops, std:
                                            bool monomial_barrier) {
   const int nb = 64;
   std::vector<Block> blocks;
+  blocks.reserve(ops.size());
   std::vector<int> open(nb, -1), last(nb, -1);
   std::vector<int> passthrough;   // ops of width >= 3 keep their place as blocks with k = 0
   auto mat2 = [&](const SchedOp& o) {
@@ -1555,6 +1561,9 @@ void stage_items(const PassPlan& pl, const StageDesc& sd, const std::vector<Sche
 // 2688 -> 1938 multiply-adds per amplitude, 325 -> 306 ms; 28-qubit gradient:
 // forward 898 -> 582, backward 1512 -> 1069, 177 -> 172 ms.
 void merge_stage_diagonals(std::vector<PassPlan>& plans, const std::vector<SchedOp>& ops) {
+  std::vector<StageItem> items;
+  std::vector<uint8_t> done;
+  std::vector<int> group;
   for (PassPlan& pl : plans) {
     PassDesc& d = pl.desc;
     if (d.R > 4) continue;
@@ -1563,8 +1572,10 @@ void merge_stage_diagonals(std::vector<PassPlan>& plans, const std::vector<Sched
     std::vector<uint32_t> nsrc, nterm;
     std::vector<std::vector<DiagFactor>> diag;
     std::vector<std::pair<uint16_t, uint16_t>> range(d.nstages);
+    nops.reserve(d.nops + d.nops / 2);
+    nsrc.reserve(d.nops);
     for (int s = 0; s < d.nstages; ++s) {
-      std::vector<StageItem> items;
+      items.clear();
       stage_items(pl, d.st[s], ops, items);
       range[s].first = (uint16_t)nops.size();
       auto emit = [&](const OpDesc& o) {
@@ -1575,7 +1586,7 @@ void merge_stage_diagonals(std::vector<PassPlan>& plans, const std::vector<Sched
         }
       };
       size_t left = items.size();
-      std::vector<uint8_t> done(items.size(), 0);
+      done.assign(items.size(), 0);
       while (left) {
         // everything that is not a diagonal and waits for nothing before it
         bool progress = true;
@@ -1596,7 +1607,7 @@ void merge_stage_diagonals(std::vector<PassPlan>& plans, const std::vector<Sched
           }
         }
         // then every diagonal with only diagonals before it on its slots
-        std::vector<int> group;
+        group.clear();
         uint32_t blocked = 0;
         for (size_t i = 0; i < items.size(); ++i) {
           if (done[i]) continue;
@@ -1650,7 +1661,7 @@ void merge_stage_diagonals(std::vector<PassPlan>& plans, const std::vector<Sched
         m.gidx = diag_units(fs, NV);
         if ((m.gidx & 0xFFFFu) == (1u << NV) - 1u) continue;   // the identity
         nops.push_back(m);
-        diag.push_back(fs);
+        diag.push_back(std::move(fs));
       }
       range[s].second = (uint16_t)nops.size();
     }
@@ -1664,8 +1675,8 @@ void merge_stage_diagonals(std::vector<PassPlan>& plans, const std::vector<Sched
       d.st[s].op1 = range[s].second;
     }
     std::copy(nterm.begin(), nterm.end(), d.grad_term);
-    pl.src = nsrc;
-    pl.diag = diag;
+    pl.src = std::move(nsrc);
+    pl.diag = std::move(diag);
   }
 }
 
