@@ -167,11 +167,14 @@ size_t iq_statevector_num_qubits(void* sv);
  * "plan_style" (0: follow "jit"; 1: plan for the interpreting kernel, fusing
  * one-qubit gates into two-qubit blocks; 2: plan for specialised kernels,
  * leaving CX/CZ/SWAP apart and normalising dense one-qubit gates), "normalize"
- * (1: normalised one-qubit gates in plans of style 2).  Plans of style 2 run
- * 4 CTAs per SM with one tile buffer unless those options (or IQ_CTAS_PER_SM,
- * IQ_NBUF) are set; get_option reports the values the handle's next plan
- * uses.  "chunk_bits" 3 with "budget" 160 plans fewer, fuller passes: a
- * faster circuit at a lower bandwidth per pass.
+ * (1: normalised one-qubit gates in plans of style 2), "jit_threads" (threads
+ * of a specialised kernel's CTA: 128 or 256, one tile per CTA at a time; 0, the
+ * default, lets tiles of 2^12 amplitudes in 4 register slots run two at a time
+ * in one CTA per SM over three buffers).  Specialised kernels of one tile per
+ * CTA run 3 CTAs per SM with one tile buffer; "ctas_per_sm" other than 3 or any
+ * "nbuf" (or IQ_NBUF) asks for that form.  get_option reports the values the
+ * handle's next plan uses.  For arrays of 2^27 amplitudes and more, plans of
+ * at most 4, 5 and 8 stages a pass are compared unless "max_stages" is set.
  * 0 = ok, -1 = unknown key or bad value. */
 int iq_handle_set_option(void* h, const char* key, double value);
 double iq_handle_get_option(void* h, const char* key);

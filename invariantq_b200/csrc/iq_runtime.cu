@@ -378,7 +378,7 @@ struct Engine : HandleRes {
   }
   TileLaunch launch_params(bool spec) const {
     TileLaunch t = tl;
-    if (spec && !set_ctas) t.ctas_per_sm = 3;
+    if (spec && !set_ctas) t.ctas_per_sm = kSpecCtas;
     if (spec && !set_nbuf) t.nbuf = 1;
     return t;
   }
@@ -566,10 +566,15 @@ struct Engine : HandleRes {
     TileLaunch tl{};                     // launch settings of the passes
   };
 
-  // The pair pipeline unless an option asks for another CTA shape.  26 qubits,
-  // three CTAs of one buffer -> pair pipeline: passes of 3 stages 0.377 -> 0.350
-  // ms, 4 stages 0.478 -> 0.412, a 30-qubit circuit of depth 20 289 -> 273 ms.
-  bool may_pair() const { return jit_threads == 0 && !set_ctas && !set_nbuf; }
+  // The pair pipeline unless an option asks for another CTA shape than the
+  // default (the autotuner sets every option, so its default candidate has to
+  // be the default).  26 qubits, three CTAs of one buffer -> pair pipeline:
+  // passes of 3 stages 0.377 -> 0.350 ms, 4 stages 0.478 -> 0.412, a 30-qubit
+  // circuit of depth 20 289 -> 273 ms.
+  static constexpr int kSpecCtas = 3;
+  bool may_pair() const {
+    return jit_threads == 0 && !set_nbuf && (!set_ctas || tl.ctas_per_sm == kSpecCtas);
+  }
 
   // Stage limits tried for arrays whose passes are long enough to pay for the
   // planning (2^kPlanTrialBits amplitudes: ~0.6 ms a pass, a plan ~1 ms): below

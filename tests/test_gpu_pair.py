@@ -59,3 +59,21 @@ def test_density_matrices(n):
         dm.close()
     assert abs(np.trace(got[0]) - 1) <= TOL
     assert np.abs(got[0] - got[1]).max() <= TOL
+
+
+def test_explicit_default_shape_is_the_default():
+    """The autotuner sets every option: the default number of CTAs, set explicitly, runs the default kernels."""
+    from invariantq_b200.binding import NativeStateVector
+    gates = list(_gates(20, 60, np.random.default_rng(5)))
+    got = []
+    for ctas in (None, 3, 4):
+        sv = NativeStateVector(20)
+        sv.set_option("jit", 2)
+        if ctas:
+            sv.set_option("ctas_per_sm", ctas)
+        for qs, m in gates:
+            sv.apply_1q(qs[0], m) if len(qs) == 1 else sv.apply_2q(qs[0], qs[1], m)
+        got.append(sv.get_amplitudes())
+        sv.close()
+    assert np.array_equal(got[0], got[1])
+    assert np.abs(got[0] - got[2]).max() <= TOL
