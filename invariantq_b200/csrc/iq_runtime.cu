@@ -336,6 +336,7 @@ struct Engine : HandleRes {
   uint64_t dim = 1;
   int num_sms = 148;
   double2* d_state = nullptr;
+  bool address_out = false;   // the caller was given d_state: other streams may work on it
 
   std::vector<SchedOp> ops;
   std::vector<cplx64> pool;          // matrices of the queued ops (dense, plus phases of monomials)
@@ -454,6 +455,9 @@ struct Engine : HandleRes {
       cudaEventDestroy(pe.second);
     }
     prof.clear();
+    // a small state whose address the caller has is freed too, not kept: cudaFree
+    // waits for what the caller's own streams still do with it
+    if (address_out && d_state == d_small) d_small = nullptr;
     if (d_state && d_state != d_small) cudaFree(d_state);
     d_state = nullptr;
     HandleRes& r = *this;
@@ -1428,6 +1432,7 @@ void* iq_statevector_device_ptr(void* sv) {
   Engine* e = as_engine(sv, 0);
   if (!e) return nullptr;
   if (!e->flush()) return nullptr;
+  e->address_out = true;
   return e->d_state;
 }
 
@@ -1846,6 +1851,7 @@ void* iq_density_matrix_device_ptr(void* dm) {
   Engine* e = as_engine(dm, 1);
   if (!e) return nullptr;
   if (!e->flush()) return nullptr;
+  e->address_out = true;
   return e->d_state;
 }
 
