@@ -24,6 +24,7 @@
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
+#include <cstdlib>
 #include <cstdint>
 #include <vector>
 
@@ -180,9 +181,6 @@ __global__ void gram_reduce_kernel(const double2* __restrict__ part, int pairs, 
 // qubits (n = 128) 3.9 -> 0.85 ms, 20 (1024) 34.5 -> 8.6, 22 (2048) 89 -> 34,
 // 24 (4096) ~400 -> ~220; a column costs ~6 us at n <= 1024: the barrier and the
 // chain load - reduce - divide around it.
-constexpr int kHhRows = 8;
-constexpr int kHhSmemMax = 1024;       // rows in shared memory up to this size
-constexpr int kHhFusedMax = 4096;      // vectors (48 B per row) fit shared memory up to this size
 constexpr uint64_t kHhWaitNs = 2000000000ull;
 
 __device__ __forceinline__ uint64_t clock_ns() {
@@ -402,29 +400,38 @@ cudaError_t launch_hh_fused(double2* A, int n, double2* rowbuf, double2* pbuf, d
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const bool smem_rows = n <= kHhSmemMax && n / kHhRows <= sms;
-  const size_t smem = (size_t)n * sizeof(double2) * (smem_rows ? 3 + kHhRows : 3);
-  const int grid = smem_rows ? n / kHhRows : std::min(sms, n / kHhRows);
+  if (const char* v = getenv("IQ_ENTROPY_SMS")) sms = std::max(1, std::min(sms, atoi(v)));
+  const HhShape h = hh_shape(n, sms);
   const void* fn = nullptr;
-  int threads = 0;
-  auto use = [&](const void* f, int nt) { fn = f; threads = nt; };
-  // shared-memory rows: 256 threads (128 at n = 128); global rows: 512, for the loads in flight
+  auto use = [&](const void* f, bool smem_rows, int threads, int rows) {
+    if (h.smem_rows == smem_rows && h.threads == threads && h.rows == rows) fn = f;
+  };
+  constexpr int RS = kHhRows, RG = kHhRows / 2;
   switch (n) {
-    case 128: use((const void*)hh_fused_kernel<true, 128, 1, kHhRows>, 128); break;
-    case 256: use((const void*)hh_fused_kernel<true, 256, 1, kHhRows>, 256); break;
-    case 512: use((const void*)hh_fused_kernel<true, 256, 2, kHhRows>, 256); break;
-    case 1024:
-      if (smem_rows) use((const void*)hh_fused_kernel<true, 256, 4, kHhRows>, 256);
-      else use((const void*)hh_fused_kernel<false, 512, 2, kHhRows / 2>, 512);
+    case 128:
+      use((const void*)hh_fused_kernel<true, 128, 1, RS>, true, 128, RS);
+      use((const void*)hh_fused_kernel<false, 128, 1, RG>, false, 128, RG);
       break;
-    case 2048: use((const void*)hh_fused_kernel<false, 512, 4, kHhRows / 2>, 512); break;
-    case 4096: use((const void*)hh_fused_kernel<false, 512, 8, kHhRows / 2>, 512); break;
-    default: return cudaErrorInvalidValue;
+    case 256:
+      use((const void*)hh_fused_kernel<true, 256, 1, RS>, true, 256, RS);
+      use((const void*)hh_fused_kernel<false, 256, 1, RG>, false, 256, RG);
+      break;
+    case 512:
+      use((const void*)hh_fused_kernel<true, 256, 2, RS>, true, 256, RS);
+      use((const void*)hh_fused_kernel<false, 512, 1, RG>, false, 512, RG);
+      break;
+    case 1024:
+      use((const void*)hh_fused_kernel<true, 256, 4, RS>, true, 256, RS);
+      use((const void*)hh_fused_kernel<false, 512, 2, RG>, false, 512, RG);
+      break;
+    case 2048: use((const void*)hh_fused_kernel<false, 512, 4, RG>, false, 512, RG); break;
+    case 4096: use((const void*)hh_fused_kernel<false, 512, 8, RG>, false, 512, RG); break;
   }
-  cudaError_t err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (!fn) return cudaErrorInvalidValue;
+  cudaError_t err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h.smem);
   if (err != cudaSuccess) return err;
   void* args[] = {&A, &n, &rowbuf, &pbuf, &d, &e, &arrived, &status};
-  return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(threads), args, smem, st);
+  return cudaLaunchCooperativeKernel(fn, dim3(h.grid), dim3(h.threads), args, h.smem, st);
 }
 
 // ---- the same column by column, for n above kHhFusedMax (sweeps of 1 GiB dwarf their launches)

@@ -156,6 +156,31 @@ cudaError_t launch_init_joint(double2* s, int n, uint64_t jdim, int nsets, cudaS
 cudaError_t launch_init_joint_c64(float2* s, int n, uint64_t jdim, int nsets, cudaStream_t st);
 cudaError_t launch_row_sums(const double* in, int rows, int cols, double* out, cudaStream_t st);
 
+// Launch shape of the fused Householder reduction (iq_entropy.cu) of an n x n
+// matrix, n a power of two in 128..kHhFusedMax, on a device of `sms` SMs.  Every
+// CTA is resident for the whole launch.  Rows in shared memory need a CTA for
+// every kHhRows of them; with fewer SMs than that (a MIG slice) and above
+// kHhSmemMax the rows stay in global memory, dealt to as many CTAs as there are.
+// Shared-memory rows: 256 threads (128 at n = 128); global rows: 512 (at most
+// n), for the loads in flight.
+constexpr int kHhRows = 8;
+constexpr int kHhSmemMax = 1024;
+constexpr int kHhFusedMax = 4096;      // vectors (48 B per row) fit shared memory up to this size
+struct HhShape {
+  bool smem_rows;
+  int threads, rows, grid;             // rows: those a CTA takes at a time
+  size_t smem;
+};
+inline HhShape hh_shape(int n, int sms) {
+  HhShape h;
+  h.smem_rows = n <= kHhSmemMax && n / kHhRows <= sms;
+  h.threads = h.smem_rows ? (n < 256 ? n : 256) : (n < 512 ? n : 512);
+  h.rows = h.smem_rows ? kHhRows : kHhRows / 2;
+  h.grid = (h.smem_rows || n / kHhRows <= sms) ? n / kHhRows : sms;
+  h.smem = (size_t)n * sizeof(double2) * (h.smem_rows ? 3 + kHhRows : 3);
+  return h;
+}
+
 // Eigenvalues (ascending) of the reduced state on the kept qubits keep[0..k) of
 // the 2^nbits state psi, computed on the device (iq_entropy.cu); 7 <= k <=
 // reduced_spectrum_max_bits(), k < nbits.  work: reduced_spectrum_bytes(nbits, k)
