@@ -248,7 +248,8 @@ struct HandleRes {
     if (stream) cudaStreamDestroy(stream);
     *this = HandleRes{};
   }
-  // at least `bytes` of scratch space (contents undefined); the stream's earlier users of it are done or ordered before
+  // at least `bytes` <= kKeepWork of scratch space (contents undefined); the stream's earlier users of it are done or
+  // ordered before.  Calls take it through Work.
   char* work(size_t bytes) {
     if (bytes > work_cap) {
       if (d_work) cudaStreamSynchronize(stream);
@@ -278,6 +279,32 @@ struct HandleRes {
     stage_cap = bytes;
     return true;
   }
+};
+
+// Scratch space of one call (p null: not to be had, the error is set): up to
+// kKeepWork from the buffer the handle keeps, more than that for this call only
+// -- 2^30 counted shots take tens of GiB.  The call's own work on the stream is
+// done when it ends.
+struct Work {
+  char* p = nullptr;
+  Work(HandleRes& r, size_t bytes) : stream(r.stream), own(bytes > kKeepWork) {
+    if (!own) p = r.work(bytes);
+    else if (!cuda_ok(cudaMallocAsync(&p, bytes, stream), "cudaMallocAsync work space")) {
+      cudaGetLastError();
+      p = nullptr;
+    }
+  }
+  ~Work() {
+    if (!own || !p) return;
+    cudaFreeAsync(p, stream);
+    cudaStreamSynchronize(stream);
+  }
+  Work(const Work&) = delete;
+  Work& operator=(const Work&) = delete;
+
+ private:
+  cudaStream_t stream;
+  bool own;
 };
 
 // id of the current CUDA context: sets of a context that was reset are not reused
@@ -312,7 +339,6 @@ bool res_take(int dev, unsigned long long ctx, HandleRes& out) {
 
 // the stream is idle and its work succeeded
 void res_give(HandleRes& r) {
-  if (r.work_cap > kKeepWork) r.free_work();
   if (std::max(r.d_pool_cap, r.h_pool_cap) * sizeof(double2) > kKeepPool) r.free_pool();
   r.pool_ev_recorded = false;
   {
@@ -1106,7 +1132,8 @@ void iq_statevector_sample(void* sv, size_t num_shots, uint64_t seed, uint64_t* 
   // everything on the device (iq_sampling.cu): block sums, their prefix, the
   // mt19937_64 stream (statevector.cpp:244-245), per-shot search
   const size_t wbytes = sample_work_bytes(e->nbits, num_shots);
-  char* dbuf = e->work(wbytes + num_shots * 8 + 256);
+  Work work(*e, wbytes + num_shots * 8 + 256);
+  char* const dbuf = work.p;
   if (!dbuf) return;
   uint64_t* d_out = reinterpret_cast<uint64_t*>(dbuf + ((wbytes + 255) & ~(size_t)255));
   ++e->st_launches;
@@ -1128,7 +1155,8 @@ int iq_statevector_sample_counts(void* sv, size_t num_shots, uint64_t seed, uint
   }
   const size_t wbytes = (std::max(sample_work_bytes(e->nbits, num_shots), count_work_bytes(num_shots)) + 255) & ~(size_t)255;
   const size_t obytes = (num_shots * 8 + 255) & ~(size_t)255;
-  char* dbuf = e->work(wbytes + 3 * obytes + 256);
+  Work work(*e, wbytes + 3 * obytes + 256);
+  char* const dbuf = work.p;
   if (!dbuf) return -1;
   uint64_t* d_shots = reinterpret_cast<uint64_t*>(dbuf + wbytes);
   uint64_t* d_vals = reinterpret_cast<uint64_t*>(dbuf + wbytes + obytes);
@@ -1201,24 +1229,15 @@ double iq_statevector_entropy(void* sv, const size_t* qubits, size_t num_subsys_
   if (kk >= 7) {
     // reduced state, tridiagonalisation and eigenvalues on the device (iq_entropy.cu)
     std::vector<double> w;
-    const size_t bytes = reduced_spectrum_bytes(n, kk);
-    void* buf = nullptr;
-    const bool kept = bytes <= kKeepWork;   // larger than that (from 11 qubits): for this call only
-    if (kept) {
-      buf = e->work(bytes);
-      if (!buf) return kNaN;
-    } else if (!cuda_ok(cudaMallocAsync(&buf, bytes, e->stream), "cudaMallocAsync entropy")) {
-      return kNaN;
-    }
-    const bool ok = cuda_ok(reduced_spectrum(e->d_state, n, keep.data(), kk, w, buf, e->stream), "reduced spectrum");
-    if (!kept) {
-      cudaFreeAsync(buf, e->stream);
-      cudaStreamSynchronize(e->stream);
-    }
+    // above kKeepWork from 11 kept qubits, for 10 from 21 qubits and for 9 from 22 (partial tiles of the split environment)
+    Work work(*e, reduced_spectrum_bytes(n, kk));
+    if (!work.p) return kNaN;
+    const bool ok = cuda_ok(reduced_spectrum(e->d_state, n, keep.data(), kk, w, work.p, e->stream), "reduced spectrum");
     return ok ? entropy_from(w) : kNaN;
   }
   const size_t kd = (size_t)1 << kk;
-  double2* d_rho = reinterpret_cast<double2*>(e->work(kd * kd * sizeof(double2)));
+  Work work(*e, kd * kd * sizeof(double2));
+  double2* const d_rho = reinterpret_cast<double2*>(work.p);
   if (!d_rho) return kNaN;
   std::vector<cd> rho(kd * kd);
   ++g_launches;

@@ -46,3 +46,24 @@ def test_reader_on_another_stream(kind, n):
     assert torch.equal(out.cpu(), want)
     for k in later:
         k.close()
+
+
+# scratch of a call: what a live handle keeps is bounded, whatever the call took (2^20 shots fit the bound, 2^21 and 2^24 do not)
+@pytest.mark.parametrize("shots", [1 << 20, 1 << 21, 1 << 24])
+def test_kept_scratch_is_bounded(shots):
+    from invariantq_b200.binding import NativeStateVector
+    sv = NativeStateVector(12)
+    for q in range(12):
+        sv.apply_1q(q, np.array([[1, 1], [1, -1]]) / np.sqrt(2))
+    sv.sample_counts(100, 1)
+    sv.sample(100, 1)
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    values, counts = sv.sample_counts(shots, 5)
+    outcomes = sv.sample(shots, 5)
+    torch.cuda.synchronize()
+    kept = before - torch.cuda.mem_get_info()[0]
+    v, c = np.unique(outcomes, return_counts=True)
+    assert np.array_equal(values, v) and np.array_equal(counts, c)
+    assert kept <= (64 << 20) + (4 << 20)   # the bound, and the allocator's granularity
+    sv.close()
