@@ -301,7 +301,9 @@ int iq_adjoint_gradient_batch(const iq_adjoint_circuit* circuits, size_t num_cir
 /* Free the device and pinned host memory the adjoint calls keep between calls
  * (and what freed state-vector and density-matrix handles left for the next
  * ones: at most four sets of streams and buffers, ~80 MiB of device memory
- * each); returns the number of adjoint workspaces freed. */
+ * each); returns the number of adjoint workspaces freed.  The library does so
+ * itself before an allocation of its own fails; call it when other code needs
+ * the memory. */
 int iq_adjoint_release(void);
 /* Energies only (grad_out unused): the forward circuit and <psi|H|psi> for each
  * parameter set of one circuit, one set after another on one stream -- the

@@ -364,7 +364,7 @@ struct DevBuf {
     n = std::max(n, 2 * cap);
     p = nullptr;
     cap = 0;
-    if (cudaMalloc(&p, std::max<size_t>(n, 1) * sizeof(T)) != cudaSuccess) {
+    if (device_alloc(&p, std::max<size_t>(n, 1) * sizeof(T)) != cudaSuccess) {
       cudaGetLastError();
       err = std::string("cannot allocate device memory for ") + what;
       return false;
@@ -902,6 +902,27 @@ void pool_give(Workspace* w, bool ok) {
   delete w;
 }
 
+}  // namespace
+
+int iqb::release_workspaces() {
+  std::vector<Workspace*> ws;
+  {
+    std::lock_guard<std::mutex> g(g_pool_mu);
+    ws.swap(*g_pool);
+  }
+  int dev = 0;
+  const bool back = !ws.empty() && cudaGetDevice(&dev) == cudaSuccess;
+  for (Workspace* w : ws) {
+    cudaSetDevice(w->device);
+    w->release();
+    delete w;
+  }
+  if (back) cudaSetDevice(dev);
+  return (int)ws.size();
+}
+
+namespace {
+
 // Run all jobs of `circs` (every parameter set of every circuit) on `nstreams` workers.
 int run_batch(std::vector<std::unique_ptr<Circuit>>& circs, int nstreams, bool want_grad, bool c64 = false) {
   const auto t0 = std::chrono::steady_clock::now();
@@ -1246,16 +1267,16 @@ int adjoint_c64(const iq_adjoint_circuit& in) {
     return ok;
   };
   check(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "stream");
-  if (ok && (cudaMalloc(&psi, dim * sizeof(float2)) != cudaSuccess ||
-             cudaMalloc(&lam, dim * sizeof(float2)) != cudaSuccess)) {
+  if (ok && (device_alloc(&psi, dim * sizeof(float2)) != cudaSuccess ||
+             device_alloc(&lam, dim * sizeof(float2)) != cudaSuccess)) {
     cudaGetLastError();
     ok = false;
     err = "cannot allocate device memory for the complex64 states";
   }
-  check(cudaMalloc(&partials, ((size_t)T + 1) * kC64Blocks * sizeof(double)), "cudaMalloc partials");
-  check(cudaMalloc(&sums, ((size_t)T + 1) * sizeof(double)), "cudaMalloc sums");
-  check(cudaMalloc(&zm, c.ham.zmask.size() * 8), "cudaMalloc Hamiltonian");
-  check(cudaMalloc(&co, c.ham.coef.size() * 16), "cudaMalloc Hamiltonian");
+  check(device_alloc(&partials, ((size_t)T + 1) * kC64Blocks * sizeof(double)), "cudaMalloc partials");
+  check(device_alloc(&sums, ((size_t)T + 1) * sizeof(double)), "cudaMalloc sums");
+  check(device_alloc(&zm, c.ham.zmask.size() * 8), "cudaMalloc Hamiltonian");
+  check(device_alloc(&co, c.ham.coef.size() * 16), "cudaMalloc Hamiltonian");
   check(cudaMemcpyAsync(zm, c.ham.zmask.data(), c.ham.zmask.size() * 8, cudaMemcpyHostToDevice, st), "H2D");
   check(cudaMemcpyAsync(co, c.ham.coef.data(), c.ham.coef.size() * 16, cudaMemcpyHostToDevice, st), "H2D");
   check(c64_set_basis(psi, c.n, st), "reset");
@@ -1366,17 +1387,7 @@ int iq_adjoint_release(void) {
     std::lock_guard<std::mutex> g(g_shape_mu);
     g_shapes->clear();
   }
-  std::vector<Workspace*> ws;
-  {
-    std::lock_guard<std::mutex> g(g_pool_mu);
-    ws.swap(*g_pool);
-  }
-  for (Workspace* w : ws) {
-    cudaSetDevice(w->device);
-    w->release();
-    delete w;
-  }
-  return (int)ws.size();
+  return release_workspaces();
 }
 
 int iq_adjoint_stats(double* out, size_t n) {

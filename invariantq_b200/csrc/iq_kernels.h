@@ -207,6 +207,18 @@ cudaError_t count_outcomes(const uint64_t* d_shots, uint64_t shots, void* work, 
 
 // Free the streams and buffers that freed handles left for the next ones (iq_runtime.cu).
 void release_handle_resources();
+// Free the adjoint workspaces that no call uses (iq_adjoint.cu); returns their number.
+int release_workspaces();
+// Device memory.  If there is no room, what earlier calls left for later ones is
+// given back first: an allocation fails only where it would without that reuse.
+cudaError_t device_alloc_bytes(void** p, size_t bytes);
+cudaError_t device_alloc_bytes_async(void** p, size_t bytes, cudaStream_t st);
+template <class T>
+cudaError_t device_alloc(T** p, size_t bytes) { return device_alloc_bytes(reinterpret_cast<void**>(p), bytes); }
+template <class T>
+cudaError_t device_alloc_async(T** p, size_t bytes, cudaStream_t st) {
+  return device_alloc_bytes_async(reinterpret_cast<void**>(p), bytes, st);
+}
 // Record an error for iq_last_error (defined in iq_runtime.cu).
 void record_error(int code, const char* msg);
 // Add to the iq_kernel_launches counter (defined in iq_runtime.cu).

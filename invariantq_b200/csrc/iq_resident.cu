@@ -435,7 +435,7 @@ bool cuda_ok(cudaError_t e, const char* what, std::string& err) {
 template <class T>
 bool upload(Plan& p, const std::vector<T>& v, T** out, std::string& err) {
   void* d = nullptr;
-  if (!cuda_ok(cudaMalloc(&d, std::max<size_t>(v.size(), 1) * sizeof(T)), "cudaMalloc", err)) return false;
+  if (!cuda_ok(device_alloc(&d, std::max<size_t>(v.size(), 1) * sizeof(T)), "cudaMalloc", err)) return false;
   p.dbufs.push_back(d);
   if (!v.empty() && !cuda_ok(cudaMemcpy(d, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice), "H2D", err))
     return false;

@@ -211,8 +211,8 @@ struct HandleRes {
     // the largest partials of any handle (34 index bits), so that a set serves every size
     scratch_bytes = std::max<size_t>({zsums_partials_doubles(34) * 8, (size_t)kRedBlocks * 16, kHamPartials * 16}) + 4096;
     return cuda_ok(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "cudaStreamCreate") &&
-           cuda_ok(cudaMalloc(&d_scratch, scratch_bytes), "cudaMalloc scratch") &&
-           cuda_ok(cudaMalloc(&d_status, sizeof(int)), "cudaMalloc status") &&
+           cuda_ok(device_alloc(&d_scratch, scratch_bytes), "cudaMalloc scratch") &&
+           cuda_ok(device_alloc(&d_status, sizeof(int)), "cudaMalloc status") &&
            cuda_ok(cudaMallocHost(&h_small, 64 * 1024), "cudaMallocHost") &&
            cuda_ok(cudaEventCreateWithFlags(&pool_ev, cudaEventDisableTiming), "cudaEventCreate") &&
            cuda_ok(cudaEventCreateWithFlags(&stage_ev[0], cudaEventDisableTiming), "cudaEventCreate") &&
@@ -255,7 +255,7 @@ struct HandleRes {
       if (d_work) cudaStreamSynchronize(stream);
       free_work();
       if (!cuda_ok(cudaSetDevice(device), "cudaSetDevice") ||
-          !cuda_ok(cudaMalloc(&d_work, bytes), "cudaMalloc work space")) {
+          !cuda_ok(device_alloc(&d_work, bytes), "cudaMalloc work space")) {
         cudaGetLastError();
         d_work = nullptr;
         return nullptr;
@@ -270,7 +270,7 @@ struct HandleRes {
     if (d_stage) cudaStreamSynchronize(stream);
     free_stage();
     if (!cuda_ok(cudaSetDevice(device), "cudaSetDevice") ||
-        !cuda_ok(cudaMalloc(&d_stage, 2 * bytes), "cudaMalloc staging") ||
+        !cuda_ok(device_alloc(&d_stage, 2 * bytes), "cudaMalloc staging") ||
         !cuda_ok(cudaMallocHost(&h_stage, 2 * bytes), "cudaMallocHost staging")) {
       cudaGetLastError();
       free_stage();
@@ -289,7 +289,7 @@ struct Work {
   char* p = nullptr;
   Work(HandleRes& r, size_t bytes) : stream(r.stream), own(bytes > kKeepWork) {
     if (!own) p = r.work(bytes);
-    else if (!cuda_ok(cudaMallocAsync(&p, bytes, stream), "cudaMallocAsync work space")) {
+    else if (!cuda_ok(device_alloc_async(&p, bytes, stream), "cudaMallocAsync work space")) {
       cudaGetLastError();
       p = nullptr;
     }
@@ -446,9 +446,9 @@ struct Engine : HandleRes {
     }
     const size_t bytes = dim * sizeof(double2);
     if (bytes <= kSmallState) {
-      if (!d_small && !cuda_ok(cudaMalloc(&d_small, kSmallState), "cudaMalloc small state")) return false;
+      if (!d_small && !cuda_ok(device_alloc(&d_small, kSmallState), "cudaMalloc small state")) return false;
       d_state = d_small;
-    } else if (cudaMalloc(&d_state, bytes) != cudaSuccess) {
+    } else if (device_alloc(&d_state, bytes) != cudaSuccess) {
       cudaGetLastError();
       set_error(E_MEM, "cannot allocate %.3f GiB of device memory for %d qubits", dim * 16.0 / (1 << 30), nq);
       d_state = nullptr;
@@ -551,7 +551,7 @@ struct Engine : HandleRes {
         cudaFree(d_pool);
       }
       d_pool_cap = std::max<size_t>(n, 1 << 16);
-      if (!cuda_ok(cudaMalloc(&d_pool, d_pool_cap * sizeof(double2)), "cudaMalloc matrix pool")) {
+      if (!cuda_ok(device_alloc(&d_pool, d_pool_cap * sizeof(double2)), "cudaMalloc matrix pool")) {
         d_pool = nullptr;
         d_pool_cap = 0;
         return false;
@@ -712,7 +712,7 @@ struct Engine : HandleRes {
     pg.pool_elems = nsrc;
     if (own) {
       if (nsrc) {
-        if (!cuda_ok(cudaMalloc(&pg.d_mats, nsrc * sizeof(double2)), "cudaMalloc program matrices")) return false;
+        if (!cuda_ok(device_alloc(&pg.d_mats, nsrc * sizeof(double2)), "cudaMalloc program matrices")) return false;
         pg.owns = true;
         if (!cuda_ok(cudaMemcpy(pg.d_mats, src, nsrc * sizeof(double2), cudaMemcpyHostToDevice),
                      "H2D program matrices"))
@@ -953,6 +953,24 @@ void iqb::release_handle_resources() {
   }
   if (back) cudaSetDevice(dev);
 }
+
+namespace {
+template <class F>
+cudaError_t alloc_or_give_back(F alloc) {
+  const cudaError_t e = alloc();
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  release_handle_resources();
+  release_workspaces();
+  return alloc();
+}
+}  // namespace
+cudaError_t iqb::device_alloc_bytes(void** p, size_t bytes) {
+  return alloc_or_give_back([&] { return cudaMalloc(p, bytes); });
+}
+cudaError_t iqb::device_alloc_bytes_async(void** p, size_t bytes, cudaStream_t st) {
+  return alloc_or_give_back([&] { return cudaMallocAsync(p, bytes, st); });
+}
 void iqb::record_error(int code, const char* msg) { set_error(code, "%s", msg); }
 void iqb::count_launches(uint64_t n) { g_launches += n; }
 
@@ -1182,7 +1200,7 @@ int iq_mt64_uniform(uint64_t seed, size_t count, double* out) {
   double* d = nullptr;
   cudaStream_t st = nullptr;
   if (!cuda_ok(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "stream")) return -1;
-  bool ok = cuda_ok(cudaMallocAsync(reinterpret_cast<void**>(&d), count * 8, st), "cudaMallocAsync") &&
+  bool ok = cuda_ok(device_alloc_async(&d, count * 8, st), "cudaMallocAsync") &&
             cuda_ok(launch_mt64_uniform(seed, count, d, st), "mt19937_64") &&
             cuda_ok(cudaMemcpyAsync(out, d, count * 8, cudaMemcpyDeviceToHost, st), "D2H") &&
             cuda_ok(cudaStreamSynchronize(st), "sync");
