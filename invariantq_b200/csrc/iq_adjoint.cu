@@ -426,10 +426,7 @@ struct Workspace {
   // The state arrays are sized up front for the batch's largest job; matrix,
   // partial and staging buffers grow on demand (doubling, so a worker
   // reallocates a few times at the start: the largest jobs run first).
-  struct Bounds {
-    uint64_t psi_amps = 1, joint_amps = 1;
-    size_t mats = 1, sets = 1, grads = 1;   // per job: matrix elements, sets, gradient terms x sets
-  };
+  using Bounds = AdjointBounds;
 
   // Make ready for a call on device `dev` (a workspace can come back from the
   // pool of an earlier call: pointers into that call's shapes and circuits are
@@ -1008,8 +1005,7 @@ int run_batch(std::vector<std::unique_ptr<Circuit>>& circs, int nstreams, bool w
   size_t freeb = 0, totalb = 0;
   cudaMemGetInfo(&freeb, &totalb);
   const int max_grid = sms * std::max(1, cfg.tl.ctas_per_sm);
-  const double per = 16.0 * ((double)bd.psi_amps + (double)bd.joint_amps) + 16.0 * (double)bd.mats +
-                     8.0 * (double)bd.grads * (max_grid + 2) / 3.0 + (64 << 20);
+  const double per = bd.worker_bytes(max_grid);
   int nw = nstreams > 0 ? nstreams : env_int("IQ_ADJOINT_STREAMS", 8);
   nw = std::min<int>(nw, (int)jobs.size());
   nw = std::min<int>(nw, std::max(1, (int)(0.8 * (double)freeb / per)));

@@ -205,6 +205,22 @@ size_t count_work_bytes(uint64_t shots);
 cudaError_t count_outcomes(const uint64_t* d_shots, uint64_t shots, void* work, uint64_t* d_vals, uint64_t* d_cnts,
                            uint64_t* d_nuniq, cudaStream_t st);
 
+// What one worker of a gradient or energy call works with (iq_adjoint.cu): the
+// largest of its jobs, in amplitudes of 16 B, matrix elements, parameter sets
+// and gradient terms x sets.
+struct AdjointBounds {
+  uint64_t psi_amps = 1, joint_amps = 1;
+  size_t mats = 1, sets = 1, grads = 1;
+  // device memory of a worker, for the number of workers that fit: arrays,
+  // matrices (a bound several times what circuits need), Hamiltonian partial
+  // sums, gradient partials of a grid of max_grid CTAs (a third of the bound on
+  // the terms), and the rest
+  double worker_bytes(int max_grid) const {
+    return 16.0 * ((double)psi_amps + (double)joint_amps) + 16.0 * (double)mats +
+           8.0 * (double)sets * (double)(kHamPartials + 1) + 8.0 * (double)grads * (max_grid + 2) / 3.0 + (64 << 20);
+  }
+};
+
 // Free the streams and buffers that freed handles left for the next ones (iq_runtime.cu).
 void release_handle_resources();
 // Free the adjoint workspaces that no call uses (iq_adjoint.cu); returns their number.

@@ -30,3 +30,13 @@ def test_tridiagonalisation_shape(lib, n, sms):
     if smem_rows:
         assert grid * rows >= n   # rows in shared memory: each has a CTA of its own group
     assert smem_rows == (n <= 1024 and 8 * sms >= n)
+
+
+# many parameter sets of a small circuit: their Hamiltonian partials alone are more than the estimate's fixed slack
+@pytest.mark.parametrize("sets", [1, 64, 5000, 16384, 32768])
+def test_worker_estimate_covers_the_partials(lib, sets):
+    lib.worker_bytes.restype = lib.ham_partial_bytes.restype = ctypes.c_double
+    lib.worker_bytes.argtypes = [ctypes.c_longlong] * 4 + [ctypes.c_int]
+    joint, mats = sets << 14, 4 * sets
+    need = 16 * joint + 16 * mats + sets * lib.ham_partial_bytes()
+    assert lib.worker_bytes(joint, mats, sets, sets, 444) >= need
