@@ -457,6 +457,9 @@ void normalize_one_qubit_ops(std::vector<SchedOp>& ops, std::vector<cplx64>& poo
 // through the later gates as it does diagonals, and writes each qubit's last
 // rotation as a plain real 2x2 that absorbs the pending X (2 multiply-adds per
 // amplitude more, once per qubit).
+// A phase is dropped only if it is exactly 1; phases that cancel are formed so
+// that they come out exactly 1, and one that only rounding keeps from 1 (a
+// fused product of complex gates, nothing pending) is emitted for every angle.
 enum DecompMode { DECOMP_BY_ANGLE = 0, DECOMP_STEADY_SCALARS = 1, DECOMP_STEADY = 2 };
 void decompose_one_qubit_ops(std::vector<SchedOp>& ops, std::vector<cplx64>& pool, DecompMode mode = DECOMP_BY_ANGLE);
 // Re-pack the matrix data each pass references (absolute offsets into `pool`)

@@ -806,10 +806,16 @@ inline cplx64 cdiv(cplx64 a, cplx64 b) {
 inline double cabs2(cplx64 a) { return a.re * a.re + a.im * a.im; }
 inline bool is_one(cplx64 a) { return a.re == 1.0 && a.im == 0.0; }
 
+// A phase is dropped only where it is exactly 1.  So that an operation does not
+// come and go with the rounding of the angles, phases that cancel come out
+// exactly 1: a pending diagonal is kept as diag(1, b), the phases of a gate's
+// entries are taken relative to its own first entry, and what does not enter a
+// phase is not multiplied into it; where rounding decides (a product of complex
+// gates), the phase is emitted even if it is 1 (dense1).
 struct Decomposer {
   std::vector<SchedOp>& out;
   std::vector<cplx64>& pool;
-  std::vector<cplx64> pa, pb;   // pending output diagonal diag(pa[q], pb[q]) of each qubit
+  std::vector<cplx64> pa, pb;   // pending output diagonal diag(pa[q], pb[q]) of each qubit (set_pending)
   std::vector<uint8_t> px;      // DECOMP_STEADY: a pending X of the qubit, before that diagonal
   cplx64 G{1.0, 0.0};           // scalar factored out of the emitted operations
   DecompMode mode;
@@ -820,11 +826,16 @@ struct Decomposer {
   Decomposer(std::vector<SchedOp>& o, std::vector<cplx64>& p, DecompMode m)
       : out(o), pool(p), pa(64, {1.0, 0.0}), pb(64, {1.0, 0.0}), px(64, 0), mode(m) {}
 
-  // exactly 1 -- in the steady modes also 1 up to rounding, so that a phase that
-  // cancels does not come and go with the angles
-  bool unit_phase(cplx64 a) const {
-    if (is_one(a)) return true;
-    return mode != DECOMP_BY_ANGLE && std::fabs(a.re - 1.0) <= 2e-15 && std::fabs(a.im) <= 2e-15;
+  // the pending diagonal of q becomes diag(a, b): diag(1, b / a), a in G, when
+  // a has modulus 1 (other diagonals keep their scale to themselves)
+  void set_pending(int q, cplx64 a, cplx64 b) {
+    if (std::fabs(cabs2(a) - 1.0) < 1e-12 && !is_one(a)) {
+      G = cm(G, a);
+      b = (b.re == a.re && b.im == a.im) ? cplx64{1.0, 0.0} : cdiv(b, a);
+      a = {1.0, 0.0};
+    }
+    pa[q] = a;
+    pb[q] = b;
   }
   uint32_t put(std::initializer_list<cplx64> v) {
     const uint32_t at = (uint32_t)pool.size();
@@ -832,10 +843,10 @@ struct Decomposer {
     return at;
   }
   // one-qubit diagonal diag(a, b) = a diag(1, b / a): the scalar goes to G
-  void emit_phase(int q, cplx64 a, cplx64 b) {
+  void emit_phase(int q, cplx64 a, cplx64 b, bool always = false) {
     const cplx64 r = cdiv(b, a);
     G = cm(G, a);
-    if (unit_phase(r)) return;
+    if (is_one(r) && !always) return;
     SchedOp o{};
     o.k = 1;
     o.q[0] = (uint8_t)q;
@@ -881,19 +892,19 @@ struct Decomposer {
     o.dense = put({{0.0, 0.0}, {1.0, 0.0}, {1.0, 0.0}, {0.0, 0.0}});
     out.push_back(o);
   }
-  // real rotation [[c, -s], [s, c]] (c > 0, c^2 + s^2 = 1), normalised by max(c, |s|)
-  void emit_rotation(int q, double c, double s) {
+  // [[c, -s], [s, c]] (c > 0) times the scalar g, normalised by max(c, |s|)
+  void emit_rotation(int q, double c, double s, cplx64 g) {
     SchedOp o{};
     o.k = 1;
     o.q[0] = (uint8_t)q;
     if (c >= std::fabs(s)) {
       const double t = s / c;
-      G = cm(G, {c, 0.0});
+      G = cm(G, {g.re * c, g.im * c});
       o.rot = 1;
       o.dense = put({{1.0, 0.0}, {-t, 0.0}, {t, 0.0}, {1.0, 0.0}});
     } else {
       const double u = c / s;
-      G = cm(G, {s, 0.0});
+      G = cm(G, {g.re * s, g.im * s});
       o.rot = 2;
       o.dense = put({{u, 0.0}, {-1.0, 0.0}, {1.0, 0.0}, {u, 0.0}});
     }
@@ -907,41 +918,45 @@ struct Decomposer {
       rotations = 0;
     }
   }
-  void emit_real(int q, double c, double s) {   // [[c, -s], [s, c]] as it is
+  void emit_real(int q, double c, double s, cplx64 g) {   // [[c, -s], [s, c]] as it is, times g
     SchedOp o{};
     o.k = 1;
     o.q[0] = (uint8_t)q;
     o.realm = 1;
     o.dense = o.mat = put({{c, 0.0}, {-s, 0.0}, {s, 0.0}, {c, 0.0}});
     out.push_back(o);
+    G = cm(G, g);
   }
   // dense one-qubit U (row-major) on q, after the pending diagonal of q
   // (`last`: no dense one-qubit operation on q follows)
   void dense1(const SchedOp& src, bool last) {
     const int q = src.q[0];
     const bool steady = mode == DECOMP_STEADY;
-    const cplx64* U0 = pool.data() + src.dense;
-    cplx64 A = cm(U0[0], pa[q]), B = cm(U0[1], pb[q]), C = cm(U0[2], pa[q]), D = cm(U0[3], pb[q]);
-    if (px[q]) {   // the pending X swaps the columns
+    const cplx64* U = pool.data() + src.dense;
+    cplx64 A = U[0], B = U[1], C = U[2], D = U[3];
+    if (px[q]) {   // the pending X swaps the columns, and the diagonal's entries with them
       std::swap(A, B);
       std::swap(C, D);
+      set_pending(q, pb[q], pa[q]);
       px[q] = 0;
     }
+    A = cm(A, pa[q]);
+    B = cm(B, pb[q]);
+    C = cm(C, pa[q]);
+    D = cm(D, pb[q]);
     const double n0 = cabs2(A) + cabs2(C), n1 = cabs2(B) + cabs2(D);
     const cplx64 ip{A.re * B.re + A.im * B.im + C.re * D.re + C.im * D.im,
                     A.re * B.im - A.im * B.re + C.re * D.im - C.im * D.re};   // conj(A) B + conj(C) D
     const bool unitary = std::fabs(n0 - 1.0) < 1e-12 && std::fabs(n1 - 1.0) < 1e-12 && cabs2(ip) < 1e-24;
     const double c0 = std::sqrt(cabs2(A)), s0 = std::sqrt(cabs2(C));
     if (unitary && s0 == 0.0 && cabs2(B) == 0.0) {     // diagonal: joins the pending diagonal
-      pa[q] = A;
-      pb[q] = D;
+      set_pending(q, A, D);
       return;
     }
     if (unitary && c0 == 0.0 && cabs2(D) == 0.0) {     // anti-diagonal: X, then diag(B, C)
       if (steady) px[q] = 1;
       else emit_x(q);
-      pa[q] = B;
-      pb[q] = C;
+      set_pending(q, B, C);
       return;
     }
     if (unitary && c0 > 0.0 && s0 > 0.0) {
@@ -951,25 +966,26 @@ struct Decomposer {
         std::swap(A, C);
         std::swap(B, D);
       }
-      const double r = std::hypot(c0, s0);
-      const double c = (swap ? s0 : c0) / r;
-      double s = (swap ? c0 : s0) / r;
-      const cplx64 d0 = cdiv(A, {c, 0.0});
-      cplx64 d1 = cdiv(C, {s, 0.0});
-      cplx64 e1 = cdiv({-B.re, -B.im}, cm(d0, {s, 0.0}));
-      if (mode != DECOMP_BY_ANGLE && e1.re < 0.0) {   // the sign goes to s: a real gate has no phase, whatever its angle
+      // u diag(1, d) [[c, -s], [s, c]] diag(1, e), u the phase of A: a real gate gives d and e of exactly +-1
+      const double c = swap ? s0 : c0;
+      double s = swap ? c0 : s0;
+      const cplx64 u{A.re / c, A.im / c}, uc{u.re, -u.im};
+      const cplx64 du = cm(C, uc), eu = cm(B, uc);
+      cplx64 d{du.re / s, du.im / s}, e{-eu.re / s, -eu.im / s};
+      if (mode != DECOMP_BY_ANGLE && e.re < 0.0) {   // the sign goes to s: a real gate has no phase, whatever its angle
         s = -s;
-        d1 = {-d1.re, -d1.im};
-        e1 = {-e1.re, -e1.im};
+        d = {-d.re, -d.im};
+        e = {-e.re, -e.im};
       }
-      const cplx64 Dr = cm(cm(d1, {c, 0.0}), e1);           // the rebuilt entry D
+      const cplx64 Dr = cm(cm(u, cm(d, e)), {c, 0.0});      // the rebuilt entry D
       if (cabs2({Dr.re - D.re, Dr.im - D.im}) < 1e-28) {
-        emit_phase(q, {1.0, 0.0}, e1);
-        if (steady && last) emit_real(q, c, s);
-        else emit_rotation(q, c, s);
-        pa[q] = swap ? d1 : d0;
-        pb[q] = swap ? d0 : d1;
+        // A and B both real or both imaginary: e is 1 or not for every angle
+        const bool exact = (A.im == 0.0 && B.im == 0.0) || (A.re == 0.0 && B.re == 0.0);
+        emit_phase(q, {1.0, 0.0}, e, mode != DECOMP_BY_ANGLE && !exact);
+        if (steady && last) emit_real(q, c, s, u);
+        else emit_rotation(q, c, s, u);
         px[q] = swap ? 1 : 0;
+        set_pending(q, swap ? d : cplx64{1.0, 0.0}, swap ? cplx64{1.0, 0.0} : d);
         return;
       }
       if (swap) {
@@ -1027,20 +1043,30 @@ struct Decomposer {
       out.push_back(o);
       return;
     }
-    const cplx64 s0 = Dp[0];
-    const cplx64 x1 = cdiv(Dp[1], s0), y1 = cdiv(Dp[2], s0);
-    // a diagonal gate's own part does not depend on the pending diagonals (CZ: exactly -1)
-    const cplx64 gamma = src.perm == 0xE4 ? cdiv(cm(php[0], php[3]), cm(php[1], php[2])) : cdiv(Dp[3], cm(s0, cm(x1, y1)));
+    // Dp[z] = s0 x1^z0 y1^z1 gamma^(z0 z1): the gate's own phases, and of each
+    // pending diag(a, b) the a in s0 and b / a by the bit of its qubit that row z
+    // reads, an affine function of z0 and z1
+    cplx64 s0 = php[0], x1 = cdiv(php[1], php[0]), y1 = cdiv(php[2], php[0]);
+    cplx64 gamma = cdiv(cm(php[0], php[3]), cm(php[1], php[2]));
+    for (int j = 0; j < 2; ++j) {
+      const cplx64 a = pa[j ? q1 : q0], w = cdiv(pb[j ? q1 : q0], a), wi = cdiv({1.0, 0.0}, w);
+      int bit[4];
+      for (int z = 0; z < 4; ++z) bit[z] = (column(z ^ mo) >> j) & 1;
+      s0 = cm(s0, a);
+      if (bit[0]) s0 = cm(s0, w);
+      if (bit[1] != bit[0]) x1 = cm(x1, bit[1] ? w : wi);
+      if (bit[2] != bit[0]) y1 = cm(y1, bit[2] ? w : wi);
+      const int g = bit[3] + bit[0] - bit[1] - bit[2];       // 0, 2 or -2
+      if (g) gamma = cm(gamma, cm(g > 0 ? w : wi, g > 0 ? w : wi));
+    }
     G = cm(G, s0);
     px[q0] = (uint8_t)(mo & 1);
     px[q1] = (uint8_t)(mo >> 1);
-    pa[q0] = pa[q1] = {1.0, 0.0};
-    pb[q0] = x1;
-    pb[q1] = y1;
-    if (px[q0]) std::swap(pa[q0], pb[q0]);   // the diagonal comes after the X
-    if (px[q1]) std::swap(pa[q1], pb[q1]);
+    // the diagonal comes after the X
+    set_pending(q0, px[q0] ? x1 : cplx64{1.0, 0.0}, px[q0] ? cplx64{1.0, 0.0} : x1);
+    set_pending(q1, px[q1] ? y1 : cplx64{1.0, 0.0}, px[q1] ? cplx64{1.0, 0.0} : y1);
     SchedOp o = src;
-    const bool unit = unit_phase(gamma);
+    const bool unit = is_one(gamma);
     o.unit = unit ? 1 : 0;
     o.urows = unit ? 15 : 7;
     o.nrows = (gamma.re == -1.0 && gamma.im == 0.0) ? 8 : 0;
@@ -1109,12 +1135,9 @@ void decompose_one_qubit_ops(std::vector<SchedOp>& ops, std::vector<cplx64>& poo
       if (o.perm & 1) {
         if (mode == DECOMP_STEADY) dc.px[q] ^= 1;
         else dc.emit_x(q);
-        const cplx64 a = cm(p0, dc.pb[q]), b = cm(p1, dc.pa[q]);
-        dc.pa[q] = a;
-        dc.pb[q] = b;
+        dc.set_pending(q, cm(p0, dc.pb[q]), cm(p1, dc.pa[q]));
       } else {
-        dc.pa[q] = cm(dc.pa[q], p0);
-        dc.pb[q] = cm(dc.pb[q], p1);
+        dc.set_pending(q, cm(dc.pa[q], p0), cm(dc.pb[q], p1));
       }
     } else if (o.k == 2 && o.mono) {
       dc.mono2(o);
