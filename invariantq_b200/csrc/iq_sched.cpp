@@ -799,10 +799,29 @@ void normalize_one_qubit_ops(std::vector<SchedOp>& ops, std::vector<cplx64>& poo
 
 namespace {
 
-inline cplx64 cdiv(cplx64 a, cplx64 b) {
-  const double n = b.re * b.re + b.im * b.im;
-  return {(a.re * b.re + a.im * b.im) / n, (a.im * b.re - a.re * b.im) / n};
+// A product or quotient in extended precision, rounded once: the scalar of a
+// whole circuit, the entries of merged diagonals, phases.  (|b|^2 of a phase
+// rounded to double before a division is biased: the grid is twice as coarse
+// above 1 as below.)
+struct WideScalar {
+  long double re = 1.0L, im = 0.0L;
+  void times(WideScalar f) {
+    const long double r = re * f.re - im * f.im;
+    im = re * f.im + im * f.re;
+    re = r;
+  }
+  void times(cplx64 f) { times(WideScalar{f.re, f.im}); }
+  WideScalar inverse() const {
+    const long double n = re * re + im * im;
+    return {re / n, -im / n};
+  }
+  cplx64 rounded() const { return {(double)re, (double)im}; }
+};
+WideScalar quotient(cplx64 a, cplx64 b) {
+  const long double n = (long double)b.re * b.re + (long double)b.im * b.im;
+  return {((long double)a.re * b.re + (long double)a.im * b.im) / n, ((long double)a.im * b.re - (long double)a.re * b.im) / n};
 }
+inline cplx64 cdiv(cplx64 a, cplx64 b) { return quotient(a, b).rounded(); }
 inline double cabs2(cplx64 a) { return a.re * a.re + a.im * a.im; }
 inline bool is_one(cplx64 a) { return a.re == 1.0 && a.im == 0.0; }
 
@@ -817,7 +836,7 @@ struct Decomposer {
   std::vector<cplx64>& pool;
   std::vector<cplx64> pa, pb;   // pending output diagonal diag(pa[q], pb[q]) of each qubit (set_pending)
   std::vector<uint8_t> px;      // DECOMP_STEADY: a pending X of the qubit, before that diagonal
-  cplx64 G{1.0, 0.0};           // scalar factored out of the emitted operations
+  WideScalar G;                 // scalar factored out of the emitted operations
   DecompMode mode;
   int rotations = 0;            // since the last scalar
   // a tan form divides by c >= 1/sqrt 2: this many keep the scale above 2^-96
@@ -830,7 +849,7 @@ struct Decomposer {
   // a has modulus 1 (other diagonals keep their scale to themselves)
   void set_pending(int q, cplx64 a, cplx64 b) {
     if (std::fabs(cabs2(a) - 1.0) < 1e-12 && !is_one(a)) {
-      G = cm(G, a);
+      G.times(a);
       b = (b.re == a.re && b.im == a.im) ? cplx64{1.0, 0.0} : cdiv(b, a);
       a = {1.0, 0.0};
     }
@@ -845,7 +864,7 @@ struct Decomposer {
   // one-qubit diagonal diag(a, b) = a diag(1, b / a): the scalar goes to G
   void emit_phase(int q, cplx64 a, cplx64 b, bool always = false) {
     const cplx64 r = cdiv(b, a);
-    G = cm(G, a);
+    G.times(a);
     if (is_one(r) && !always) return;
     SchedOp o{};
     o.k = 1;
@@ -869,16 +888,17 @@ struct Decomposer {
     pa[q] = pb[q] = {1.0, 0.0};
   }
   void emit_scalar(int q) {
-    if (is_one(G)) return;
+    const cplx64 g = G.rounded();
+    if (is_one(g)) return;
     SchedOp o{};
     o.k = 1;
     o.q[0] = (uint8_t)q;
     o.mono = 1;
     o.perm = 0;
-    o.mat = put({G, G});
-    o.dense = put({G, {0.0, 0.0}, {0.0, 0.0}, G});
+    o.mat = put({g, g});
+    o.dense = put({g, {0.0, 0.0}, {0.0, 0.0}, g});
     out.push_back(o);
-    G = {1.0, 0.0};
+    G = WideScalar{};
   }
   void emit_x(int q) {
     SchedOp o{};
@@ -899,19 +919,21 @@ struct Decomposer {
     o.q[0] = (uint8_t)q;
     if (c >= std::fabs(s)) {
       const double t = s / c;
-      G = cm(G, {g.re * c, g.im * c});
+      G.times(g);
+      G.times(cplx64{c, 0.0});
       o.rot = 1;
       o.dense = put({{1.0, 0.0}, {-t, 0.0}, {t, 0.0}, {1.0, 0.0}});
     } else {
       const double u = c / s;
-      G = cm(G, {g.re * s, g.im * s});
+      G.times(g);
+      G.times(cplx64{s, 0.0});
       o.rot = 2;
       o.dense = put({{u, 0.0}, {-1.0, 0.0}, {1.0, 0.0}, {u, 0.0}});
     }
     o.mat = o.dense;
     out.push_back(o);
     // keep the scale of the intermediate state within 2^+-100
-    const double g2 = cabs2(G);
+    const double g2 = cabs2(G.rounded());
     ++rotations;
     if (g2 < 0x1p-200 || g2 > 0x1p200 || (mode != DECOMP_BY_ANGLE && rotations >= kScalarEvery)) {
       emit_scalar(q);
@@ -925,7 +947,7 @@ struct Decomposer {
     o.realm = 1;
     o.dense = o.mat = put({{c, 0.0}, {-s, 0.0}, {s, 0.0}, {c, 0.0}});
     out.push_back(o);
-    G = cm(G, g);
+    G.times(g);
   }
   // dense one-qubit U (row-major) on q, after the pending diagonal of q
   // (`last`: no dense one-qubit operation on q follows)
@@ -969,8 +991,8 @@ struct Decomposer {
       // u diag(1, d) [[c, -s], [s, c]] diag(1, e), u the phase of A: a real gate gives d and e of exactly +-1
       const double c = swap ? s0 : c0;
       double s = swap ? c0 : s0;
-      const cplx64 u{A.re / c, A.im / c}, uc{u.re, -u.im};
-      const cplx64 du = cm(C, uc), eu = cm(B, uc);
+      const cplx64 u{A.re / c, A.im / c};
+      const cplx64 du = cdiv(C, u), eu = cdiv(B, u);   // divided: |u| is 1 up to rounding only, and the same way each time
       cplx64 d{du.re / s, du.im / s}, e{-eu.re / s, -eu.im / s};
       if (mode != DECOMP_BY_ANGLE && e.re < 0.0) {   // the sign goes to s: a real gate has no phase, whatever its angle
         s = -s;
@@ -1046,36 +1068,39 @@ struct Decomposer {
     // Dp[z] = s0 x1^z0 y1^z1 gamma^(z0 z1): the gate's own phases, and of each
     // pending diag(a, b) the a in s0 and b / a by the bit of its qubit that row z
     // reads, an affine function of z0 and z1
-    cplx64 s0 = php[0], x1 = cdiv(php[1], php[0]), y1 = cdiv(php[2], php[0]);
-    cplx64 gamma = cdiv(cm(php[0], php[3]), cm(php[1], php[2]));
+    WideScalar s0, x1 = quotient(php[1], php[0]), y1 = quotient(php[2], php[0]), gamma = quotient(php[3], php[0]);
+    s0.times(php[0]);
+    gamma.times(x1.inverse());
+    gamma.times(y1.inverse());
     for (int j = 0; j < 2; ++j) {
-      const cplx64 a = pa[j ? q1 : q0], w = cdiv(pb[j ? q1 : q0], a), wi = cdiv({1.0, 0.0}, w);
+      const cplx64 a = pa[j ? q1 : q0];
+      const WideScalar w = quotient(pb[j ? q1 : q0], a), wi = w.inverse();
       int bit[4];
       for (int z = 0; z < 4; ++z) bit[z] = (column(z ^ mo) >> j) & 1;
-      s0 = cm(s0, a);
-      if (bit[0]) s0 = cm(s0, w);
-      if (bit[1] != bit[0]) x1 = cm(x1, bit[1] ? w : wi);
-      if (bit[2] != bit[0]) y1 = cm(y1, bit[2] ? w : wi);
-      const int g = bit[3] + bit[0] - bit[1] - bit[2];       // 0, 2 or -2
-      if (g) gamma = cm(gamma, cm(g > 0 ? w : wi, g > 0 ? w : wi));
+      s0.times(a);
+      if (bit[0]) s0.times(w);
+      if (bit[1] != bit[0]) x1.times(bit[1] ? w : wi);
+      if (bit[2] != bit[0]) y1.times(bit[2] ? w : wi);
+      for (int g = bit[3] + bit[0] - bit[1] - bit[2]; g; g += g > 0 ? -1 : 1) gamma.times(g > 0 ? w : wi);   // 0, 2 or -2
     }
-    G = cm(G, s0);
+    G.times(s0);
     px[q0] = (uint8_t)(mo & 1);
     px[q1] = (uint8_t)(mo >> 1);
     // the diagonal comes after the X
-    set_pending(q0, px[q0] ? x1 : cplx64{1.0, 0.0}, px[q0] ? cplx64{1.0, 0.0} : x1);
-    set_pending(q1, px[q1] ? y1 : cplx64{1.0, 0.0}, px[q1] ? cplx64{1.0, 0.0} : y1);
+    const cplx64 one{1.0, 0.0}, xr = x1.rounded(), yr = y1.rounded(), gr = gamma.rounded();
+    set_pending(q0, px[q0] ? xr : one, px[q0] ? one : xr);
+    set_pending(q1, px[q1] ? yr : one, px[q1] ? one : yr);
     SchedOp o = src;
-    const bool unit = is_one(gamma);
+    const bool unit = is_one(gr);
     o.unit = unit ? 1 : 0;
     o.urows = unit ? 15 : 7;
-    o.nrows = (gamma.re == -1.0 && gamma.im == 0.0) ? 8 : 0;
-    o.mat = put({{1.0, 0.0}, {1.0, 0.0}, {1.0, 0.0}, gamma});
+    o.nrows = (gr.re == -1.0 && gr.im == 0.0) ? 8 : 0;
+    o.mat = put({{1.0, 0.0}, {1.0, 0.0}, {1.0, 0.0}, gr});
     o.dense = (uint32_t)pool.size();
     for (int r = 0; r < 4; ++r)
       for (int c = 0; c < 4; ++c) {
         const bool hit = ((src.perm >> (2 * r)) & 3) == c;
-        pool.push_back(hit ? (r == 3 ? gamma : cplx64{1.0, 0.0}) : cplx64{0.0, 0.0});
+        pool.push_back(hit ? (r == 3 ? gr : cplx64{1.0, 0.0}) : cplx64{0.0, 0.0});
       }
     out.push_back(o);
   }
@@ -1770,7 +1795,14 @@ void PackRecipe::fill(const cplx64* pool, cplx64* dst) const {
     return i == kPackOne ? cplx64{1.0, 0.0} : (i == kPackMinusOne ? cplx64{-1.0, 0.0} : pool[i]);
   };
   for (size_t i = 0; i < base.size(); ++i) dst[i] = at(base[i]);
-  for (const auto& m : mults) dst[m.first] = cm(dst[m.first], at(m.second));
+  // an element's factors follow each other; their product is rounded once (an
+  // entry's error is shared by every amplitude it multiplies)
+  for (size_t k = 0; k < mults.size();) {
+    const uint32_t i = mults[k].first;
+    WideScalar w{dst[i].re, dst[i].im};
+    for (; k < mults.size() && mults[k].first == i; ++k) w.times(at(mults[k].second));
+    dst[i] = w.rounded();
+  }
 }
 
 void pack_pass_matrices(std::vector<PassPlan>& plans, const cplx64* pool, std::vector<cplx64>& packed) {
