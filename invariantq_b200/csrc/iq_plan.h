@@ -424,7 +424,8 @@ struct cplx64 { double re, im; };
 // Operation order per qubit is preserved.  Returns the fused list.
 // With monomial_barrier, two-qubit monomials (CX, CZ, SWAP: free renamings or
 // phase products in the specialised kernels) are left alone and end the
-// one-qubit runs of their qubits.
+// one-qubit runs of their qubits, and so are the phases at a run's ends, which
+// decompose_one_qubit_ops carries along.
 std::vector<SchedOp> fuse_two_qubit_blocks(const std::vector<SchedOp>& ops, std::vector<cplx64>& pool,
                                            bool monomial_barrier = false);
 // Divide every dense one-qubit operation but the last of each run of at most
@@ -451,16 +452,19 @@ void normalize_one_qubit_ops(std::vector<SchedOp>& ops, std::vector<cplx64>& poo
 // the larger of |c| and |s|, X is emitted where a gate or a pending diagonal
 // makes one, and scalars where their magnitude asks for it.  Kernels compiled
 // for one circuit's structure then do not fit the next circuit of the same
-// gates, so two steadier forms exist: DECOMP_STEADY_SCALARS emits the scalar
+// gates, so steadier forms exist: DECOMP_STEADY_SCALARS emits the scalar
 // after a fixed number of rotations; DECOMP_STEADY also pulls an X out of every
 // gate with |c| < |s| (the tan form always), carries pending X operators
 // through the later gates as it does diagonals, and writes each qubit's last
 // rotation as a plain real 2x2 that absorbs the pending X (2 multiply-adds per
-// amplitude more, once per qubit).
+// amplitude more, once per qubit); DECOMP_STEADY_ENDS also writes the X and the
+// phase that carried operators may have left on a qubit at the end of the list
+// (a qubit whose last rotation comes before a two-qubit gate with one that still
+// turns) whether they are there or not.
 // A phase is dropped only if it is exactly 1; phases that cancel are formed so
 // that they come out exactly 1, and one that only rounding keeps from 1 (a
 // fused product of complex gates, nothing pending) is emitted for every angle.
-enum DecompMode { DECOMP_BY_ANGLE = 0, DECOMP_STEADY_SCALARS = 1, DECOMP_STEADY = 2 };
+enum DecompMode { DECOMP_BY_ANGLE = 0, DECOMP_STEADY_SCALARS = 1, DECOMP_STEADY = 2, DECOMP_STEADY_ENDS = 3 };
 void decompose_one_qubit_ops(std::vector<SchedOp>& ops, std::vector<cplx64>& pool, DecompMode mode = DECOMP_BY_ANGLE);
 // Re-pack the matrix data each pass references (absolute offsets into `pool`)
 // into one contiguous block per pass: sets desc.mat_base / mat_elems and makes
@@ -550,7 +554,11 @@ struct AdjointOps {
   PauliFrame frame;                  // with `framed` only
   std::vector<int8_t> grad_sign;
 };
-// framed: with single_set, in a Pauli frame -- one structure for every parameter set
+// framed: with single_set, in a Pauli frame -- one structure for every parameter
+// set, but for angles at which a gate degenerates (a rotation by exactly 0 or pi
+// is left out, one by pi/2 may tie).  Where neighbouring one-qubit gates multiply
+// into one whose larger modulus the angles decide, the forward list carries X
+// operators (DECOMP_STEADY_ENDS).
 void adjoint_ops(int n, const std::vector<AnsatzOp>& ops, const double* params, bool backward, bool fuse,
                  bool single_set, AdjointOps& j, bool framed = false);
 // The scale factors of a backward sweep's gradient terms in the order the

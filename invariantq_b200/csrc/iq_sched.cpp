@@ -590,6 +590,46 @@ struct Block {
   bool xpat = false;    // a run of OP_X2R-shaped operations on one pair, kept apart from one-qubit blocks
 };
 
+// The phases at either end of a run of one-qubit operations between barriers (of
+// which `ends` says where they are).  They stay out of the run's product: the
+// decomposition carries them along as they are, where a product's entries would
+// give them back up to rounding only, as phases that are 1 or not by the angles.
+template <class Barrier>
+std::vector<uint8_t> phases_at_ends(const std::vector<SchedOp>& ops, const std::vector<cplx64>& pool, Barrier ends) {
+  struct Run { bool only = true, dense = false; std::vector<size_t> tail; };   // only: since a barrier, one-qubit operations
+  std::vector<Run> runs(64);
+  std::vector<uint8_t> alone(ops.size(), 0);
+  auto unit = [](cplx64 a) { return std::fabs(a.re * a.re + a.im * a.im - 1.0) < 1e-12; };
+  auto end = [&](Run& r) {
+    if (r.only)
+      for (size_t i : r.tail) alone[i] = 1;
+    r = Run{};
+  };
+  for (size_t i = 0; i < ops.size(); ++i) {
+    const SchedOp& o = ops[i];
+    if (ends(o)) {
+      for (int j = 0; j < o.k; ++j) end(runs[o.q[j]]);
+    } else if (o.k == 2) {
+      for (int j = 0; j < 2; ++j) {
+        runs[o.q[j]].only = false;
+        runs[o.q[j]].tail.clear();
+      }
+    } else {
+      Run& r = runs[o.q[0]];
+      if (!o.mono || (o.perm & 1) || (!o.unit && !(unit(pool[o.mat]) && unit(pool[o.mat + 1])))) {
+        r.dense = true;
+        r.tail.clear();
+      } else if (r.only && !r.dense) {
+        alone[i] = 1;
+      } else {
+        r.tail.push_back(i);
+      }
+    }
+  }
+  for (Run& r : runs) end(r);
+  return alone;
+}
+
 }  // namespace
 
 std::vector<SchedOp> fuse_two_qubit_blocks(const std::vector<SchedOp>& ops, std::vector<cplx64>& pool,
@@ -605,6 +645,11 @@ std::vector<SchedOp> fuse_two_qubit_blocks(const std::vector<SchedOp>& ops, std:
     m[0] = U[0]; m[1] = U[1]; m[4] = U[2]; m[5] = U[3];
     return m;
   };
+  std::vector<uint8_t> alone;
+  if (monomial_barrier)
+    alone = phases_at_ends(ops, pool, [](const SchedOp& o) {   // what ends a run in the loop below
+      return o.k >= 3 || o.grad || o.smul != 0.0 || (o.k == 2 && (o.mono || o.xpat));
+    });
   for (size_t i = 0; i < ops.size(); ++i) {
     const SchedOp& o = ops[i];
     // wide blocks and adjoint steps pass through unchanged, and so do two-qubit
@@ -640,7 +685,7 @@ std::vector<SchedOp> fuse_two_qubit_blocks(const std::vector<SchedOp>& ops, std:
       blocks.push_back(b);
       continue;
     }
-    if (o.k >= 3 || o.grad || o.smul != 0.0 || (monomial_barrier && o.k == 2 && o.mono)) {
+    if (o.k >= 3 || o.grad || o.smul != 0.0 || (monomial_barrier && ((o.k == 2 && o.mono) || alone[i]))) {
       for (int j = 0; j < o.k; ++j) { open[o.q[j]] = -1; last[o.q[j]] = (int)blocks.size(); }
       Block b;
       b.k = 0;
@@ -835,7 +880,10 @@ struct Decomposer {
   std::vector<SchedOp>& out;
   std::vector<cplx64>& pool;
   std::vector<cplx64> pa, pb;   // pending output diagonal diag(pa[q], pb[q]) of each qubit (set_pending)
-  std::vector<uint8_t> px;      // DECOMP_STEADY: a pending X of the qubit, before that diagonal
+  std::vector<uint8_t> px;      // a pending X of the qubit, before that diagonal (modes that carry them)
+  // DECOMP_STEADY_ENDS: the angles decide whether an X (bit 0) or a sign of the
+  // pending diagonal (bit 1) is pending
+  std::vector<uint8_t> open;
   WideScalar G;                 // scalar factored out of the emitted operations
   DecompMode mode;
   int rotations = 0;            // since the last scalar
@@ -843,7 +891,8 @@ struct Decomposer {
   static constexpr int kScalarEvery = 192;
 
   Decomposer(std::vector<SchedOp>& o, std::vector<cplx64>& p, DecompMode m)
-      : out(o), pool(p), pa(64, {1.0, 0.0}), pb(64, {1.0, 0.0}), px(64, 0), mode(m) {}
+      : out(o), pool(p), pa(64, {1.0, 0.0}), pb(64, {1.0, 0.0}), px(64, 0), open(64, 0), mode(m) {}
+  bool carries() const { return mode == DECOMP_STEADY || mode == DECOMP_STEADY_ENDS; }   // pending X operators
 
   // the pending diagonal of q becomes diag(a, b): diag(1, b / a), a in G, when
   // a has modulus 1 (other diagonals keep their scale to themselves)
@@ -886,6 +935,25 @@ struct Decomposer {
     if (is_one(pa[q]) && is_one(pb[q])) return;
     emit_phase(q, pa[q], pb[q]);
     pa[q] = pb[q] = {1.0, 0.0};
+  }
+  // at the end of the list
+  void close(int q) {
+    if (mode == DECOMP_STEADY_ENDS && open[q]) {
+      if (open[q] & 1) {   // X or the identity, as a real 2x2
+        const cplx64 x{(double)px[q], 0.0}, i{1.0 - px[q], 0.0};
+        SchedOp o{};
+        o.k = 1;
+        o.q[0] = (uint8_t)q;
+        o.realm = 1;
+        o.dense = o.mat = put({i, x, x, i});
+        out.push_back(o);
+        px[q] = 0;
+      }
+      emit_phase(q, pa[q], pb[q], true);
+      pa[q] = pb[q] = {1.0, 0.0};
+      return;
+    }
+    flush(q);
   }
   void emit_scalar(int q) {
     const cplx64 g = G.rounded();
@@ -953,7 +1021,7 @@ struct Decomposer {
   // (`last`: no dense one-qubit operation on q follows)
   void dense1(const SchedOp& src, bool last) {
     const int q = src.q[0];
-    const bool steady = mode == DECOMP_STEADY;
+    const bool steady = carries();
     const cplx64* U = pool.data() + src.dense;
     cplx64 A = U[0], B = U[1], C = U[2], D = U[3];
     if (px[q]) {   // the pending X swaps the columns, and the diagonal's entries with them
@@ -994,19 +1062,21 @@ struct Decomposer {
       const cplx64 u{A.re / c, A.im / c};
       const cplx64 du = cdiv(C, u), eu = cdiv(B, u);   // divided: |u| is 1 up to rounding only, and the same way each time
       cplx64 d{du.re / s, du.im / s}, e{-eu.re / s, -eu.im / s};
-      if (mode != DECOMP_BY_ANGLE && e.re < 0.0) {   // the sign goes to s: a real gate has no phase, whatever its angle
+      // A and B both real or both imaginary: e is 1 or not for every angle
+      const bool exact = (A.im == 0.0 && B.im == 0.0) || (A.re == 0.0 && B.re == 0.0);
+      // the sign goes to s: a real gate has no phase, whatever its angle (behind a pending one, none after it)
+      if (mode != DECOMP_BY_ANGLE && (exact ? e.re < 0.0 : d.im == 0.0 && d.re < 0.0)) {
         s = -s;
         d = {-d.re, -d.im};
         e = {-e.re, -e.im};
       }
       const cplx64 Dr = cm(cm(u, cm(d, e)), {c, 0.0});      // the rebuilt entry D
       if (cabs2({Dr.re - D.re, Dr.im - D.im}) < 1e-28) {
-        // A and B both real or both imaginary: e is 1 or not for every angle
-        const bool exact = (A.im == 0.0 && B.im == 0.0) || (A.re == 0.0 && B.re == 0.0);
         emit_phase(q, {1.0, 0.0}, e, mode != DECOMP_BY_ANGLE && !exact);
         if (steady && last) emit_real(q, c, s, u);
         else emit_rotation(q, c, s, u);
         px[q] = swap ? 1 : 0;
+        open[q] = last ? (open[q] ? 2 : 0) : 3;
         set_pending(q, swap ? d : cplx64{1.0, 0.0}, swap ? cplx64{1.0, 0.0} : d);
         return;
       }
@@ -1037,6 +1107,13 @@ struct Decomposer {
     const int m = (px[q0] ? 1 : 0) | (px[q1] ? 2 : 0);
     int mo = 0;
     while ((column(mo) ^ column(0)) != m) ++mo;
+    if (open[q0] | open[q1]) {   // an X spreads as this permutation's does, its sign to both qubits
+      int may = 0;
+      for (int z = 1; z < 4; ++z)
+        if (((column(z) ^ column(0)) & ~((open[q0] & 1) | (open[q1] & 1) << 1)) == 0) may |= z;
+      open[q0] = (uint8_t)((may & 1) | 2);
+      open[q1] = (uint8_t)((may >> 1) | 2);
+    }
     cplx64 Dp[4], php[4];
     for (int z = 0; z < 4; ++z) {
       const int r = z ^ mo, col = column(r);
@@ -1158,7 +1235,7 @@ void decompose_one_qubit_ops(std::vector<SchedOp>& ops, std::vector<cplx64>& poo
       const int q = o.q[0];
       const cplx64 p0 = o.unit ? cplx64{1.0, 0.0} : pool[o.mat], p1 = o.unit ? cplx64{1.0, 0.0} : pool[o.mat + 1];
       if (o.perm & 1) {
-        if (mode == DECOMP_STEADY) dc.px[q] ^= 1;
+        if (dc.carries()) dc.px[q] ^= 1;
         else dc.emit_x(q);
         dc.set_pending(q, cm(p0, dc.pb[q]), cm(p1, dc.pa[q]));
       } else {
@@ -1171,7 +1248,7 @@ void decompose_one_qubit_ops(std::vector<SchedOp>& ops, std::vector<cplx64>& poo
     }
     last_q = o.q[0];
   }
-  for (int q = 0; q < 64; ++q) dc.flush(q);
+  for (int q = 0; q < 64; ++q) dc.close(q);
   dc.emit_scalar(last_q);
   ops.swap(out);
 }
@@ -1450,6 +1527,48 @@ void ansatz_backward(int n, const std::vector<AnsatzOp>& ops, const double* para
   }
 }
 
+namespace {
+
+// Whether the angles decide which of |c| and |s| is larger in a product of
+// neighbouring one-qubit gates of a framed circuit (its rotations have |c| >=
+// |s|).  They do not in a run of one X or Y rotation, H or SX (an H or SX with Z
+// rotations on one side only: on both, rounding decides between equal moduli),
+// nor in RX and RY side by side ((1 + cos a cos b) / 2 >= 1/2).
+bool runs_tilt(const std::vector<AnsatzOp>& ops) {
+  struct Run { int tilts = 0, gen = -1; bool z = false, z_after = false; };   // gen: 0 X, 1 Y rotation, 2 H or SX
+  std::vector<Run> runs(64);
+  for (const AnsatzOp& o : ops) {
+    if (o.q1 >= 0) {   // a two-qubit gate ends its qubits' runs
+      runs[o.q0] = runs[o.q1] = Run{};
+      continue;
+    }
+    Run& r = runs[o.q0];
+    auto turn = [&](int gen) {
+      if (gen == 3) {   // about Z
+        if (r.gen == 2 && r.z) return true;
+        (r.tilts ? r.z_after : r.z) = true;
+        return false;
+      }
+      const bool side = r.tilts == 1 && !r.z_after && gen < 2 && r.gen < 2 && gen != r.gen;
+      ++r.tilts;
+      if (r.tilts > 1 && !side) return true;
+      r.gen = gen;
+      return false;
+    };
+    switch (o.kind) {
+      case GATE_RX: if (turn(0)) return true; break;
+      case GATE_RY: if (turn(1)) return true; break;
+      case GATE_RZ: case GATE_P: if (turn(3)) return true; break;
+      case GATE_U3: if (turn(3) || turn(1) || turn(3)) return true; break;
+      case GATE_H: case GATE_SX: if (turn(2)) return true; break;
+      default: break;   // X
+    }
+  }
+  return false;
+}
+
+}  // namespace
+
 void adjoint_ops(int n, const std::vector<AnsatzOp>& ops, const double* params, bool backward, bool fuse,
                  bool single_set, AdjointOps& j, bool framed) {
   j.fw.clear(); j.bw.clear(); j.fpool.clear(); j.bpool.clear(); j.grad_param.clear(); j.grad_scale.clear();
@@ -1462,7 +1581,7 @@ void adjoint_ops(int n, const std::vector<AnsatzOp>& ops, const double* params, 
   ansatz_forward(n, ops, params, raw, j.fpool, /*phase_free=*/!single_set, frame);
   if (single_set) {
     j.fw = fuse_two_qubit_blocks(raw, j.fpool, true);
-    decompose_one_qubit_ops(j.fw, j.fpool, framed ? DECOMP_STEADY_SCALARS : DECOMP_BY_ANGLE);
+    decompose_one_qubit_ops(j.fw, j.fpool, !framed ? DECOMP_BY_ANGLE : runs_tilt(ops) ? DECOMP_STEADY_ENDS : DECOMP_STEADY_SCALARS);
     normalize_one_qubit_ops(j.fw, j.fpool);
   } else {
     // forms that do not depend on the angles, every gate alone: RY (and any

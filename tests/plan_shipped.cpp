@@ -328,3 +328,27 @@ extern "C" int shipped_adjoint(int n, int nops, const int* kinds, const int* q0,
   for (const SchedOp& o : jo.bw) counts[2] += o.smul != 0.0 && !o.grad;
   return 0;
 }
+
+// Fingerprint of the plans (what shapes and kernels are found by) of one
+// parameter set's forward or backward list; 0 on an error.
+extern "C" unsigned long long shipped_structure(int n, int nops, const int* kinds, const int* q0, const int* q1,
+                                                const int* pidx, const double* params, int backward) {
+  std::vector<AnsatzOp> ops(nops);
+  for (int i = 0; i < nops; ++i) ops[i] = {kinds[i], q0[i], q1[i], pidx[i]};
+  std::string err;
+  if (ansatz_check(n, ops, err) < 0) return 0;
+  AdjointOps jo;
+  adjoint_ops(n, ops, params, true, true, true, jo, true);
+  const std::vector<SchedOp>& list = backward ? jo.bw : jo.fw;
+  SchedParams p = sched_params(12, 4, 4, 8, 160.0);
+  p.nbits = n + (backward ? 1 : 0);
+  std::vector<PassPlan> plans;
+  if (plan_passes(p, list, plans, err) < 0) return 0;
+  merge_stage_diagonals(plans, list);
+  PackRecipe rec;
+  pack_recipe(plans, rec);
+  uint64_t h = 1469598103934665603ull;
+  for (const PassPlan& pl : plans)
+    for (unsigned char ch : jit_pass_key(pl.desc, 3, 128, true, false)) h = (h ^ ch) * 1099511628211ull;
+  return h;
+}
