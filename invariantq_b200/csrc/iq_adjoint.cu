@@ -25,6 +25,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <atomic>
 #include <chrono>
 #include <cmath>
@@ -247,8 +248,10 @@ bool make_shape(const Cfg& cfg, int nbits, const std::vector<SchedOp>& fused, si
 // and the settings, so any circuit of the same gates shares them; at most
 // kMaxShapes, the least recently used goes first; iq_adjoint_release drops them.
 constexpr size_t kMaxShapes = 64;
+using ShapeSettings = std::array<uint64_t, 14>;   // what a plan follows besides the operations
 struct ShapeEntry {
-  uint64_t key;
+  uint64_t key;              // hash of the settings and the operations
+  ShapeSettings settings;
   uint64_t used;
   std::shared_ptr<const Shape> shape;
 };
@@ -256,18 +259,22 @@ std::mutex g_shape_mu;
 std::vector<ShapeEntry>* g_shapes = new std::vector<ShapeEntry>();
 uint64_t g_shape_clock = 0;
 
-uint64_t shape_key(const Cfg& cfg, int dev, int nbits, const std::vector<SchedOp>& ops, size_t pool_size, int num_sms) {
-  uint64_t h = 1469598103934665603ull;
-  auto put = [&](uint64_t v) { h = (h ^ v) * 1099511628211ull; };
-  for (uint64_t v : {(uint64_t)dev, (uint64_t)nbits, (uint64_t)pool_size, (uint64_t)num_sms, (uint64_t)cfg.sp.M,
-                     (uint64_t)cfg.sp.c, (uint64_t)cfg.sp.R, (uint64_t)cfg.sp.max_stages, (uint64_t)cfg.tl.nbuf,
-                     (uint64_t)cfg.tl.ctas_per_sm, (uint64_t)cfg.jit, (uint64_t)cfg.c64, (uint64_t)ops.size()})
-    put(v);
-  for (double v : {cfg.sp.budget, cfg.sp.grad_cost}) {
+ShapeSettings shape_settings(const Cfg& cfg, int dev, int nbits, size_t pool_size, int num_sms) {
+  auto bits = [](double v) {
     uint64_t b;
     std::memcpy(&b, &v, 8);
-    put(b);
-  }
+    return b;
+  };
+  return {(uint64_t)dev, (uint64_t)nbits, (uint64_t)pool_size, (uint64_t)num_sms, (uint64_t)cfg.sp.M, (uint64_t)cfg.sp.c,
+          (uint64_t)cfg.sp.R, (uint64_t)cfg.sp.max_stages, (uint64_t)cfg.tl.nbuf, (uint64_t)cfg.tl.ctas_per_sm,
+          (uint64_t)cfg.jit, (uint64_t)cfg.c64, bits(cfg.sp.budget), bits(cfg.sp.grad_cost)};
+}
+
+uint64_t shape_key(const ShapeSettings& settings, const std::vector<SchedOp>& ops) {
+  uint64_t h = 1469598103934665603ull;
+  auto put = [&](uint64_t v) { h = (h ^ v) * 1099511628211ull; };
+  for (uint64_t v : settings) put(v);
+  put(ops.size());
   for (const SchedOp& o : ops) {
     put(o.k | (uint64_t)o.mono << 8 | (uint64_t)o.perm << 16 | (uint64_t)o.unit << 24 | (uint64_t)o.norm << 32 |
         (uint64_t)o.rot << 40 | (uint64_t)o.urows << 48 | (uint64_t)o.nrows << 56);
@@ -280,10 +287,11 @@ uint64_t shape_key(const Cfg& cfg, int dev, int nbits, const std::vector<SchedOp
 
 std::shared_ptr<const Shape> shape_for(const Cfg& cfg, int dev, int nbits, const std::vector<SchedOp>& ops,
                                        size_t pool_size, int num_sms, int ngrads, std::string& err) {
-  const uint64_t key = shape_key(cfg, dev, nbits, ops, pool_size, num_sms);
-  auto find = [&]() -> std::shared_ptr<const Shape> {   // g_shape_mu held; the key's whole structure is compared
+  const ShapeSettings settings = shape_settings(cfg, dev, nbits, pool_size, num_sms);
+  const uint64_t key = shape_key(settings, ops);
+  auto find = [&]() -> std::shared_ptr<const Shape> {   // g_shape_mu held; settings and operations are compared whole
     for (ShapeEntry& e : *g_shapes)
-      if (e.key == key && e.shape->nbits == nbits && matches(*e.shape, ops, pool_size)) {
+      if (e.key == key && e.settings == settings && matches(*e.shape, ops, pool_size)) {
         e.used = ++g_shape_clock;
         return e.shape;
       }
@@ -306,7 +314,7 @@ std::shared_ptr<const Shape> shape_for(const Cfg& cfg, int dev, int nbits, const
   if (g_shapes->size() >= kMaxShapes)
     g_shapes->erase(std::min_element(g_shapes->begin(), g_shapes->end(),
                                      [](const ShapeEntry& a, const ShapeEntry& b) { return a.used < b.used; }));
-  g_shapes->push_back({key, ++g_shape_clock, s});
+  g_shapes->push_back({key, settings, ++g_shape_clock, s});
   return s;
 }
 

@@ -385,10 +385,11 @@ struct Engine : HandleRes {
   // settings given explicitly (option or environment); the others take the
   // defaults of the plan style.  Specialised kernels: tiles of 2^12 amplitudes
   // holding the 4 lowest qubits, a budget of 160 FMAs per amplitude per pass,
-  // 3 CTAs per SM with one tile buffer each (the fastest 30-qubit brick-wall
-  // measured: 78 passes, ~627 ms, against 110 passes and ~776 ms with the
-  // interpreting kernel's 11 / 5 / 120 / 4 CTAs).  Interpreting kernel: tiles of
-  // 2^11 holding 5, budget 120, 2 CTAs per SM with three buffers.
+  // the pair pipeline (may_pair), else 3 CTAs per SM with one tile buffer each
+  // (30-qubit brick-wall of depth 40: 77 passes, 507 ms; 76 passes, 602-633 ms
+  // with the three CTAs; 110 passes, 706-776 ms with the interpreting kernel's
+  // 11 / 5 / 120 / 4 CTAs).  Interpreting kernel: tiles of 2^11 holding 5, budget
+  // 120, 2 CTAs per SM with three buffers.
   bool set_M = false, set_c = false, set_budget = false, set_nbuf = false, set_ctas = false, set_stages = false;
 
   bool spec_style() const {
