@@ -100,8 +100,12 @@ struct HamTerms {
 };
 // The Hamiltonian sweeps of iq_ham.cu: a plan (host), its tables (device) and the launch.
 constexpr int kHamMaxSweeps = 6;
-// up to this size the state stays in the caches: the few flips beyond a tile gather in the one sweep
-constexpr int kHamOneSweepBits = 18;
+// Up to this size one sweep: the few flips beyond a tile gather from the caches.
+// A sweep costs ~2 us of launch and ramp, a flip that gathers ~4 us (TFIM, one
+// state, one sweep / two: 13 qubits 25.8 / 27.9 us, 14: 29.9 / 27.9, 16: 38.2 /
+// 30.0, 18: 49.3 / 32.1; 16 states of 18 qubits 203 / 148; 60 random groups of 4
+// flips at 14 qubits 250 / 177, of any number at 18 qubits 385 / 376).
+constexpr int kHamOneSweepBits = 13;
 constexpr int kHamBlocks = 2 * 148;    // CTAs per set and sweep: two tiles of 64 KiB fit an SM
 // partial sums a launch needs per set (twice that with the imaginary part)
 constexpr size_t kHamPartials = (size_t)kHamMaxSweeps * kHamBlocks;

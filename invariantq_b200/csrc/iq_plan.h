@@ -409,7 +409,12 @@ constexpr int kPairForm = 512;
 // Time of a pass of the pair pipeline on a large array, in milliseconds at 2^30
 // amplitudes: the larger of its HBM traffic and 0.78 times the sum of its FP64
 // multiply-adds (0.065 ms each per amplitude) and its shared-memory round trips
-// (1.02 ms per stage and for the copies) -- within 8 % of passes of 2 to 6 stages.
+// (1.02 ms per stage and for the copies).  It chooses among plans, so their order
+// counts: of the limits 4, 5 and 8 it named the fastest, or one within 0.1 % of
+// it, for eight circuits of 27 to 30 qubits (brick-walls, CZ rings, QFTs of 7
+// neighbours, random pairs).  Whole circuits take 0.92-1.02 times what it says,
+// those of random pairs 1.21 (their tile bits form many runs, so more and smaller
+// copies); single passes 0.82-1.65.
 double pass_time_model(const PassDesc& d);
 inline bool pair_form_fits(const PassDesc& d) { return d.M == 12 && d.R == 4 && d.nH - d.nbox <= 7; }
 std::string jit_pass_source(const PassDesc& d, std::string& err, int min_blocks = 2, int threads = 0,
