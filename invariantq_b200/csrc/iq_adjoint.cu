@@ -976,11 +976,12 @@ int run_batch(std::vector<std::unique_ptr<Circuit>>& circs, int nstreams, bool w
       resident_sets += c->nsets;
       continue;
     }
-    plan_hamiltonian(c->n, c->ham.groups, c->ham.zmask.data(), c->ham.coef.data(), (c64 || c->n <= kHamOneSweepBits) ? 1 : kHamMaxSweeps, c->ham.plan);
-    c->ham.tables.resize(c->ham.plan.table_bytes() / 8 + 1);
-    c->ham.plan.pack(c->ham.tables.data());
     const double per_set = (c64 ? 8.0 : 16.0) * std::ldexp(1.0, joint_bits(c->n));
     const size_t group = want_grad ? (size_t)std::max(1.0, std::floor(job_bytes / per_set)) : 1;
+    plan_hamiltonian(c->n, c->ham.groups, c->ham.zmask.data(), c->ham.coef.data(),
+                     (c64 || c->n <= kHamOneSweepBits) ? 1 : kHamMaxSweeps, (int)std::min(group, c->nsets), c->ham.plan);
+    c->ham.tables.resize(c->ham.plan.table_bytes() / 8 + 1);
+    c->ham.plan.pack(c->ham.tables.data());
     // per set: at most 3 rotations per gate, each at most a dense 4x4 (16
     // elements) forward and one backward; at most 3 gradient terms per gate
     const size_t nops = c->ops.size() + 1;

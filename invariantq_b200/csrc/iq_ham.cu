@@ -24,6 +24,8 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
+#include <cstdlib>
 #include <cstring>
 #include <vector>
 
@@ -68,11 +70,20 @@ __device__ __forceinline__ double block_total(double v, double* red) {
 // words: one bit per thread].
 // Strings past kHamSmemTerms are summed from global memory, sign by sign.
 constexpr int kHamSmemTerms = 512;
+constexpr int kHamStringBytes = 32 + kHamThreads / 8 + 4;
+// Groups of up to this many strings add each string to the 16 sums with its own
+// signs (48 instructions a string); larger ones sum per pattern and transform (64
+// additions, 16 loops that few strings leave mostly empty).  One state, 60 groups
+// of 3 strings with up to four flips, all by transform / these two: 14 qubits 140 /
+// 90 us, 22 869 / 672; 8 strings 209 / 159, 1058 / 938; 16 to 23 strings 372 / 363,
+// but 1306 / 1502 at 22.
+constexpr int kHamFewStrings = 16;
+constexpr int kHamLoads = 4;           // partners on their way at a time (2 and 8 spill 400 to 600 bytes)
 __host__ __device__ inline int ham_smem_terms(const HamSweep& s) {
   return s.term1 - s.term0 <= kHamSmemTerms ? s.term1 - s.term0 : 0;
 }
 size_t ham_smem_bytes(const HamSweep& s, size_t amp) {
-  return (amp << kHamM) + (size_t)ham_smem_terms(s) * (32 + kHamThreads / 8) + (size_t)(s.item1 - s.item0) * sizeof(HamItem);
+  return (amp << kHamM) + (size_t)ham_smem_terms(s) * kHamStringBytes + (size_t)(s.item1 - s.item0) * sizeof(HamItem);
 }
 
 // One sweep.  blockIdx.y = set: psi + set * pstride, lam + set * lstride.
@@ -89,7 +100,10 @@ size_t ham_smem_bytes(const HamSweep& s, size_t amp) {
 // the integer rate.  256 threads of 16 amplitudes: 512 threads of 8 twice the
 // warps but spilled at 64 registers and read the strings twice as often (26
 // qubits: 1.10 / 0.77 / 0.78 ms).  L1 at 58 %, 16 warps per SM: latency-bound.
-template <class T>
+// PLAIN: a sweep whose strings are all staged and whose items are all real, in the
+// tile, and flat or of many strings (the other paths cost the chains' sweeps 2 % in
+// registers).
+template <class T, bool PLAIN>
 __global__ void __launch_bounds__(kHamThreads, 2)
 ham_sweep_kernel(const T* __restrict__ psi, uint64_t pstride, const __grid_constant__ HamSweep P,
                  const HamItem* __restrict__ g_items, const uint64_t* __restrict__ tz, const uint64_t* __restrict__ txm,
@@ -104,6 +118,7 @@ ham_sweep_kernel(const T* __restrict__ psi, uint64_t pstride, const __grid_const
   uint64_t* const sx = sz + nterms;
   HamItem* const items = reinterpret_cast<HamItem*>(sx + nterms);
   uint32_t* const words = reinterpret_cast<uint32_t*>(items + (P.item1 - P.item0));
+  uint32_t* const pats = words + nterms * (kHamThreads / 32);   // bit v: the string's sign at the thread's amplitude v
   __shared__ double red[kHamThreads / 32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   psi += blockIdx.y * pstride;
@@ -131,6 +146,14 @@ ham_sweep_kernel(const T* __restrict__ psi, uint64_t pstride, const __grid_const
       sz[k] = tz[P.term0 + k];
       sx[k] = txm[P.term0 + k];
       c0[k] = tc[P.term0 + k];
+      if (PLAIN) continue;
+      uint32_t m = 0;
+#pragma unroll
+      for (int j = 0; j < kHamRegBits; ++j) {
+        constexpr uint32_t kSet[kHamRegBits] = {0xAAAAu, 0xCCCCu, 0xF0F0u, 0xFF00u};   // amplitudes with register bit j
+        if ((sz[k] >> P.bit[kHamTidBits + j]) & 1) m ^= kSet[j];
+      }
+      pats[k] = m;
     }
     __syncthreads();
     for (int k = 0; k < nterms; ++k) {
@@ -170,7 +193,7 @@ ham_sweep_kernel(const T* __restrict__ psi, uint64_t pstride, const __grid_const
     // sum of the strings [k0, k1) at the thread's amplitude 0
     auto strings = [&](int k0, int k1) {
       double f = 0.0;
-      if (nterms) {
+      if (PLAIN || nterms) {
         for (int k = k0 - P.term0; k < k1 - P.term0; ++k) {
           const double c = sc[k];
           f += ((words[k * (kHamThreads / 32) + warp] >> lane) & 1) ? -c : c;
@@ -184,7 +207,7 @@ ham_sweep_kernel(const T* __restrict__ psi, uint64_t pstride, const __grid_const
       const HamItem& I = items[it];
       const uint32_t flags = I.flags, mt = I.lmask & (kHamThreads - 1), mv = I.lmask / kHamThreads;
       const T* const row = tile + (tid ^ mt);
-      if (flags == HAM_FLAT) {         // real, in the tile, one f for the thread's amplitudes
+      if (PLAIN ? (flags & HAM_FLAT) != 0 : flags == HAM_FLAT) {   // real, in the tile, one f for the thread's amplitudes
         const double f = strings(I.first[0], I.first[1]);
 #pragma unroll
         for (int v = 0; v < kHamV; ++v) {
@@ -195,10 +218,20 @@ ham_sweep_kernel(const T* __restrict__ psi, uint64_t pstride, const __grid_const
         continue;
       }
       double f[kHamV];
-      if (flags & HAM_FLAT) {
+      if (!PLAIN && (flags & HAM_FLAT)) {
         const double f0 = strings(I.first[0], I.first[1]);
 #pragma unroll
         for (int v = 0; v < kHamV; ++v) f[v] = f0;
+      } else if (!PLAIN && nterms && I.first[kHamV] - I.first[0] <= kHamFewStrings) {
+#pragma unroll
+        for (int v = 0; v < kHamV; ++v) f[v] = 0.0;
+        for (int k = I.first[0] - P.term0; k < I.first[kHamV] - P.term0; ++k) {
+          const int hi = __double2hiint(sc[k]), lo = __double2loint(sc[k]);
+          const uint32_t neg = pats[k] ^ (((words[k * (kHamThreads / 32) + warp] >> lane) & 1) ? 0xFFFFu : 0u);
+#pragma unroll
+          for (int v = 0; v < kHamV; ++v)
+            f[v] += __hiloint2double(hi ^ (int)((neg << (31 - v)) & 0x80000000u), lo);
+        }
       } else {
 #pragma unroll
         for (int p = 0; p < kHamV; ++p) f[p] = strings(I.first[p], I.first[p + 1]);
@@ -212,7 +245,7 @@ ham_sweep_kernel(const T* __restrict__ psi, uint64_t pstride, const __grid_const
               f[v | h] = a - b;
             }
       }
-      if (!(flags & (HAM_GATHER | HAM_IMAG))) {
+      if (PLAIN || !(flags & (HAM_GATHER | HAM_IMAG))) {
 #pragma unroll
         for (int v = 0; v < kHamV; ++v) {
           const double2 a = wide(row[(v ^ mv) * kHamThreads]);
@@ -222,18 +255,23 @@ ham_sweep_kernel(const T* __restrict__ psi, uint64_t pstride, const __grid_const
         continue;
       }
       const uint64_t gx = tx ^ I.xmask;
+      const bool gather = flags & HAM_GATHER, imag = flags & HAM_IMAG;
 #pragma unroll
-      for (int v = 0; v < kHamV; ++v) {
-        double2 a = make_double2(0.0, 0.0);
-        if (flags & HAM_GATHER) {
-          const uint64_t x = gx ^ vphys(v);
-          if (x < dim) a = wide(psi[x]);
-        } else {
-          a = wide(row[(v ^ mv) * kHamThreads]);
+      for (int v0 = 0; v0 < kHamV; v0 += kHamLoads) {
+        double2 a[kHamLoads];
+#pragma unroll
+        for (int v = 0; v < kHamLoads; ++v) {
+          const uint64_t x = gx ^ vphys(v0 + v);
+          a[v] = make_double2(0.0, 0.0);
+          if (!gather) a[v] = wide(row[((v0 + v) ^ mv) * kHamThreads]);
+          else if (x < dim) a[v] = wide(psi[x]);
         }
-        if (flags & HAM_IMAG) a = make_double2(-a.y, a.x);   // times i
-        acc[v].x = fma(f[v], a.x, acc[v].x);
-        acc[v].y = fma(f[v], a.y, acc[v].y);
+#pragma unroll
+        for (int v = 0; v < kHamLoads; ++v) {
+          const double2 t = imag ? make_double2(-a[v].y, a[v].x) : a[v];   // times i
+          acc[v0 + v].x = fma(f[v0 + v], t.x, acc[v0 + v].x);
+          acc[v0 + v].y = fma(f[v0 + v], t.y, acc[v0 + v].y);
+        }
       }
     }
 #pragma unroll
@@ -257,22 +295,117 @@ ham_sweep_kernel(const T* __restrict__ psi, uint64_t pstride, const __grid_const
   }
 }
 
+// The sum with one amplitude per thread, partners from global memory (sweeps[0]
+// of a plan of one sweep holds every item).  Arrays of few tiles leave most SMs
+// without one, and a group costs its tile ~1 us of a serial chain; here the array
+// is spread over every SM and a group costs a sweep over it.  gather_pays has the
+// line between the two.
+constexpr int kGatherThreads = 256;
+static_assert(kRedBlocks <= kHamPartials, "a gather launch has a partial sum per block");
+constexpr int kGatherStrings = 2048;   // staged at a time
+template <class T>
+__global__ void __launch_bounds__(kGatherThreads)
+ham_gather_kernel(const T* __restrict__ psi, uint64_t pstride, const __grid_constant__ HamSweep P,
+                  const HamItem* __restrict__ g_items, const uint64_t* __restrict__ tz, const uint64_t* __restrict__ txm,
+                  const double* __restrict__ tc, const ulonglong2* __restrict__ frames, T* __restrict__ lam,
+                  uint64_t lstride, double* __restrict__ re, double* __restrict__ im, uint32_t rstride) {
+  struct Group { uint64_t xmask; int first, last; };   // last: bit 30 marks imaginary coefficients
+  __shared__ Group groups[2 * kMaxHamGroups];
+  __shared__ ulonglong2 strings[kGatherStrings];       // Z mask; coefficient with the sign of the set's Pauli frame
+  __shared__ double red[kHamThreads / 32];
+  const int tid = threadIdx.x, ng = P.item1 - P.item0, nt = P.term1 - P.term0;
+  const int chunks = (nt + kGatherStrings - 1) / kGatherStrings;
+  const ulonglong2 frame = frames ? frames[blockIdx.y] : make_ulonglong2(0, 0);
+  psi += blockIdx.y * pstride;
+  if (lam) lam += blockIdx.y * lstride;
+  for (int i = tid; i < ng; i += kGatherThreads) {
+    const HamItem& I = g_items[P.item0 + i];
+    groups[i] = {I.xmask, I.first[0] - P.term0, (I.first[kHamV] - P.term0) | ((I.flags & HAM_IMAG) ? 1 << 30 : 0)};
+  }
+  auto stage = [&](int chunk) {
+    for (int k = chunk * kGatherStrings + tid; k < min(nt, (chunk + 1) * kGatherStrings); k += kGatherThreads) {
+      const uint64_t z = tz[P.term0 + k];
+      const double c = tc[P.term0 + k];
+      const bool neg = (__popcll(frame.x & z) + __popcll(txm[P.term0 + k] & frame.y)) & 1;
+      strings[k - chunk * kGatherStrings] = make_ulonglong2(z, (uint64_t)__double_as_longlong(neg ? -c : c));
+    }
+  };
+  if (chunks == 1) stage(0);
+  __syncthreads();
+  const uint64_t dim = 1ULL << P.nbits;
+  double er = 0.0, ei = 0.0;
+  for (uint64_t x0 = blockIdx.x * (uint64_t)kGatherThreads; x0 < dim; x0 += (uint64_t)gridDim.x * kGatherThreads) {
+    const uint64_t x = x0 + tid;
+    const bool on = x < dim;
+    double2 acc = make_double2(0.0, 0.0);
+    for (int ch = 0; ch < chunks; ++ch) {
+      if (chunks > 1) {
+        __syncthreads();
+        stage(ch);
+        __syncthreads();
+      }
+      if (!on) continue;
+      const int k0 = ch * kGatherStrings, k1 = k0 + kGatherStrings;
+      double2 next = wide(psi[x ^ groups[0].xmask]);
+      for (int g = 0; g < ng; ++g) {
+        double2 a = next;
+        if (g + 1 < ng && groups[g + 1].xmask != groups[g].xmask)
+          next = wide(psi[x ^ groups[g + 1].xmask]);   // on its way during the signs
+        const int first = max(groups[g].first, k0), last = min(groups[g].last & ((1 << 30) - 1), k1);
+        if (first >= last) continue;
+        double f = 0.0;
+        for (int k = first; k < last; ++k) {
+          const ulonglong2 s = strings[k - k0];
+          const double c = __longlong_as_double((long long)s.y);
+          f += (__popcll(x & s.x) & 1) ? -c : c;
+        }
+        if (groups[g].last >> 30) a = make_double2(-a.y, a.x);   // times i
+        acc.x = fma(f, a.x, acc.x);
+        acc.y = fma(f, a.y, acc.y);
+      }
+    }
+    if (!on) continue;
+    if (lam) store(lam + x, acc);
+    const double2 px = wide(psi[x]);
+    er += px.x * acc.x + px.y * acc.y;
+    ei += px.x * acc.y - px.y * acc.x;
+  }
+  er = block_total(er, red);
+  if (im) ei = block_total(ei, red);
+  if (tid == 0) {
+    re[(size_t)blockIdx.y * rstride + blockIdx.x] = er;
+    if (im) im[(size_t)blockIdx.y * rstride + blockIdx.x] = ei;
+  }
+}
+
 // the largest sweep: 64 groups of two items, kHamSmemTerms strings
 template <class T>
 constexpr size_t ham_smem_limit() {
-  return (sizeof(T) << kHamM) + (size_t)kHamSmemTerms * (32 + kHamThreads / 8) + 2 * kMaxHamGroups * sizeof(HamItem);
+  return (sizeof(T) << kHamM) + (size_t)kHamSmemTerms * kHamStringBytes + 2 * kMaxHamGroups * sizeof(HamItem);
 }
 
 template <class T>
 cudaError_t run_sweeps(const HamPlan& hp, const HamTables& tb, const ulonglong2* frames, const T* psi,
                        uint64_t pstride, int nsets, T* lam, uint64_t lstride, double* partials, double* energy, double* energy_im, cudaStream_t st) {
   if (nsets < 1) nsets = 1;
+  if (hp.gather) {
+    const HamSweep& s = hp.sweeps[0];
+    const uint32_t grid = (uint32_t)std::min<uint64_t>(((1ULL << s.nbits) + kGatherThreads - 1) / kGatherThreads, kRedBlocks);
+    double* const im = energy_im ? partials + (size_t)nsets * grid : nullptr;
+    ham_gather_kernel<T><<<dim3(grid, nsets), kGatherThreads, 0, st>>>(psi, pstride, s, tb.items, tb.z, tb.x, tb.c, frames, lam,
+                                                                      lstride, partials, im, grid);
+    cudaError_t e = launch_row_sums(partials, nsets, (int)grid, energy, st);
+    if (e == cudaSuccess && energy_im) e = launch_row_sums(im, nsets, (int)grid, energy_im, st);
+    return e;
+  }
   size_t smem_max = 0;
   for (const HamSweep& w : hp.sweeps) smem_max = std::max(smem_max, ham_smem_bytes(w, sizeof(T)));
   // per device, so on every call (always the same value: threads may race on it)
-  const cudaError_t attr =
-      cudaFuncSetAttribute(ham_sweep_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)ham_smem_limit<T>());
+  cudaError_t attr = cudaFuncSetAttribute(ham_sweep_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)ham_smem_limit<T>());
+  if (attr == cudaSuccess)
+    attr = cudaFuncSetAttribute(ham_sweep_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)ham_smem_limit<T>());
   if (attr != cudaSuccess) return attr;
   if (smem_max > ham_smem_limit<T>()) return cudaErrorInvalidValue;
   // sums: one column per block; every sweep's when lambda is not kept, else the last one's
@@ -286,7 +419,13 @@ cudaError_t run_sweeps(const HamPlan& hp, const HamTables& tb, const ulonglong2*
     s.add = (lam && i > 0) ? 1 : 0;
     const bool sums = !lam || i == np - 1;
     const size_t at = lam ? 0 : (size_t)i * grid;
-    ham_sweep_kernel<T><<<dim3(grid, nsets), kHamThreads, ham_smem_bytes(s, sizeof(T)), st>>>(
+    bool plain = ham_smem_terms(s) > 0;
+    for (int it = s.item0; it < s.item1; ++it) {
+      const HamItem& I = hp.items[it];
+      plain = plain && !(I.flags & (HAM_GATHER | HAM_IMAG)) &&
+              ((I.flags & HAM_FLAT) || I.first[kHamV] - I.first[0] > kHamFewStrings);
+    }
+    (plain ? ham_sweep_kernel<T, true> : ham_sweep_kernel<T, false>)<<<dim3(grid, nsets), kHamThreads, ham_smem_bytes(s, sizeof(T)), st>>>(
         psi, pstride, s, tb.items, tb.z, tb.x, tb.c, frames, lam, lstride, sums ? partials + at : nullptr,
         (sums && im) ? im + at : nullptr, rstride);
   }
@@ -297,8 +436,39 @@ cudaError_t run_sweeps(const HamPlan& hp, const HamTables& tb, const ulonglong2*
 
 }  // namespace
 
-void plan_hamiltonian(int n, const HamTerms& h, const uint64_t* zmask, const double2* coef, int max_sweeps,
+// Whether one amplitude per thread is the faster form for a plan's sweeps.  Its
+// time (us) follows groups and strings and the array past 2^16 amplitudes, where
+// every SM is busy; the sweeps' is a chain of groups per tile, the same for every
+// array of up to as many tiles as fit the GPU at once.  Both sides measured, one
+// state, sweeps / gather: TFIM 13 qubits 22.2 / 11.5, 18 34.4 / 28.8, 20 43 / 82;
+// 60 groups of 3 strings with up to four flips 87 / 24, 124 / 78, 166 / 248; 400
+// diagonal strings 47 / 22, 47 / 78, 54 / 249; 16 states of 14 qubits 31 / 22, 91 /
+// 64, 47 / 66.
+static bool gather_pays(const HamPlan& hp, int n, int nsets) {
+  const double amps = std::ldexp((double)std::max(1, nsets), n);
+  double tiles = 8.0 + 2.0 * (double)hp.sweeps.size(), groups = 0.0;
+  for (size_t i = 0; i < hp.items.size(); ++i) {
+    const HamItem& I = hp.items[i];
+    const double k = I.first[kHamV] - I.first[0];
+    tiles += (I.flags & HAM_FLAT) ? 0.5 + std::min(0.2 * k, 3.0 + 0.1 * k) : std::min(0.8 + 0.3 * k, 4.0 + 0.1 * k);
+    if (I.flags & HAM_GATHER) tiles += 0.8;
+    groups += i && I.xmask == hp.items[i - 1].xmask ? 0.25 : 1.0;   // a group's imaginary part reads the same partner
+  }
+  const double gather = 8.0 + std::max(1.0, amps / 65536.0) * (0.2 * groups + 0.04 * (double)hp.z.size());
+  return gather < tiles * std::max(1.0, amps / ((double)kHamBlocks * (1 << kHamM)));
+}
+
+static void plan_sweeps(int n, const HamTerms& h, const uint64_t* zmask, const double2* coef, int max_sweeps, HamPlan& hp);
+
+void plan_hamiltonian(int n, const HamTerms& h, const uint64_t* zmask, const double2* coef, int max_sweeps, int nsets,
                       HamPlan& hp) {
+  plan_sweeps(n, h, zmask, coef, max_sweeps, hp);
+  const char* form = getenv("IQ_HAM_GATHER");   // 0, 1: this form whatever the sizes
+  hp.gather = form && *form ? atoi(form) != 0 : gather_pays(hp, n, nsets);
+  if (hp.gather && hp.sweeps.size() > 1) plan_sweeps(n, h, zmask, coef, 1, hp);
+}
+
+static void plan_sweeps(int n, const HamTerms& h, const uint64_t* zmask, const double2* coef, int max_sweeps, HamPlan& hp) {
   hp.sweeps.clear();
   hp.items.clear();
   hp.z.clear();

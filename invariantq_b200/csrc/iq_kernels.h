@@ -131,6 +131,7 @@ struct HamTables {
   const double* c;
 };
 struct HamPlan {
+  bool gather = false;                 // one amplitude per thread instead of tiles (sweeps[0] holds everything)
   std::vector<HamSweep> sweeps;
   std::vector<HamItem> items;
   std::vector<uint64_t> z, x;
@@ -139,8 +140,9 @@ struct HamPlan {
   void pack(void* dst) const;          // table_bytes() bytes, 8-byte aligned
   HamTables tables(const void* dev) const;
 };
-// max_sweeps (1..kHamMaxSweeps): groups left over after that many sweeps gather from global memory
-void plan_hamiltonian(int n, const HamTerms& h, const uint64_t* zmask, const double2* coef, int max_sweeps,
+// max_sweeps (1..kHamMaxSweeps): groups left over after that many sweeps gather from global memory.
+// nsets: states of a launch (a plan serves any number; the form is chosen for this one)
+void plan_hamiltonian(int n, const HamTerms& h, const uint64_t* zmask, const double2* coef, int max_sweeps, int nsets,
                       HamPlan& hp);
 // For each of nsets states psi_s = psi + s * pstride (2^n amplitudes):
 // lambda_s = H psi_s written to lam + s * lstride (when lam is not null), and

@@ -1399,7 +1399,7 @@ int iq_statevector_expval_pauli_sum(void* sv, size_t nterms, const double* coeff
     }
     h.first[h.ngroups] = (int)z.size();
     HamPlan hp;
-    plan_hamiltonian(n, h, z.data(), co.data(), kHamMaxSweeps, hp);
+    plan_hamiltonian(n, h, z.data(), co.data(), kHamMaxSweeps, 1, hp);
     blob.resize(hp.table_bytes() / 16 + 1);
     hp.pack(blob.data());
     if (!e->upload_pool(blob.data(), blob.size())) return -1;
