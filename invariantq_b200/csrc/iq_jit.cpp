@@ -347,13 +347,13 @@ bool jit_prepare(const std::vector<const PassDesc*>& passes, std::vector<const J
     std::set<std::string> seen;
     std::lock_guard<std::mutex> lk(S.mu);
     for (size_t i = 0; i < passes.size(); ++i) {
-      keys[i] = jit_pass_key(*passes[i], min_blocks, threads, set_mode, narrow);
+      keys[i] = jit_pass_key(*passes[i], min_blocks, jit_pass_threads(*passes[i], threads), set_mode, narrow);
       auto it = S.cache.find({dev, keys[i]});
       if (it != S.cache.end()) { out[i] = it->second.get(); continue; }
       if (S.cache.size() + todo.size() >= kMaxKernels) continue;
       if (!seen.insert(keys[i]).second) continue;
       std::string e;
-      srcs[i] = jit_pass_source(*passes[i], e, min_blocks, threads, set_mode, narrow);
+      srcs[i] = jit_pass_source(*passes[i], e, min_blocks, jit_pass_threads(*passes[i], threads), set_mode, narrow);
       if (!srcs[i].empty()) todo.push_back((int)i);
     }
   }
@@ -393,12 +393,13 @@ void jit_lookup(const std::vector<const PassDesc*>& passes, std::vector<const Ji
   {
     std::lock_guard<std::mutex> lk(S.mu);
     for (size_t i = 0; i < passes.size(); ++i) {
-      std::pair<int, std::string> key(dev, jit_pass_key(*passes[i], min_blocks, threads, set_mode));
+      const int t = jit_pass_threads(*passes[i], threads);
+      std::pair<int, std::string> key(dev, jit_pass_key(*passes[i], min_blocks, t, set_mode));
       auto it = S.cache.find(key);
       if (it != S.cache.end()) { out[i] = it->second.get(); continue; }
       if (!queue_missing || S.pending.count(key) || S.cache.size() + S.pending.size() >= kMaxKernels) continue;
       std::string e;
-      std::string src = jit_pass_source(*passes[i], e, min_blocks, threads, set_mode);
+      std::string src = jit_pass_source(*passes[i], e, min_blocks, t, set_mode);
       if (src.empty()) continue;
       S.pending.insert(key);
       S.queue.push_back({dev, key.second, std::move(src)});

@@ -33,7 +33,8 @@ struct JitKernel;
 // compile fails.
 // min_blocks: resident CTAs per SM the kernels are compiled for (the launch's
 // TileLaunch::ctas_per_sm).
-// threads: CTA size of the kernels (128, 256; 0 = by register slots).
+// threads: CTA size of the kernels (128, 256; 0 = by register slots; kPairForm =
+// the pair pipeline where it pays, jit_pass_threads).
 // set_mode: the shared-memory form (passes over parameter sets, adjoint steps;
 // launched with jit_launch_sets).
 // narrow (with set_mode): kernels for complex64 arrays (jit_launch_narrow).

@@ -410,13 +410,23 @@ constexpr int kPairForm = 512;
 // amplitudes: the larger of its HBM traffic and 0.78 times the sum of its FP64
 // multiply-adds (0.065 ms each per amplitude) and its shared-memory round trips
 // (1.02 ms per stage and for the copies).  It chooses among plans, so their order
-// counts: of the limits 4, 5 and 8 it named the fastest, or one within 0.1 % of
+// counts: of the limits 4, 5 and 8 it named the fastest, or one within 0.3 % of
 // it, for eight circuits of 27 to 30 qubits (brick-walls, CZ rings, QFTs of 7
-// neighbours, random pairs).  Whole circuits take 0.92-1.02 times what it says,
-// those of random pairs 1.21 (their tile bits form many runs, so more and smaller
-// copies); single passes 0.82-1.65.
+// neighbours, random pairs).  Whole circuits take 0.93-1.03 times what it says,
+// those of random pairs 1.04-1.09; single passes 0.83-1.43.
 double pass_time_model(const PassDesc& d);
 inline bool pair_form_fits(const PassDesc& d) { return d.M == 12 && d.R == 4 && d.nH - d.nbox <= 7; }
+// A tile of 64 copies (its high bits scattered) keeps the pair pipeline's one
+// producer warp busy for 1.5 times its HBM time, where three CTAs issue from all
+// their threads; passes with more work than that still run faster in pairs.  27
+// qubits, pair / three CTAs: 64 copies 1.10-1.13 / 0.76-0.93 ms at up to 3 stages,
+// with dense two-qubit gates 1.16 / 2.1; 32 copies 0.69-0.70 / 0.75-0.87; one 0.74 /
+// 0.77.  24 qubits 0.15 / 0.105, 29 qubits 4.4 / 3.0.
+inline bool pair_form_pays(const PassDesc& d) { return d.nH - d.nbox < 6 || pass_time_model(d) > 7.2; }
+// CTA size for a pass of a program compiled with `threads` (kPairForm: the pair pipeline where it pays)
+inline int jit_pass_threads(const PassDesc& d, int threads) {
+  return threads == kPairForm && !pair_form_pays(d) ? 0 : threads;
+}
 std::string jit_pass_source(const PassDesc& d, std::string& err, int min_blocks = 2, int threads = 0,
                             bool set_mode = false, bool narrow = false);
 // Compact byte string of everything jit_pass_source's output depends on

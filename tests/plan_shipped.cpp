@@ -352,3 +352,42 @@ extern "C" unsigned long long shipped_structure(int n, int nops, const int* kind
     for (unsigned char ch : jit_pass_key(pl.desc, 3, 128, true, false)) h = (h ^ ch) * 1099511628211ull;
   return h;
 }
+
+// For every pass of a state program's plan: log2 of its tile's copies, and
+// whether it runs in the pair pipeline.  Returns the passes, -1 on an error.
+extern "C" int shipped_forms(int nbits, int nops, const int* ks, const int* qs, const double* mats,
+                             const long long* mat_off, int* boxes, int* pair, int max_passes) {
+  std::vector<cplx64> pool;
+  std::vector<SchedOp> ops;
+  for (int i = 0; i < nops; ++i) {
+    SchedOp o{};
+    o.k = (uint8_t)ks[i];
+    for (int j = 0; j < ks[i]; ++j) o.q[j] = (uint8_t)qs[i * 5 + j];
+    const int d = 1 << ks[i];
+    const double* m = mats + 2 * mat_off[i];
+    o.mat = o.dense = (uint32_t)pool.size();
+    for (int j = 0; j < d * d; ++j) pool.push_back({m[2 * j], m[2 * j + 1]});
+    double ph[8];
+    if (ks[i] <= 2 && classify_monomial(m, ks[i], &o.perm, ph, &o.unit)) {
+      o.mono = 1;
+      o.mat = (uint32_t)pool.size();
+      for (int j = 0; j < d; ++j) pool.push_back({ph[2 * j], ph[2 * j + 1]});
+    }
+    ops.push_back(o);
+  }
+  ops = fuse_two_qubit_blocks(ops, pool, true);
+  decompose_one_qubit_ops(ops, pool, DECOMP_STEADY);
+  normalize_one_qubit_ops(ops, pool);
+  SchedParams p = sched_params(12, 4, 4, 8, 160.0);
+  p.nbits = nbits;
+  std::vector<PassPlan> plans;
+  std::string err;
+  if (plan_passes(p, ops, plans, err) < 0 || (int)plans.size() > max_passes) return -1;
+  merge_stage_diagonals(plans, ops);
+  for (size_t i = 0; i < plans.size(); ++i) {
+    const PassDesc& d = plans[i].desc;
+    boxes[i] = d.nH - d.nbox;
+    pair[i] = pair_form_fits(d) && jit_pass_threads(d, kPairForm) == kPairForm;
+  }
+  return (int)plans.size();
+}
